@@ -18,7 +18,7 @@ LIB = os.path.join(HERE, '_lgx.so')
 
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 NVCC_FLAGS = ['-O3', '-lineinfo', '-std=c++17', '--expt-relaxed-constexpr', '-Xcompiler', '-fPIC',
-              '-Xcompiler', '-fvisibility=hidden', '-Xptxas', '-warn-spills']
+              '-Xcompiler', '-fvisibility=hidden', '-Xptxas', '-warn-spills', '--split-compile=4']
 
 
 def nvcc_path():

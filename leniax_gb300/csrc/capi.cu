@@ -176,18 +176,16 @@ size_t streamed_ws(const Model& m, int n_sols, int n_init, int steps, bool with_
   return b;
 }
 
-// General N-D engine: status, prepared spectra, raw moments, state ping-pong,
-// carried shifts, the step's own buffers.
+// General N-D engine: status, raw moments, state ping-pong, carried shifts,
+// the step's own buffers.
 struct NdLayout {
-  size_t kf, raw, sa, sb, shift, step, end;
+  size_t raw, sa, sb, shift, step, end;
 };
 
 NdLayout nd_layout(const Model& m, int n_sols, int n_init, int steps) {
   NdLayout L;
   const size_t nw = (size_t)n_sols * n_init;
   size_t off = kStatusBytes;
-  L.kf = off;
-  off += nd_prepared_bytes(m, n_sols);
   L.raw = off;
   off += al256((size_t)n_sols * std::max(steps, 1) * n_init * raw_stride(m.C) * sizeof(float));
   L.sa = off;
@@ -379,14 +377,13 @@ int lgx_run(const lgx_plan* plan, const lgx_rollout* j, void* ws, size_t ws_byte
   } else if (e == LGX_ENGINE_ND) {
     const NdLayout L = nd_layout(m, j->n_sols, j->n_init, j->steps);
     char* base = static_cast<char*>(ws);
-    float2* kf = reinterpret_cast<float2*>(base + L.kf);
     raw = reinterpret_cast<float*>(base + L.raw);
     float* sa = reinterpret_cast<float*>(base + L.sa);
     float* sb = reinterpret_cast<float*>(base + L.sb);
     int* shift = reinterpret_cast<int*>(base + L.shift);
-    ce = launch_nd_prepare(m, j->n_sols, reinterpret_cast<const float2*>(j->k_half), kf, st);
+    ce = launch_nd_begin(m, base + L.step, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(shift, 0, (size_t)nw * 4 * sizeof(int), st);
-    if (ce != cudaSuccess) return cuda_fail(ce, "prepare spectrum");
+    if (ce != cudaSuccess) return cuda_fail(ce, "N-D tables");
     const long raws = raw_stride(m.C);
     const float* cur = j->cells0;
     if (j->main_events[0]) cudaEventRecord(static_cast<cudaEvent_t>(j->main_events[0]), st);
@@ -399,8 +396,10 @@ int lgx_run(const lgx_plan* plan, const lgx_rollout* j, void* ws, size_t ws_byte
       ns.n_init = j->n_init;
       ns.state = cur;
       ns.state_out = out;
-      ns.kf = kf;
-      ns.kf_sol_stride = (long)m.C * m.max_k * m.cells;
+      ns.k_half = reinterpret_cast<const float2*>(j->k_half);
+      ns.k_sol_stride = (long)m.C * m.max_k * m.D * m.H * (m.W / 2 + 1);
+      ns.spec_ready = s > 0;
+      ns.emit_spec = s + 1 < j->steps;
       ns.gf = j->gf_params;
       ns.gf_sol_stride = 2L * m.K;
       ns.w = j->weights;
@@ -682,12 +681,11 @@ int lgx_update(const lgx_plan* plan, int n, const float* state, const float* k_h
     // one step of the general N-D engine, scalar or per-world dt
     const NdLayout L = nd_layout(m, 1, n, 1);
     char* base = static_cast<char*>(ws);
-    float2* kf = reinterpret_cast<float2*>(base + L.kf);
     int* shift = reinterpret_cast<int*>(base + L.shift);
     ce = cudaMemsetAsync(ws, 0, sizeof(int), st);
-    if (ce == cudaSuccess) ce = launch_nd_prepare(m, 1, reinterpret_cast<const float2*>(k_half), kf, st);
+    if (ce == cudaSuccess) ce = launch_nd_begin(m, base + L.step, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(shift, 0, (size_t)n * 4 * sizeof(int), st);
-    if (ce != cudaSuccess) return cuda_fail(ce, "prepare spectrum");
+    if (ce != cudaSuccess) return cuda_fail(ce, "N-D tables");
     NdStep ns;
     ns.state_copy = nullptr;
     ns.done = shift + 3 * n;
@@ -696,8 +694,9 @@ int lgx_update(const lgx_plan* plan, int n, const float* state, const float* k_h
     ns.n_init = n;
     ns.state = state;
     ns.state_out = state_out;
-    ns.kf = kf;
-    ns.kf_sol_stride = 0;
+    ns.k_half = reinterpret_cast<const float2*>(k_half);
+    ns.k_sol_stride = 0;
+    ns.spec_ready = ns.emit_spec = false;
     ns.gf = gf_params;
     ns.gf_sol_stride = 0;
     ns.w = weights;

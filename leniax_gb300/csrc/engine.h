@@ -183,23 +183,20 @@ cudaError_t launch_prepare_streamed_spectrum(const Model& m, int n_sols, const f
                                              cudaStream_t st);
 
 // ---------------------------------------------------------------- general N-D engine
-// Any 2D / 3D torus whose sides factor into 2, 3, 5, 7 (2..512), any C and K:
-// mixed-radix line passes over full complex spectra in HBM (nd.cu).
+// Any 2D / 3D torus with sides nd_side_ok takes, any C and K: line transforms
+// over half spectra in HBM / L2 (nd.cu).
 bool nd_side_ok(int n);
 int nd_max_side();  // longest world axis of the N-D engine
 bool nd_supported(const Model& m);
-int nd_blocks_per_world(const Model& m, long n_worlds);
-// Prepared spectra [Ns, C, max_k, cells] complex: the Hermitian half
-// [Ns, C, max_k, D, H, W/2+1] extended to the full spectrum, scaled by 1/cells.
-size_t nd_prepared_bytes(const Model& m, int n_sols);
-cudaError_t launch_nd_prepare(const Model& m, int n_sols, const float2* k_half, float2* kf, cudaStream_t st);
 struct NdStep {
   const Model* m;
   int n_worlds, n_init;
   const float* state;   // [n_worlds, C, cells]
   float* state_out;     // [n_worlds, C, cells]
-  const float2* kf;     // prepared spectra per solution
-  long kf_sol_stride;   // float2 elements between solutions (0: shared)
+  const float2* k_half; // Hermitian half spectra [Ns, C, max_k, D, H, W/2+1] as given
+  long k_sol_stride;    // float2 elements between solutions (0: shared)
+  bool spec_ready;      // the previous step of this workspace emitted the spectra of `state`
+  bool emit_spec;       // write the spectra of state_out for the next step
   const float* gf;      // [Ns, K, 2]
   long gf_sol_stride;
   const float* w;       // [Ns, C, K]
@@ -213,8 +210,9 @@ struct NdStep {
   int* shift;           // [n_worlds, 3] carried torus shift (read, then advanced)
   int* done;            // [n_worlds] per-world block counters, zero before the first step (kept zero)
   float* state_copy;    // [n_worlds, C, cells] copy of the entering state (trajectory), or null
-  void* ws;             // nd_step_workspace_bytes
+  void* ws;             // nd_step_workspace_bytes; launch_nd_begin once before its first step
 };
+cudaError_t launch_nd_begin(const Model& m, void* ws, cudaStream_t st);
 size_t nd_step_workspace_bytes(const Model& m, int n_worlds);
 cudaError_t launch_nd_step(const NdStep& s, cudaStream_t st);
 struct NdAdjoint {
@@ -227,7 +225,7 @@ struct NdAdjoint {
   const float* traj_potential;  // [steps, nw, K, cells]
   const float* lambda_in;       // [nw, C, cells]
   float* lambda_out;            // [nw, C, cells]
-  float2* gk;                   // [nw, K, cells] kernel-gradient spectra (+=)
+  float2* gk;                   // [nw, K, D, H, W/2+1] kernel-gradient spectra (+=)
   float* grad_gf;               // [Ns, K, 2] (+=)
   float* grad_weights;          // [Ns, C, K] (+=)
   const float* cells_after;     // [nw, C, cells] state after the last step, or null

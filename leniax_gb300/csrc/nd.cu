@@ -1,64 +1,70 @@
-// General N-D engine: any 2D or 3D torus whose sides factor into 2, 3, 5
-// and 7 (odd, non-square and non-power-of-two sides included, e.g. 48^3),
-// any number of channels and kernels -- the forward Euler step and its
+// General N-D engine: any 2D or 3D torus with sides 2..4096 of factors 2, 3, 5
+// and 7 or any side 2..2048 (odd, prime and non-square sides included, e.g.
+// 48^3), any number of channels and kernels -- the forward Euler step and its
 // adjoint.  leniax's get_potential_fft transforms every world axis
-// (core.py:74-87); here each axis is one pass of mixed-radix line FFTs over
-// complex planes in HBM:
+// (core.py:74-87); here real rows travel in packed pairs and every later axis
+// works on half spectra of W/2 + 1 columns:
 //
-//   forward step : x pass (real state in), y pass, z pass   -> state spectra S
-//                  S[c_in(k)] x prepared spectrum[k]           -> products P
-//                  z, y, x inverse passes (real part out)      -> potentials u_k
-//                  growth, weighted field, state update and the statistics
-//                  moments per block (core.py:163-319, statistics.py:36-126)
-//                  per-world reduction of the moments, carried torus shift
+//   first step   : x (2D) or x and y (3D) transforms of the states -> S
+//   Euler step   : conv   (nd_conv.cu): last axis forward, x spectrum of every
+//                  kernel, last axis inverse                      -> P
+//                  epilogue (nd_rows.cu, nd_plane.cu): inverse y and x
+//                  transforms -> potentials u_k, growth, weighted field, state
+//                  update (core.py:163-319), statistics moments
+//                  (statistics.py:36-126), per-world reduction and carried
+//                  shift, x (and y) transforms of the new states -> S
 //   adjoint step : clip / state-function gradient, dL/df, dL/dg, growth
-//                  derivative -> a_k = dL/du_k; forward passes of a_k and of
-//                  the state; kernel gradient A_k conj(S) accumulated; the
+//                  derivative -> a_k = dL/du_k; forward transforms of a_k and
+//                  of the state; kernel gradient A_k conj(S) accumulated; the
 //                  correlation sum_k A_k conj(K_k) per input channel through
-//                  the inverse passes added to lambda; growth-parameter and
-//                  weight gradients reduced per (world, kernel)
+//                  the inverse transforms added to lambda; growth-parameter
+//                  and weight gradients reduced per (world, kernel)
 //
-// A pass stages a tile of lines in shared memory (consecutive lines of the
-// same group so that global loads and stores are coalesced), runs the
-// Stockham transform of fft_mixed.cuh and writes the tile back in place.
-// Spectra are full complex (no Hermitian packing), so odd sides need no
-// special case.  This engine serves the worlds the specialised engines do not
-// (resident: 2D 32..128 C = K = 1; streamed: square 2D; one world per CTA:
-// 3D 32^3 / 64^3 C = K = 1) and every differentiated model beyond C = K = 1.
+// 3D worlds whose z-planes do not fit a tile take their y transforms as a pass
+// of their own (nd_columns).  An Euler step is two launches.  Measured against
+// the engine this replaced (full complex planes, one radix-2..7 stage per
+// block barrier, three to six launches a step): see the kernels.
+//
+// This engine serves the worlds the specialised engines do not (resident: 2D
+// 32..128 C = K = 1; streamed: square 2D powers of two; one world per CTA: 3D
+// 32^3 / 64^3 C = K = 1) and every differentiated model beyond C = K = 1.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <mutex>
+#include <utility>
 #include <vector>
 
-#include "common.cuh"
-#include "engine.h"
-#include "fft_mixed.cuh"
+#include "nd.cuh"
 
 namespace lgx {
+
+// (kernel, context) pairs whose dynamic shared-memory limit is already raised
+cudaError_t nd_allow_smem(const void* kernel) {
+  static std::mutex mu;
+  static std::vector<std::pair<const void*, unsigned long long>> done;
+  unsigned long long ctx = 0;
+  const bool known = current_context_id(&ctx);
+  const std::pair<const void*, unsigned long long> key(kernel, ctx);
+  if (known) {
+    std::lock_guard<std::mutex> lk(mu);
+    if (std::find(done.begin(), done.end(), key) != done.end()) return cudaSuccess;
+  }
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kNdSmemMax - (int)fa.sharedSizeBytes);
+  if (e == cudaSuccess && known) {
+    std::lock_guard<std::mutex> lk(mu);
+    done.push_back(key);
+  }
+  return e;
+}
+
 namespace {
 
-constexpr int kNT = 256;          // threads per block
-constexpr int kNdMaxN = 4096;     // longest world axis (one 4096-point line per pass tile)
-constexpr int kBluesteinMaxN = 2048;  // longest axis with a prime factor above 7 (M <= 4096)
-constexpr int kMaxPts = 4096;     // complex points of one pass tile (two buffers in shared memory)
-// Launches smaller than this many blocks (two on each of GB300's 152 SMs)
-// get smaller tiles / chunks so that one small world still spreads over the
-// whole GPU; large batches keep the full-size tiles.  Measured on one 48^3
-// world (forward + adjoint): 1, 2, 4 and 8 blocks per SM gave 8.45, 8.7,
-// 6.25 and 5.6 thousand fwd+bwd world-steps/s (more, smaller blocks pay
-// more per-block start-up than they gain in parallelism).
-constexpr long kFillBlocks = 2 * 152;
-constexpr int kRawMax = RAW_CM + kMaxChannels;
-
-struct NdTab {  // kernel table of a model, passed by value
-  int C, K, max_k, mean, state_fn, dt_mode, nd;
-  int D, H, W;
-  long cells;
-  int cin[kMaxKernels];
-  int slot[kMaxKernels];
-  int gf[kMaxKernels];
-};
+constexpr int kNT = 256;  // threads of the pointwise kernels
 
 NdTab make_tab(const Model& m, int dt_mode) {
   NdTab t;
@@ -72,7 +78,9 @@ NdTab make_tab(const Model& m, int dt_mode) {
   t.D = m.D;
   t.H = m.H;
   t.W = m.W;
+  t.Wh = m.W / 2 + 1;
   t.cells = m.cells;
+  t.hcells = (long)m.D * m.H * t.Wh;
   for (int k = 0; k < kMaxKernels; ++k) {
     t.cin[k] = k < m.K ? m.cin[k] : 0;
     t.slot[k] = k < m.K ? m.slot[k] : 0;
@@ -81,973 +89,113 @@ NdTab make_tab(const Model& m, int dt_mode) {
   return t;
 }
 
-// ------------------------------------------------------------------ passes
-// Lines of a pass: line (g, i) starts at g * gstride + i and has L points
-// `stride` apart; g < G, i < I.  I == 1: a tile is nl consecutive groups
-// (rows of the x pass, contiguous); I > 1: nl consecutive i of one group.
-// The smallest M >= 2L - 1 whose prime factors are 2, 3, 5, 7 (the
-// Bluestein transform length of an L-point line), or 0 past the tile size.
-inline int bluestein_size(int L) {
-  if (L < 2 || L > kBluesteinMaxN) return 0;
-  for (int m = 2 * L - 1; m <= kMaxPts; ++m)
-    if (make_plan(m).stages > 0) return m;
+// ------------------------------------------------------------------ tables
+// Length of an n-point line's transforms: n, or the smallest m >= 2n - 1 of
+// factors 2, 3, 5, 7 (Bluestein); 0 when neither fits a tile.
+int transform_len(int n) {
+  int r[kLineStages];
+  if (n < 2) return 0;
+  if (n <= kNdMaxN && line_radices(n, r) > 0) return n;
+  if (n > kBluesteinMaxN) return 0;
+  for (int m = 2 * n - 1; m <= kMaxPts; ++m)
+    if (line_radices(m, r) > 0 && make_plan(m).stages > 0) return m;
   return 0;
 }
 
-struct Pass {
-  float2* data;          // complex planes (in and out, in place)
-  const float* src_real;  // IN_REAL: real input of the same geometry
-  float* dst_real;        // OUT_REAL: Re(result) * scale (stored, or added when accumulate)
-  long G, I, gstride, stride;
-  int L, nl;
-  int M;                  // Bluestein lines: the transform length M >= 2L - 1 (0: an L-point transform)
-  FastDivU fnl;            // division by nl
-  int in_real, out_real, accumulate;
-  float scale;
+size_t axis_table_bytes(int n) { return al256(line_table_elems(n, transform_len(n)) * sizeof(float2)); }
+size_t table_bytes(int D, int H, int W) {
+  return axis_table_bytes(W) + axis_table_bytes(H) + (D > 1 ? axis_table_bytes(D) : 0);
+}
+
+// The axes of a D x H x W world with their tables at `ws`.
+NdAxes make_axes(int D, int H, int W, void* ws) {
+  NdAxes a{};
+  char* p = static_cast<char*>(ws);
+  make_line_axis(W, transform_len(W), reinterpret_cast<float2*>(p), &a.x);
+  p += axis_table_bytes(W);
+  make_line_axis(H, transform_len(H), reinterpret_cast<float2*>(p), &a.y);
+  p += axis_table_bytes(H);
+  if (D > 1) make_line_axis(D, transform_len(D), reinterpret_cast<float2*>(p), &a.z);
+  return a;
+}
+
+// Tables of one axis per block: the twiddles W_m^j and, for Bluestein lines,
+// the chirp c_n = exp(-i pi n^2 / L) (exact reduction of n^2 mod 2L) and the
+// m-point spectrum of conj(c) wrapped around.  They are made once per call
+// and shared by all its launches; building them in every block of every pass
+// cost each block a sincospif per point, or a whole transform.
+struct TableArgs {
+  float2* t[3];
+  int n[3], m[3];
+  GPlan p[3];
 };
-
-// Bluestein's chirp-z transform (L. Bluestein, "A linear filtering approach
-// to the computation of discrete Fourier transform", 1970) for lines whose
-// length has a prime factor above 7: with c_n = exp(-i pi n^2 / L),
-// X_k = c_k sum_n (x_n c_n) conj(c_{k-n}), a cyclic convolution of length
-// M >= 2L - 1 done with M-point transforms (the inverse transform uses
-// conj(c)).  The tile holds nl lines of M points (x_n c_n, then zeros);
-// `chirp` c_n (n < L) and `bhat` = FFT_M(b), b_m = conj(c_|m|) for |m| < L
-// (indices mod M), are in shared memory.  b is even, so FFT_M(conj(b)) =
-// conj(bhat).  Unnormalised like fft_line; returns the buffer holding X.
-template <bool INV>
-__device__ float2* bluestein_lines(float2* A, float2* B, const GPlan& p, const float2* tw, const float2* chirp,
-                                   const float2* bhat, int nl, int L) {
-  const int M = p.n;
-  for (int l = 0; l < nl; ++l)
-    for (int j = threadIdx.x; j < L; j += blockDim.x) {
-      const float2 c = chirp[j];
-      A[l * M + j] = INV ? cmulc(A[l * M + j], c) : cmul(A[l * M + j], c);
-    }
+__global__ void __launch_bounds__(kNT) nd_tables_kernel(TableArgs a) {
+  extern __shared__ __align__(16) float2 sm[];
+  const int b = blockIdx.x, n = a.n[b], m = a.m[b];
+  float2* out = a.t[b];
+  if (m == n) {
+    for (int j = threadIdx.x; j < m; j += blockDim.x) out[j] = tw_entry(j, m);
+    return;
+  }
+  float2 *tw = sm, *A = sm + m, *B = A + m;
+  for (int j = threadIdx.x; j < m; j += blockDim.x) out[j] = tw[j] = tw_entry(j, m);
+  for (int j = threadIdx.x; j < m; j += blockDim.x) {
+    const int d = j < n ? j : (m - j < n ? m - j : -1);
+    const float2 c = d >= 0 ? tw_entry((int)(((long)d * d) % (2L * n)), 2 * n) : make_float2(0.f, 0.f);
+    if (j < n) out[m + j] = c;
+    A[j] = d >= 0 ? conjf2(c) : c;
+  }
   __syncthreads();
-  float2* r = fft_line<false>(A, B, p, tw, nl);
-  for (int l = 0; l < nl; ++l)
-    for (int k = threadIdx.x; k < M; k += blockDim.x)
-      r[l * M + k] = INV ? cmulc(r[l * M + k], bhat[k]) : cmul(r[l * M + k], bhat[k]);
-  __syncthreads();
-  float2* q = fft_line<true>(r, r == A ? B : A, p, tw, nl);
-  const float inv_m = 1.f / (float)M;
-  for (int l = 0; l < nl; ++l)
-    for (int k = threadIdx.x; k < L; k += blockDim.x) {
-      const float2 v = INV ? cmulc(q[l * M + k], chirp[k]) : cmul(q[l * M + k], chirp[k]);
-      q[l * M + k] = make_float2(v.x * inv_m, v.y * inv_m);
-    }
-  __syncthreads();
-  return q;
+  const float2* r = fft_line<false>(A, B, a.p[b], tw);
+  for (int j = threadIdx.x; j < m; j += blockDim.x) out[m + n + j] = r[j];
 }
 
-// chirp c_n = exp(-2 pi i (n^2 mod 2L) / 2L) and bhat = FFT_M(b), computed by
-// the block in shared memory with A and B as the transform's scratch
-__device__ void bluestein_tables(float2* chirp, float2* bhat, float2* A, float2* B, const GPlan& p,
-                                 const float2* tw, int L) {
-  const int M = p.n;
-  for (int n = threadIdx.x; n < L; n += blockDim.x) chirp[n] = tw_entry((int)(((long)n * n) % (2L * L)), 2 * L);
-  __syncthreads();
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    const int d = m < L ? m : (M - m < L ? M - m : -1);
-    A[m] = d >= 0 ? conjf2(chirp[d]) : make_float2(0.f, 0.f);
+cudaError_t launch_tables(const NdAxes& ax, int D, cudaStream_t st) {
+  TableArgs a{};
+  const LineAxis* l[3] = {&ax.x, &ax.y, &ax.z};
+  const int naxes = D > 1 ? 3 : 2;
+  size_t smem = 0;
+  for (int i = 0; i < naxes; ++i) {
+    a.t[i] = const_cast<float2*>(l[i]->tw);
+    a.n[i] = l[i]->n;
+    a.m[i] = l[i]->m;
+    a.p[i] = make_plan(l[i]->m);
+    if (l[i]->m != l[i]->n) smem = std::max(smem, 3 * (size_t)l[i]->m * sizeof(float2));
   }
-  __syncthreads();
-  const float2* r = fft_line<false>(A, B, p, tw, 1);
-  for (int m = threadIdx.x; m < M; m += blockDim.x) bhat[m] = r[m];
-  __syncthreads();
-}
-
-template <bool INV, bool BL>
-__global__ void __launch_bounds__(kNT, 3) nd_pass_kernel(Pass a, GPlan p) {
-  extern __shared__ __align__(16) float2 ndsm[];
-  const int L = a.L, nl = a.nl;
-  const int S = BL ? a.M : L;  // points per line in the tile
-  float2* tw = ndsm;
-  float2* A = tw + S;
-  float2* B = A + (size_t)nl * S;
-  float2* chirp = B + (size_t)nl * S;  // Bluestein tables (BL only)
-  float2* bhat = chirp + L;
-  long g0, i0;
-  int lines;
-  if (a.I == 1) {
-    g0 = (long)blockIdx.x * nl;
-    i0 = 0;
-    lines = (int)min((long)nl, a.G - g0);
-  } else {
-    const long tiles = (a.I + nl - 1) / nl;
-    g0 = blockIdx.x / tiles;
-    i0 = (blockIdx.x % tiles) * nl;
-    lines = (int)min((long)nl, a.I - i0);
+  if (smem > 0) {
+    const cudaError_t e = nd_allow_smem((const void*)nd_tables_kernel);
+    if (e != cudaSuccess) return e;
   }
-  fill_twiddles(tw, S);
-  if (BL) {
-    __syncthreads();
-    bluestein_tables(chirp, bhat, A, B, p, tw, L);
-  }
-  const int pts = nl * L;
-  // A tile of the x pass is nl whole rows, contiguous in memory and in the
-  // tile (point idx at row-block offset idx); a strided pass's tile holds
-  // nl adjacent lines, point idx = j nl + l of the global walk landing at
-  // l L + j in the tile.
-  const bool rows = a.I == 1;
-  const long gbase = rows ? g0 * a.gstride : g0 * a.gstride + i0;
-  const int valid = rows ? lines * L : pts;
-  // kLoadBatch independent global loads in flight per thread before their
-  // shared-memory stores (one load per iteration would serialise on latency)
-  constexpr int kLoadBatch = 8;
-  for (int base = threadIdx.x; base < pts; base += kLoadBatch * blockDim.x) {
-    float2 v[kLoadBatch];
-    int dst[kLoadBatch];
-#pragma unroll
-    for (int u = 0; u < kLoadBatch; ++u) {
-      const int idx = base + u * blockDim.x;
-      long off;
-      bool in;
-      if (rows && !BL) {
-        dst[u] = idx < pts ? idx : -1;
-        in = idx < valid;
-        off = gbase + idx;
-      } else if (rows) {  // Bluestein rows: tile lines of M points
-        const int l = idx / L, j = idx - l * L;
-        dst[u] = idx < pts ? l * S + j : -1;
-        in = idx < valid;
-        off = gbase + idx;
-      } else {
-        const int j = a.fnl.div(idx), l = idx - j * nl;
-        dst[u] = idx < pts ? l * S + j : -1;
-        in = idx < pts && l < lines;
-        off = gbase + l + (long)j * a.stride;
-      }
-      v[u] = make_float2(0.f, 0.f);
-      if (in) v[u] = a.in_real ? make_float2(__ldg(a.src_real + off), 0.f) : a.data[off];
-    }
-#pragma unroll
-    for (int u = 0; u < kLoadBatch; ++u)
-      if (dst[u] >= 0) A[dst[u]] = v[u];
-  }
-  if (BL)  // the zero padding of every tile line
-    for (int l = 0; l < nl; ++l)
-      for (int j = L + threadIdx.x; j < S; j += blockDim.x) A[l * S + j] = make_float2(0.f, 0.f);
-  __syncthreads();
-  const float2* res = BL ? bluestein_lines<INV>(A, B, p, tw, chirp, bhat, nl, L) : fft_line<INV>(A, B, p, tw, nl);
-  for (int idx = threadIdx.x; idx < valid; idx += blockDim.x) {
-    long off;
-    int src;
-    if (rows && !BL) {
-      off = gbase + idx;
-      src = idx;
-    } else if (rows) {
-      const int l = idx / L;
-      off = gbase + idx;
-      src = l * S + (idx - l * L);
-    } else {
-      const int j = a.fnl.div(idx), l = idx - j * nl;
-      if (l >= lines) continue;
-      off = gbase + l + (long)j * a.stride;
-      src = l * S + j;
-    }
-    const float2 v = res[src];
-    if (a.out_real) {
-      const float r = v.x * a.scale;
-      a.dst_real[off] = a.accumulate ? a.dst_real[off] + r : r;
-    } else {
-      a.data[off] = v;
-    }
-  }
-}
-
-// Raise the N-D kernels' dynamic shared-memory limits once per CUDA context
-// (the attribute belongs to the context: a context created later, after a
-// device reset for example, gets them again).
-cudaError_t allow_nd_smem();
-
-// One axis pass over `planes` planes of D x H x W points.  axis 0 = x
-// (contiguous), 1 = y, 2 = z.
-cudaError_t run_pass(bool inv, int axis, const NdTab& t, long planes, float2* data, const float* src_real,
-                     float* dst_real, bool accumulate, float scale, cudaStream_t st) {
-  Pass a;
-  a.data = data;
-  a.src_real = src_real;
-  a.dst_real = dst_real;
-  a.in_real = src_real != nullptr;
-  a.out_real = dst_real != nullptr;
-  a.accumulate = accumulate ? 1 : 0;
-  a.scale = scale;
-  const long HW = (long)t.H * t.W;
-  if (axis == 0) {
-    a.L = t.W;
-    a.G = planes * t.D * t.H;
-    a.I = 1;
-    a.gstride = t.W;
-    a.stride = 1;
-  } else if (axis == 1) {
-    a.L = t.H;
-    a.G = planes * t.D;
-    a.I = t.W;
-    a.gstride = HW;
-    a.stride = t.W;
-  } else {
-    a.L = t.D;
-    a.G = planes;
-    a.I = HW;
-    a.gstride = HW * t.D;
-    a.stride = HW;
-  }
-  GPlan p = make_plan(a.L);
-  a.M = 0;
-  if (p.stages == 0) {  // Bluestein lines
-    a.M = bluestein_size(a.L);
-    if (a.M == 0) return cudaErrorInvalidValue;
-    p = make_plan(a.M);
-  }
-  const bool bl = a.M > 0;
-  const int S = bl ? a.M : a.L;
-  const int cap = std::max(1, kMaxPts / S);
-  // lines per tile: the full tile, or fewer when the pass has too few lines
-  // to fill the GPU (at least 4 adjacent lines of a strided pass, so each
-  // load still covers a 32-byte sector)
-  const long fill = (a.G * a.I + kFillBlocks - 1) / kFillBlocks;
-  const long want = std::max<long>(a.I == 1 ? 1 : 4, fill);
-  a.nl = (int)std::min<long>(std::min<long>(cap, want), a.I == 1 ? a.G : a.I);
-  a.fnl = make_fastdiv((unsigned)a.nl);
-  const long tiles = a.I == 1 ? (a.G + a.nl - 1) / a.nl : a.G * ((a.I + a.nl - 1) / a.nl);
-  const size_t smem = (size_t)(S + 2L * a.nl * S + (bl ? a.L + S : 0)) * sizeof(float2);
-  cudaError_t e = allow_nd_smem();
-  if (e != cudaSuccess) return e;
-  if (tiles >= (1L << 31)) return cudaErrorInvalidConfiguration;
-  if (bl) {
-    if (inv) nd_pass_kernel<true, true><<<(unsigned)tiles, kNT, smem, st>>>(a, p);
-    else nd_pass_kernel<false, true><<<(unsigned)tiles, kNT, smem, st>>>(a, p);
-  } else {
-    if (inv) nd_pass_kernel<true, false><<<(unsigned)tiles, kNT, smem, st>>>(a, p);
-    else nd_pass_kernel<false, false><<<(unsigned)tiles, kNT, smem, st>>>(a, p);
-  }
+  nd_tables_kernel<<<naxes, kNT, smem, st>>>(a);
   return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------- plane passes
-// 3D worlds whose z-planes fit one tile (H W <= kMaxPts): the x and y
-// transforms of a plane in one block -- rows as contiguous lines, then the
-// columns of the same row-major tile -- one global read and write per plane
-// instead of one per axis.  The line transforms and their order are those of
-// the axis passes: x then y forward, y then x inverse.
-struct PlaneArgs {
-  float2* data;           // complex planes (in and out, in place)
-  const float* src_real;  // forward: real input of the same geometry, or null
-  float* dst_real;        // inverse: Re(result) * scale (stored, or added when accumulate), or null
-  int accumulate;
-  float scale;
-  int H, W;
-  FastDivU wdiv;  // division by W
-};
-
-template <bool INV>
-__global__ void __launch_bounds__(kNT, 3) nd_plane_kernel(PlaneArgs a, GPlan px, GPlan py) {
-  extern __shared__ __align__(16) float2 ndsm[];
-  const int H = a.H, W = a.W, pts = H * W;
-  float2* twx = ndsm;
-  float2* twy = twx + W;
-  float2* A = twy + H;
-  float2* B = A + pts;
-  const long base = (long)blockIdx.x * pts;
-  fill_twiddles(twx, W);
-  fill_twiddles(twy, H);
-  constexpr int kLoadBatch = 8;
-  for (int b0 = threadIdx.x; b0 < pts; b0 += kLoadBatch * blockDim.x) {
-    float2 v[kLoadBatch];
-#pragma unroll
-    for (int u = 0; u < kLoadBatch; ++u) {
-      const int idx = b0 + u * blockDim.x;
-      v[u] = make_float2(0.f, 0.f);
-      if (idx < pts) v[u] = a.src_real ? make_float2(__ldg(a.src_real + base + idx), 0.f) : a.data[base + idx];
-    }
-#pragma unroll
-    for (int u = 0; u < kLoadBatch; ++u) {
-      const int idx = b0 + u * blockDim.x;
-      if (idx < pts) A[idx] = v[u];
-    }
-  }
-  __syncthreads();
-  float2* r;
-  if (!INV) {
-    r = fft_line<false>(A, B, px, twx, H);                          // x: H rows of W points
-    r = fft_cols<false>(r, r == A ? B : A, py, twy, W, W, a.wdiv);  // y: W columns of H points
-  } else {
-    r = fft_cols<true>(A, B, py, twy, W, W, a.wdiv);
-    r = fft_line<true>(r, r == A ? B : A, px, twx, H);
-  }
-  for (int idx = threadIdx.x; idx < pts; idx += blockDim.x) {
-    const float2 v = r[idx];
-    if (a.dst_real) {
-      const float x = v.x * a.scale;
-      a.dst_real[base + idx] = a.accumulate ? a.dst_real[base + idx] + x : x;
-    } else {
-      a.data[base + idx] = v;
-    }
-  }
-}
-
-bool plane_ok(const NdTab& t) {
-  return t.D > 1 && (long)t.H * t.W <= kMaxPts && make_plan(t.H).stages > 0 && make_plan(t.W).stages > 0;
-}
-
-// Shared memory of the fused plane epilogue (twiddles, two tiles, the
-// channels' fields), or 0 when the world does not take it.
-constexpr size_t kPlaneEpiSmemMax = 200 * 1024;
-size_t plane_epi_smem(const NdTab& t) {
-  if (!plane_ok(t)) return 0;
-  const size_t pts = (size_t)t.H * t.W;
-  const size_t bytes = (t.W + t.H + 2 * pts) * sizeof(float2) + (size_t)t.C * pts * sizeof(float);
-  return bytes <= kPlaneEpiSmemMax ? bytes : 0;
-}
-
-// The x and y transforms of `planes` 3D planes (each D z-planes of H x W).
-cudaError_t run_plane(bool inv, const NdTab& t, long planes, float2* data, const float* src_real, float* dst_real,
-                      bool accumulate, float scale, cudaStream_t st) {
-  PlaneArgs a;
-  a.data = data;
-  a.src_real = src_real;
-  a.dst_real = dst_real;
-  a.accumulate = accumulate ? 1 : 0;
-  a.scale = scale;
-  a.H = t.H;
-  a.W = t.W;
-  a.wdiv = make_fastdiv((unsigned)t.W);
-  const GPlan px = make_plan(t.W), py = make_plan(t.H);
-  if (px.stages == 0 || py.stages == 0) return cudaErrorInvalidValue;
-  const long blocks = planes * t.D;
-  if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
-  const size_t smem = (size_t)(t.W + t.H + 2L * t.H * t.W) * sizeof(float2);
-  cudaError_t e = allow_nd_smem();
-  if (e != cudaSuccess) return e;
-  if (inv) nd_plane_kernel<true><<<(unsigned)blocks, kNT, smem, st>>>(a, px, py);
-  else nd_plane_kernel<false><<<(unsigned)blocks, kNT, smem, st>>>(a, px, py);
-  return cudaGetLastError();
-}
-
-// Full forward transform of real planes (src) into complex planes (dst).
-cudaError_t forward_real(const NdTab& t, long planes, const float* src, float2* dst, cudaStream_t st) {
-  cudaError_t e;
-  if (plane_ok(t)) {
-    e = run_plane(false, t, planes, dst, src, nullptr, false, 1.f, st);
-  } else {
-    e = run_pass(false, 0, t, planes, dst, src, nullptr, false, 1.f, st);
-    if (e == cudaSuccess) e = run_pass(false, 1, t, planes, dst, nullptr, nullptr, false, 1.f, st);
-  }
-  if (e == cudaSuccess && t.D > 1) e = run_pass(false, 2, t, planes, dst, nullptr, nullptr, false, 1.f, st);
-  return e;
-}
-
-// Unnormalised inverse transform of complex planes; the real part times
-// `scale` is stored into (or added to) dst.
-cudaError_t inverse_real(const NdTab& t, long planes, float2* data, float* dst, bool accumulate, float scale,
-                         cudaStream_t st) {
-  cudaError_t e = cudaSuccess;
-  if (t.D > 1) e = run_pass(true, 2, t, planes, data, nullptr, nullptr, false, 1.f, st);
-  if (e != cudaSuccess) return e;
-  if (plane_ok(t)) return run_plane(true, t, planes, data, nullptr, dst, accumulate, scale, st);
-  e = run_pass(true, 1, t, planes, data, nullptr, nullptr, false, 1.f, st);
-  if (e == cudaSuccess) e = run_pass(true, 0, t, planes, data, nullptr, dst, accumulate, scale, st);
-  return e;
-}
-
-// ------------------------------------------------------------------ spectra
-// Prepared spectra: the Hermitian half [planes, D, H, W/2+1] extended to the
-// full spectrum [planes, D, H, W] and scaled by 1/cells (the inverse passes
-// are unnormalised).
-__global__ void nd_prepare_kernel(long planes, int D, int H, int W, float scale, const float2* __restrict__ kh,
-                                  float2* __restrict__ kf) {
-  const int HWH = W / 2 + 1;
-  const long cells = (long)D * H * W, total = planes * cells;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const long pl = i / cells;
-    long r = i - pl * cells;
-    const int x = (int)(r % W);
-    r /= W;
-    const int y = (int)(r % H), z = (int)(r / H);
-    float2 v;
-    if (x < HWH) {
-      v = kh[((pl * D + z) * H + y) * HWH + x];
-    } else {  // K[z, y, x] = conj(K[-z, -y, W - x])
-      const int zz = z == 0 ? 0 : D - z, yy = y == 0 ? 0 : H - y;
-      const float2 c = kh[((pl * D + zz) * H + yy) * HWH + (W - x)];
-      v = make_float2(c.x, -c.y);
-    }
-    kf[i] = make_float2(v.x * scale, v.y * scale);
-  }
-}
-
-// Hermitian half of full spectra: [planes, D, H, W] -> [planes, D, H, W/2+1].
-__global__ void nd_half_kernel(long planes, int D, int H, int W, const float2* __restrict__ full,
-                               float2* __restrict__ half) {
-  const int HWH = W / 2 + 1;
-  const long rows = planes * D * H, total = rows * HWH;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const long row = i / HWH;
-    const int x = (int)(i - row * HWH);
-    half[i] = full[row * W + x];
-  }
 }
 
 inline int grid_for(long total) { return (int)std::max(1L, std::min<long>((total + kNT - 1) / kNT, 1L << 16)); }
 
-// ------------------------------------------------------------------ separate last-axis passes
-// For worlds whose fused-pass tile set does not fit (long last axes with many
-// channels): the last forward axis, these products, then the first inverse
-// axis run as three launches.
-// P[w, k] = S[w, c_in(k)] * prepared[sol(w), c_in(k), slot(k)]
-__global__ void nd_multiply_kernel(NdTab t, int n_worlds, int n_init, const float2* __restrict__ S,
-                                   const float2* __restrict__ kf, long kf_sol_stride, float2* __restrict__ P) {
-  const long total = (long)n_worlds * t.K * t.cells;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const long cell = i % t.cells;
-    const long wk = i / t.cells;
-    const int k = (int)(wk % t.K), w = (int)(wk / t.K);
-    const int sol = w / n_init, c = t.cin[k];
-    const float2 s = S[((long)w * t.C + c) * t.cells + cell];
-    const float2 kk = __ldg(kf + sol * kf_sol_stride + ((long)c * t.max_k + t.slot[k]) * t.cells + cell);
-    P[i] = cmul(s, kk);
-  }
+// ------------------------------------------------------------------ transforms
+const LineAxis& last_axis(const NdTab& t, const NdAxes& ax) { return t.nd == 3 ? ax.z : ax.y; }
+
+// Every axis but the last: real planes -> half spectra, and back (the result
+// times `scale` stored into dst or added to it; half is overwritten when the
+// y transforms are a pass of their own).
+cudaError_t forward_head(const NdTab& t, const NdAxes& ax, long planes, const float* src, float2* half,
+                         cudaStream_t st) {
+  if (nd_plane_ok(t, ax)) return nd_plane_forward(t, ax, planes, src, half, st);
+  const cudaError_t e = nd_rows_forward(ax.x, planes, t.D * t.H, src, half, st);
+  return e == cudaSuccess && t.D > 1 ? nd_columns(false, t, ax.y, planes, half, st) : e;
 }
-
-// gk[w, k] += A_k conj(S_cin(k)) (kernel gradient), Q[w, c] = sum_{k: c_in(k)
-// = c} A_k conj(prepared K_k)
-__global__ void nd_adj_spectral_kernel(NdTab t, int n_worlds, int n_init, const float2* __restrict__ A,
-                                       const float2* __restrict__ S, const float2* __restrict__ kf,
-                                       long kf_sol_stride, float2* __restrict__ gk, float2* __restrict__ Q) {
-  const long total = (long)n_worlds * t.cells;
-  const int C = t.C, K = t.K;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int w = (int)(i / t.cells);
-    const long cell = i - (long)w * t.cells;
-    const int sol = w / n_init;
-    float2 q[kMaxChannels];
-#pragma unroll
-    for (int c = 0; c < kMaxChannels; ++c) q[c] = make_float2(0.f, 0.f);
-    for (int k = 0; k < K; ++k) {
-      const int c = t.cin[k];
-      const float2 ak = A[((long)w * K + k) * t.cells + cell];
-      const float2 sc = S[((long)w * C + c) * t.cells + cell];
-      float2* g = gk + ((long)w * K + k) * t.cells + cell;
-      *g = cadd(*g, cmulc(ak, sc));
-      const float2 kk = __ldg(kf + sol * kf_sol_stride + ((long)c * t.max_k + t.slot[k]) * t.cells + cell);
-      const float2 pr = cmulc(ak, kk);
-#pragma unroll
-      for (int cc = 0; cc < kMaxChannels; ++cc)
-        if (cc == c) q[cc] = cadd(q[cc], pr);
-    }
-#pragma unroll
-    for (int c = 0; c < kMaxChannels; ++c) {
-      if (c >= C) break;
-      Q[((long)w * C + c) * t.cells + cell] = q[c];
-    }
-  }
+cudaError_t inverse_tail(const NdTab& t, const NdAxes& ax, long planes, float2* half, float* dst, bool accumulate,
+                         float scale, cudaStream_t st) {
+  if (nd_plane_ok(t, ax)) return nd_plane_inverse(t, ax, planes, half, dst, accumulate, scale, st);
+  const cudaError_t e = t.D > 1 ? nd_columns(true, t, ax.y, planes, half, st) : cudaSuccess;
+  return e == cudaSuccess ? nd_rows_inverse(ax.x, planes, t.D * t.H, half, dst, accumulate, scale, st) : e;
 }
-
-// ------------------------------------------------------------------ fused convolution pass
-// Along the last world axis (z in 3D, y in 2D) line i of a plane holds the
-// points i + j I, j < L, with I = cells / L lines per plane.  One block takes
-// a tile of nl adjacent lines of one world: the forward transform along the
-// axis of each channel, the spectrum products, the inverse transform of each
-// product -- the last forward pass, the multiply and the first inverse pass
-// in one launch, with the channel spectra kept in shared memory.  The
-// arithmetic is that of the separate passes, in the same order.
-struct ConvArgs {
-  int n_init, L, nl, tiles;  // points per line, lines per tile, tiles per plane
-  FastDivU fnl;               // division by nl
-  long I;                    // lines per plane (= point stride along the axis)
-  const float2* kf;          // prepared full spectra [Ns, C, max_k, cells]
-  long kf_sol_stride;
-  const float2* S;           // forward: [nw, C] planes, the other axes transformed
-  float2* P;                 // forward: [nw, K] product planes out
-  const float2* A;           // adjoint: [nw, K] planes of a = dL/du, the other axes transformed
-  float2* gk;                // adjoint: [nw, K] kernel-gradient spectra (accumulated)
-  float2* Q;                 // adjoint: [nw, C] correlation planes out
-};
-
-// nl lines of a plane (points src[l + j I]) into a line-major tile (lines
-// past `lines` read as zero); kLoadBatch loads in flight per thread
-__device__ __forceinline__ void load_lines(float2* dst, const float2* __restrict__ src, long I, int L, int nl,
-                                           FastDivU fnl, int lines) {
-  const int pts = nl * L;
-  constexpr int kLoadBatch = 8;
-  for (int base = threadIdx.x; base < pts; base += kLoadBatch * blockDim.x) {
-    float2 v[kLoadBatch];
-    int d[kLoadBatch];
-#pragma unroll
-    for (int u = 0; u < kLoadBatch; ++u) {
-      const int idx = base + u * blockDim.x;
-      const int j = fnl.div(idx), l = idx - j * nl;
-      d[u] = idx < pts ? l * L + j : -1;
-      v[u] = make_float2(0.f, 0.f);
-      if (idx < pts && l < lines) v[u] = src[l + (long)j * I];
-    }
-#pragma unroll
-    for (int u = 0; u < kLoadBatch; ++u)
-      if (d[u] >= 0) dst[d[u]] = v[u];
-  }
-}
-
-__device__ __forceinline__ void store_lines(float2* __restrict__ dst, const float2* src, long I, int L, int nl,
-                                            FastDivU fnl, int lines) {
-  for (int idx = threadIdx.x; idx < nl * L; idx += blockDim.x) {
-    const int j = fnl.div(idx), l = idx - j * nl;
-    if (l < lines) dst[l + (long)j * I] = src[l * L + j];
-  }
-}
-
-// forward: P[w, k] = IFFT_axis(FFT_axis(S[w, c_in(k)]) * prepared[sol, c_in(k), slot(k)])
-__global__ void __launch_bounds__(kNT) nd_conv_kernel(NdTab t, ConvArgs a, GPlan p) {
-  extern __shared__ __align__(16) float2 ndsm[];
-  const int L = a.L, nl = a.nl, pts = nl * L;
-  float2* tw = ndsm;
-  float2* Sc = tw + L;  // [C][pts] channel spectra along the axis
-  float2* A = Sc + (size_t)t.C * pts;
-  float2* B = A + pts;
-  const int w = blockIdx.x / a.tiles;
-  const long i0 = (long)(blockIdx.x % a.tiles) * nl;
-  const int lines = (int)min((long)nl, a.I - i0);
-  const int sol = w / a.n_init;
-  fill_twiddles(tw, L);
-  for (int c = 0; c < t.C; ++c) {
-    load_lines(A, a.S + ((long)w * t.C + c) * t.cells + i0, a.I, L, nl, a.fnl, lines);
-    __syncthreads();
-    const float2* r = fft_line<false>(A, B, p, tw, nl);
-    for (int x = threadIdx.x; x < pts; x += blockDim.x) Sc[c * pts + x] = r[x];
-    __syncthreads();
-  }
-  for (int k = 0; k < t.K; ++k) {
-    const int c = t.cin[k];
-    load_lines(A, a.kf + sol * a.kf_sol_stride + ((long)c * t.max_k + t.slot[k]) * t.cells + i0, a.I, L, nl, a.fnl, lines);
-    __syncthreads();
-    for (int x = threadIdx.x; x < pts; x += blockDim.x) A[x] = cmul(Sc[c * pts + x], A[x]);
-    __syncthreads();
-    const float2* r = fft_line<true>(A, B, p, tw, nl);
-    store_lines(a.P + ((long)w * t.K + k) * t.cells + i0, r, a.I, L, nl, a.fnl, lines);
-    __syncthreads();
-  }
-}
-
-// adjoint: with A_k = FFT(a_k), S_c = FFT(state_c) along the axis,
-// gk[w, k] += A_k conj(S_c_in(k)) and Q[w, c] = IFFT_axis(sum_{k: c_in(k) = c}
-// A_k conj(prepared_k)) -- the last forward passes of a and of the state, the
-// spectral products and the first inverse pass of Q in one launch
-__global__ void __launch_bounds__(kNT) nd_adj_conv_kernel(NdTab t, ConvArgs a, GPlan p) {
-  extern __shared__ __align__(16) float2 ndsm[];
-  const int L = a.L, nl = a.nl, pts = nl * L;
-  float2* tw = ndsm;
-  float2* Sc = tw + L;                    // [C][pts]
-  float2* Qc = Sc + (size_t)t.C * pts;    // [C][pts]
-  float2* A = Qc + (size_t)t.C * pts;
-  float2* B = A + pts;
-  const int w = blockIdx.x / a.tiles;
-  const long i0 = (long)(blockIdx.x % a.tiles) * nl;
-  const int lines = (int)min((long)nl, a.I - i0);
-  const int sol = w / a.n_init;
-  fill_twiddles(tw, L);
-  for (int c = 0; c < t.C; ++c) {
-    load_lines(A, a.S + ((long)w * t.C + c) * t.cells + i0, a.I, L, nl, a.fnl, lines);
-    __syncthreads();
-    const float2* r = fft_line<false>(A, B, p, tw, nl);
-    for (int x = threadIdx.x; x < pts; x += blockDim.x) {
-      Sc[c * pts + x] = r[x];
-      Qc[c * pts + x] = make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-  }
-  for (int k = 0; k < t.K; ++k) {
-    const int c = t.cin[k];
-    load_lines(A, a.A + ((long)w * t.K + k) * t.cells + i0, a.I, L, nl, a.fnl, lines);
-    __syncthreads();
-    const float2* r = fft_line<false>(A, B, p, tw, nl);
-    float2* o = r == A ? B : A;  // the free buffer takes the prepared spectrum's lines
-    load_lines(o, a.kf + sol * a.kf_sol_stride + ((long)c * t.max_k + t.slot[k]) * t.cells + i0, a.I, L, nl, a.fnl,
-               lines);
-    __syncthreads();
-    float2* g = a.gk + ((long)w * t.K + k) * t.cells + i0;
-    for (int idx = threadIdx.x; idx < pts; idx += blockDim.x) {
-      const int j = a.fnl.div(idx), l = idx - j * nl;
-      if (l >= lines) continue;
-      const int x = l * L + j;
-      const float2 ak = r[x];
-      float2* gp = g + l + (long)j * a.I;
-      *gp = cadd(*gp, cmulc(ak, Sc[c * pts + x]));
-      Qc[c * pts + x] = cadd(Qc[c * pts + x], cmulc(ak, o[x]));
-    }
-    __syncthreads();
-  }
-  for (int c = 0; c < t.C; ++c) {
-    for (int x = threadIdx.x; x < pts; x += blockDim.x) A[x] = Qc[c * pts + x];
-    __syncthreads();
-    const float2* r = fft_line<true>(A, B, p, tw, nl);
-    store_lines(a.Q + ((long)w * t.C + c) * t.cells + i0, r, a.I, L, nl, a.fnl, lines);
-    __syncthreads();
-  }
-}
-
-// Tile and shared memory of a fused convolution pass; `bufs` complex tiles
-// besides the twiddles (C + 2 forward, 2C + 2 adjoint).
-constexpr long kConvSmemPts = 96 * 1024 / 8;  // 96 KB of tiles: two blocks per SM
-// the largest tile set a fused pass may take; worlds whose one-line tile set
-// is larger (long last axes with many channels) take the separate passes
-constexpr int kConvSmemMax = 200 * 1024;
-
-// Lines per tile and shared memory of the fused pass along the last axis, or
-// 0 when even one line per tile does not fit.
-size_t conv_smem(const NdTab& t, bool adjoint, long nw, int* nl_out) {
-  const long L = t.nd == 3 ? t.D : t.H;
-  if (make_plan((int)L).stages == 0) return 0;  // Bluestein lines take the separate passes
-  const long I = t.cells / L;
-  const long bufs = adjoint ? 2L * t.C + 2 : (long)t.C + 2;
-  const long cap_pts = std::min<long>(kMaxPts, (kConvSmemPts - L) / bufs);
-  const long cap = std::max<long>(1, cap_pts / L);
-  const long fill = (nw * I + kFillBlocks - 1) / kFillBlocks;
-  const long nl = std::min<long>(std::min<long>(cap, std::max<long>(4, fill)), I);
-  const size_t smem = (size_t)(L + bufs * nl * L) * sizeof(float2);
-  if (nl_out) *nl_out = (int)nl;
-  return smem <= (size_t)kConvSmemMax ? smem : 0;
-}
-
-cudaError_t run_conv(bool adjoint, const NdTab& t, long nw, ConvArgs a, cudaStream_t st) {
-  a.L = t.nd == 3 ? t.D : t.H;
-  a.I = t.cells / a.L;
-  const GPlan p = make_plan(a.L);
-  if (p.stages == 0) return cudaErrorInvalidValue;
-  const size_t smem = conv_smem(t, adjoint, nw, &a.nl);
-  if (smem == 0) return cudaErrorInvalidConfiguration;
-  a.tiles = (int)((a.I + a.nl - 1) / a.nl);
-  a.fnl = make_fastdiv((unsigned)a.nl);
-  const long blocks = nw * a.tiles;
-  if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
-  cudaError_t e = allow_nd_smem();
-  if (e != cudaSuccess) return e;
-  if (adjoint) nd_adj_conv_kernel<<<(unsigned)blocks, kNT, smem, st>>>(t, a, p);
-  else nd_conv_kernel<<<(unsigned)blocks, kNT, smem, st>>>(t, a, p);
-  return cudaGetLastError();
-}
-
-
-// The axis passes before and after the fused one: forward x (real input)
-// and, in 3D, y; inverse y (3D) and x (real part out).
-cudaError_t forward_real_head(const NdTab& t, long planes, const float* src, float2* dst, cudaStream_t st) {
-  if (plane_ok(t)) return run_plane(false, t, planes, dst, src, nullptr, false, 1.f, st);
-  cudaError_t e = run_pass(false, 0, t, planes, dst, src, nullptr, false, 1.f, st);
-  if (e == cudaSuccess && t.D > 1) e = run_pass(false, 1, t, planes, dst, nullptr, nullptr, false, 1.f, st);
-  return e;
-}
-
-cudaError_t inverse_real_tail(const NdTab& t, long planes, float2* data, float* dst, bool accumulate, float scale,
-                              cudaStream_t st) {
-  if (plane_ok(t)) return run_plane(true, t, planes, data, nullptr, dst, accumulate, scale, st);
-  cudaError_t e = cudaSuccess;
-  if (t.D > 1) e = run_pass(true, 1, t, planes, data, nullptr, nullptr, false, 1.f, st);
-  if (e == cudaSuccess) e = run_pass(true, 0, t, planes, data, nullptr, dst, accumulate, scale, st);
-  return e;
-}
-
-// ------------------------------------------------------------------ forward epilogue
-struct EpiArgs {
-  int n_worlds, n_init, bpw;
-  const float* state;   // [nw, C, cells]
-  float* state_out;     // [nw, C, cells]
-  const float* pot;     // [nw, K, cells]
-  float* pot_out;       // [nw, K, cells] potential trajectory (fused plane epilogue), or null
-  const float* gf;      // [Ns, K, 2] (sol stride gf_sol_stride)
-  long gf_sol_stride;
-  const float* w;       // [Ns, C, K]
-  long w_sol_stride;
-  const float* dt;
-  float* field_out;     // [nw, C, cells] or null
-  float* state_copy;    // [nw, C, cells] copy of the entering state (trajectory), or null
-  int* shift;           // [nw, 3] read by every block, advanced by the world's last block
-  int* done;            // [nw] blocks finished this step (zero between steps)
-  float* partial;       // [nw, bpw, RAWS]
-  float* raw;           // the step's raw record, or null
-  long raw_sol_stride, raw_init_stride;
-};
-
-// per-cell centred coordinate on one axis (statistics.py:64-81 on the world
-// rolled by the carried shift): ((i - shift) mod n) - n // 2
-// (for 0 <= i, sh < n: a carried shift is always reduced mod n)
-__device__ __forceinline__ float centred_in(int i, int sh, int n) {
-  const int d = i - sh;
-  return (float)((d < 0 ? d + n : d) - n / 2);
-}
-
-// Per-thread statistics moments of one block of cells (statistics.py:64-100
-// in the centred frame), then the block's partial and, in the world's last
-// block, the step's raw record and the carried shift.
-struct Moments {
-  float m00 = 0.f, g00 = 0.f, cpot = 0.f, cmass = 0.f, cgrow = 0.f;
-  float mx0 = 0.f, mx1 = 0.f, mx2 = 0.f, gx0 = 0.f, gx1 = 0.f, gx2 = 0.f, q0 = 0.f, q1 = 0.f, q2 = 0.f;
-  float cm[kMaxChannels];
-  bool border = false;
-  __device__ Moments() {
-#pragma unroll
-    for (int c = 0; c < kMaxChannels; ++c) cm[c] = 0.f;
-  }
-  // one channel of one cell: entering state sv, field f, centred coordinates
-  __device__ __forceinline__ void add(int c, float sv, float f, float ca, float cb, float cc, bool edge) {
-    const float fp = fmaxf(f, 0.f);
-    m00 += sv;
-    g00 += fp;
-    cm[c] += sv;
-    mx0 = fmaf(ca, sv, mx0);
-    mx1 = fmaf(cb, sv, mx1);
-    mx2 = fmaf(cc, sv, mx2);
-    gx0 = fmaf(ca, fp, gx0);
-    gx1 = fmaf(cb, fp, gx1);
-    gx2 = fmaf(cc, fp, gx2);
-    q0 = fmaf(ca * ca, sv, q0);
-    q1 = fmaf(cb * cb, sv, q1);
-    q2 = fmaf(cc * cc, sv, q2);
-    const bool live = sv > kEps;
-    cmass += live ? 1.f : 0.f;
-    cgrow += fp > kEps ? 1.f : 0.f;
-    border |= live && edge;
-  }
-};
-
-// Block b of world w: reduce the threads' moments into the block's partial;
-// the world's last block to finish (a ticket on the world's counter; no block
-// waits) reduces all of the world's block partials in a fixed order into the
-// step's raw record (with the shift s0..s2 that centred it), then advances
-// the carried shift by the integer part of the centred-frame centroid
-// (statistics.py:117-124).  Every thread of the block calls it.
-__device__ __forceinline__ void epi_finish(const NdTab& t, const EpiArgs& a, int w, int b, int bpw, Moments& mo,
-                                           int s0, int s1, int s2) {
-  constexpr int NWARP = kNT / 32;
-  __shared__ float red[NWARP][kRawMax];
-  __shared__ int last;
-  __shared__ float tot[kRawMax];
-  const int C = t.C, nd = t.nd;
-  const int sol = w / a.n_init, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  float v[14] = {mo.m00, mo.g00, mo.cpot, mo.cmass, mo.cgrow, mo.mx0, mo.mx1,
-                 mo.mx2, mo.gx0, mo.gx1, mo.gx2, mo.q0,   mo.q1,   mo.q2};
-#pragma unroll
-  for (int i = 0; i < 14; ++i) v[i] = warp_sum(v[i]);
-  const bool anyb = __any_sync(0xffffffffu, mo.border);
-#pragma unroll
-  for (int c = 0; c < kMaxChannels; ++c) {
-    if (c >= C) break;
-    mo.cm[c] = warp_sum(mo.cm[c]);
-  }
-  if (lane == 0) {
-    float* rd = red[wid];
-    rd[RAW_M00] = v[0];
-    rd[RAW_G00] = v[1];
-    rd[RAW_CNT_POT] = v[2];
-    rd[RAW_CNT_MASS] = v[3];
-    rd[RAW_CNT_GROW] = v[4];
-    for (int i = 0; i < 3; ++i) {
-      rd[RAW_MX + i] = v[5 + i];
-      rd[RAW_GX + i] = v[8 + i];
-      rd[RAW_MX2 + i] = v[11 + i];
-    }
-    rd[RAW_BORDER] = anyb ? 1.f : 0.f;
-    for (int i = 0; i < 3; ++i) rd[RAW_SHIFT + i] = 0.f;
-    for (int c = 0; c < C; ++c) rd[RAW_CM + c] = mo.cm[c];
-  }
-  __syncthreads();
-  const int RAWS = raw_stride(C);
-  float* pw = a.partial + (long)w * bpw * RAWS;
-  if (threadIdx.x < RAWS) {
-    float s = 0.f;
-    for (int i = 0; i < NWARP; ++i) s += red[i][threadIdx.x];
-    if (threadIdx.x == RAW_BORDER) s = s > 0.f ? 1.f : 0.f;
-    pw[b * RAWS + threadIdx.x] = s;
-    __threadfence();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(a.done + w, 1) == bpw - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int s = lane; s < RAWS; s += 32) {
-    float acc = 0.f;
-    for (int bb = wid; bb < bpw; bb += NWARP) acc += __ldcg(pw + bb * RAWS + s);
-    red[wid][s] = acc;
-  }
-  __syncthreads();
-  if (threadIdx.x < RAWS) {
-    const int s = threadIdx.x;
-    float acc = 0.f;
-    for (int i = 0; i < NWARP; ++i) acc += red[i][s];
-    if (s == RAW_BORDER) acc = acc > 0.f ? 1.f : 0.f;
-    if (s == RAW_SHIFT) acc = (float)s0;
-    if (s == RAW_SHIFT + 1) acc = (float)s1;
-    if (s == RAW_SHIFT + 2) acc = (float)s2;
-    tot[s] = acc;
-    if (a.raw) a.raw[sol * a.raw_sol_stride + (w - sol * a.n_init) * a.raw_init_stride + s] = acc;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int n[3] = {nd == 2 ? t.H : t.D, nd == 2 ? t.W : t.H, t.W};
-    const int sh[3] = {s0, s1, s2};
-    for (int i = 0; i < nd; ++i) a.shift[3 * w + i] = pmod(sh[i] + (int)(tot[RAW_MX + i] / (tot[RAW_M00] + kEps)), n[i]);
-    a.done[w] = 0;
-  }
-}
-
-__device__ __forceinline__ float step_dt(const NdTab& t, const EpiArgs& a, int w, int sol) {
-  if (t.dt_mode == 0) return __ldg(a.dt);
-  if (t.dt_mode == 1) return __ldg(a.dt + w);
-  return 1.f / __ldg(a.dt + sol);
-}
-
-__global__ void __launch_bounds__(kNT, 3) nd_epilogue_kernel(NdTab t, EpiArgs a) {
-  const int w = blockIdx.x / a.bpw, b = blockIdx.x % a.bpw;
-  const int sol = w / a.n_init;
-  const int C = t.C, K = t.K;
-  const float* gf = a.gf + sol * a.gf_sol_stride;
-  const float* wt = a.w + sol * a.w_sol_stride;
-  const float dt = step_dt(t, a, w, sol);
-  const int nd = t.nd;
-  // axis order of the moments: 2D (y, x), 3D (z, y, x)
-  const int s0 = a.shift[3 * w], s1 = a.shift[3 * w + 1], s2 = a.shift[3 * w + 2];
-  const long chunk = (t.cells + a.bpw - 1) / a.bpw;
-  const long c0 = (long)b * chunk, c1 = min(t.cells, c0 + chunk);
-  Moments mo;
-  // (x, y, z) of the thread's cell, advanced by the block's stride of kNT
-  // cells with one carry per axis (no divisions inside the loop)
-  long cell = c0 + threadIdx.x;
-  int x = (int)(cell % t.W), y = (int)((cell / t.W) % t.H), z = (int)(cell / ((long)t.W * t.H));
-  const int sx = kNT % t.W, sy = (kNT / t.W) % t.H, sz = (int)(kNT / ((long)t.W * t.H));
-  for (; cell < c1; cell += kNT) {
-    float ca, cb, cc;  // centred coordinates along the moment axes
-    if (nd == 2) {
-      ca = centred_in(y, s0, t.H);
-      cb = centred_in(x, s1, t.W);
-      cc = 0.f;
-    } else {
-      ca = centred_in(z, s0, t.D);
-      cb = centred_in(y, s1, t.H);
-      cc = centred_in(x, s2, t.W);
-    }
-    const bool edge = x == 0 || x == t.W - 1 || y == 0 || y == t.H - 1 || (nd == 3 && (z == 0 || z == t.D - 1));
-    for (int k = 0; k < K; ++k) mo.cpot += __ldg(a.pot + ((long)w * K + k) * t.cells + cell) > kEps ? 1.f : 0.f;
-#pragma unroll
-    for (int c = 0; c < kMaxChannels; ++c) {
-      if (c >= C) break;
-      float f = 0.f, wsum = 0.f;
-      for (int k = 0; k < K; ++k) {
-        const float wk = __ldg(wt + c * K + k);
-        wsum += wk;
-        if (wk == 0.f) continue;
-        const float u = __ldg(a.pot + ((long)w * K + k) * t.cells + cell);
-        f = fmaf(wk, growth_fn(t.gf[k], u, __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1)), f);
-      }
-      if (t.mean) f = f / wsum;
-      const long off = ((long)w * C + c) * t.cells + cell;
-      const float sv = __ldg(a.state + off);
-      a.state_out[off] = state_fn(t.state_fn, sv, f, dt);
-      if (a.field_out) a.field_out[off] = f;
-      if (a.state_copy) a.state_copy[off] = sv;
-      mo.add(c, sv, f, ca, cb, cc, edge);
-    }
-    x += sx;
-    if (x >= t.W) {
-      x -= t.W;
-      ++y;
-    }
-    y += sy;
-    if (y >= t.H) {
-      y -= t.H;
-      ++z;
-    }
-    z += sz;
-  }
-  epi_finish(t, a, w, b, a.bpw, mo, s0, s1, s2);
-}
-
-// 3D worlds whose z-planes fit one tile: the inverse y and x transforms of
-// every kernel's product plane and the epilogue in one block per (world,
-// z-plane) -- the potentials never leave shared memory (they are stored
-// only as a requested trajectory).  Per channel the weighted field is
-// accumulated over the kernels in order, as in nd_epilogue_kernel, so the
-// results are the same.
-__global__ void __launch_bounds__(kNT, 3) nd_plane_epilogue_kernel(NdTab t, EpiArgs a, const float2* __restrict__ P,
-                                                                GPlan px, GPlan py, FastDivU wdiv) {
-  extern __shared__ __align__(16) float2 ndsm[];
-  const int H = t.H, W = t.W, D = t.D, pts = H * W;
-  const int C = t.C, K = t.K;
-  const int w = blockIdx.x / D, zp = blockIdx.x % D;
-  const int sol = w / a.n_init;
-  float2* twx = ndsm;
-  float2* twy = twx + W;
-  float2* A = twy + H;
-  float2* B = A + pts;
-  float* F = reinterpret_cast<float*>(B + pts);  // [C][pts] weighted fields
-  const float* gf = a.gf + sol * a.gf_sol_stride;
-  const float* wt = a.w + sol * a.w_sol_stride;
-  const float dt = step_dt(t, a, w, sol);
-  const int s0 = a.shift[3 * w], s1 = a.shift[3 * w + 1], s2 = a.shift[3 * w + 2];
-  const long pbase = (long)zp * pts;  // the plane's first cell
-  fill_twiddles(twx, W);
-  fill_twiddles(twy, H);
-  for (int i = threadIdx.x; i < C * pts; i += kNT) F[i] = 0.f;
-  Moments mo;
-  for (int k = 0; k < K; ++k) {
-    const float2* src = P + ((long)w * K + k) * t.cells + pbase;
-    constexpr int kLoadBatch = 8;
-    for (int b0 = threadIdx.x; b0 < pts; b0 += kLoadBatch * kNT) {
-      float2 v[kLoadBatch];
-#pragma unroll
-      for (int u = 0; u < kLoadBatch; ++u) {
-        const int idx = b0 + u * kNT;
-        v[u] = idx < pts ? src[idx] : make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < kLoadBatch; ++u) {
-        const int idx = b0 + u * kNT;
-        if (idx < pts) A[idx] = v[u];
-      }
-    }
-    __syncthreads();
-    float2* r = fft_cols<true>(A, B, py, twy, W, W, wdiv);
-    r = fft_line<true>(r, r == A ? B : A, px, twx, H);
-    const int id = t.gf[k];
-    const float m = __ldg(gf + 2 * k), sg = __ldg(gf + 2 * k + 1);
-    for (int idx = threadIdx.x; idx < pts; idx += kNT) {
-      const float u = r[idx].x;
-      if (a.pot_out) a.pot_out[((long)w * K + k) * t.cells + pbase + idx] = u;
-      mo.cpot += u > kEps ? 1.f : 0.f;
-      const float g = growth_fn(id, u, m, sg);
-      for (int c = 0; c < C; ++c) {
-        const float wk = __ldg(wt + c * K + k);
-        if (wk != 0.f) F[c * pts + idx] = fmaf(wk, g, F[c * pts + idx]);
-      }
-    }
-    __syncthreads();  // A and B are reloaded for the next kernel
-  }
-  float wsum[kMaxChannels];
-#pragma unroll
-  for (int c = 0; c < kMaxChannels; ++c) {
-    wsum[c] = 0.f;
-    if (c < C)
-      for (int k = 0; k < K; ++k) wsum[c] += __ldg(wt + c * K + k);
-  }
-  const float ca = centred_in(zp, s0, D);
-  const bool zedge = zp == 0 || zp == D - 1;
-  for (int idx = threadIdx.x; idx < pts; idx += kNT) {
-    const int y = wdiv.div(idx), x = idx - y * W;
-    const float cb = centred_in(y, s1, H), cc = centred_in(x, s2, W);
-    const bool edge = zedge || x == 0 || x == W - 1 || y == 0 || y == H - 1;
-#pragma unroll
-    for (int c = 0; c < kMaxChannels; ++c) {
-      if (c >= C) break;
-      float f = F[c * pts + idx];
-      if (t.mean) f = f / wsum[c];
-      const long off = ((long)w * C + c) * t.cells + pbase + idx;
-      const float sv = __ldg(a.state + off);
-      a.state_out[off] = state_fn(t.state_fn, sv, f, dt);
-      if (a.field_out) a.field_out[off] = f;
-      if (a.state_copy) a.state_copy[off] = sv;
-      mo.add(c, sv, f, ca, cb, cc, edge);
-    }
-  }
-  epi_finish(t, a, w, zp, D, mo, s0, s1, s2);
+// The last axis on its own, in place (the z or y lines of `planes` planes).
+cudaError_t last_pass(bool inv, const NdTab& t, const NdAxes& ax, long planes, float2* half, cudaStream_t st) {
+  NdTab flat = t;  // the last axis of a D x (H Wh) plane is the y axis of a one-plane world of H Wh columns
+  flat.D = 1;
+  flat.Wh = (int)(t.hcells / last_axis(t, ax).n);
+  return nd_columns(inv, flat, last_axis(t, ax), planes, half, st);
 }
 
 // ------------------------------------------------------------------ adjoint
@@ -1304,48 +452,10 @@ __global__ void nd_sum_inits_kernel(long per_sol, int n_sols, int n_init, const 
   }
 }
 
-cudaError_t allow_nd_smem() {
-  static std::mutex mu;
-  static std::vector<unsigned long long> done;  // contexts already set up
-  unsigned long long ctx = 0;
-  const bool known = current_context_id(&ctx);
-  if (known) {
-    std::lock_guard<std::mutex> lk(mu);
-    if (std::find(done.begin(), done.end(), ctx) != done.end()) return cudaSuccess;
-  }
-  // twiddles, two tiles and, for Bluestein lines, the chirp and its spectrum
-  const int pass_bytes = (int)((kNdMaxN + 2 * kMaxPts + kBluesteinMaxN + kMaxPts) * sizeof(float2));
-  cudaError_t e = cudaSuccess;
-  for (auto f : {nd_pass_kernel<false, false>, nd_pass_kernel<true, false>, nd_pass_kernel<false, true>,
-                 nd_pass_kernel<true, true>})
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, pass_bytes);
-  const int plane_bytes = (int)((2 * kMaxPts + 2 * kNdMaxN) * sizeof(float2));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(nd_plane_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, plane_bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(nd_plane_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, plane_bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(nd_plane_epilogue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kPlaneEpiSmemMax);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(nd_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmemMax);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(nd_adj_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmemMax);
-  if (e == cudaSuccess && known) {
-    std::lock_guard<std::mutex> lk(mu);
-    done.push_back(ctx);
-  }
-  return e;
-}
-
-inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
-
 }  // namespace
 
 // ---------------------------------------------------------------------- API
-bool nd_side_ok(int n) {
-  return n >= 2 && ((n <= kNdMaxN && make_plan(n).stages > 0) || bluestein_size(n) > 0);
-}
+bool nd_side_ok(int n) { return transform_len(n) > 0; }
 
 int nd_max_side() { return kNdMaxN; }
 
@@ -1357,80 +467,86 @@ bool nd_supported(const Model& m) {
   return true;
 }
 
-int nd_blocks_per_world(const Model& m, long n_worlds) {
-  // 16 cells per thread, or more blocks when the batch is too small to fill
-  // the GPU (at least one cell per thread, at most 256 blocks)
+namespace {
+
+// chunks of cells per world of the adjoint's pointwise kernel, and per
+// (world, kernel) of its parameter reduction: 16 cells per thread, or more
+// blocks when the batch is too small to fill the GPU (at least one cell per
+// thread, at most 256 blocks)
+int nd_param_blocks(const Model& m, long n_worlds) {
   const long by_cells = (m.cells + (long)kNT * 16 - 1) / ((long)kNT * 16);
   const long fill = (kFillBlocks + n_worlds - 1) / std::max(1L, n_worlds);
   const long useful = (m.cells + kNT - 1) / kNT;
   return (int)std::max(1L, std::min<long>(256, std::min(useful, std::max(by_cells, fill))));
 }
 
-namespace {
-// chunks of cells per world of the adjoint's pointwise kernel, and per
-// (world, kernel) of its parameter reduction
-int nd_param_blocks(const Model& m, long n_worlds) { return nd_blocks_per_world(m, n_worlds); }
+// Workspace of the steps of one call: tables, S, P, block partials, and the
+// weighted fields where they do not fit shared memory.
+struct StepLayout {
+  size_t tables, S, P, partial, field, end;
+};
+StepLayout step_layout(const Model& m, int n_worlds) {
+  const NdTab t = make_tab(m, 0);
+  const NdAxes ax = make_axes(m.D, m.H, m.W, nullptr);
+  const size_t nw = (size_t)n_worlds;
+  long field = 0;
+  int bpw = m.D;
+  if (!nd_plane_ok(t, ax)) bpw = nd_rows_epi_blocks(t, ax.x, (long)nw, &field);
+  else if (nd_plane_field_global(t, ax)) field = (long)m.D * ((m.H + 1) / 2) * m.W;
+  StepLayout L;
+  size_t off = 0;
+  L.tables = off;
+  off += table_bytes(m.D, m.H, m.W);
+  L.S = off;
+  off += al256(nw * m.C * t.hcells * sizeof(float2));
+  L.P = off;
+  off += al256(nw * m.K * t.hcells * sizeof(float2));
+  L.partial = off;
+  off += al256(nw * bpw * raw_stride(m.C) * sizeof(float));
+  L.field = off;
+  off += al256(nw * m.C * field * sizeof(float2));
+  L.end = off;
+  return L;
+}
+
 }  // namespace
 
-size_t nd_step_workspace_bytes(const Model& m, int n_worlds) {
-  const size_t nw = (size_t)n_worlds, cells = (size_t)m.cells;
-  return al256(nw * m.C * cells * sizeof(float2)) + al256(nw * m.K * cells * sizeof(float2)) +
-         al256(nw * m.K * cells * sizeof(float)) +
-         al256(nw * std::max(nd_blocks_per_world(m, (long)nw), m.D) * raw_stride(m.C) * sizeof(float));
-}
+size_t nd_step_workspace_bytes(const Model& m, int n_worlds) { return step_layout(m, n_worlds).end; }
 
-size_t nd_prepared_bytes(const Model& m, int n_sols) {
-  return al256((size_t)n_sols * m.C * m.max_k * m.cells * sizeof(float2));
-}
-
-cudaError_t launch_nd_prepare(const Model& m, int n_sols, const float2* k_half, float2* kf, cudaStream_t st) {
-  const long planes = (long)n_sols * m.C * m.max_k;
-  nd_prepare_kernel<<<grid_for(planes * m.cells), kNT, 0, st>>>(planes, m.D, m.H, m.W, 1.f / (float)m.cells, k_half,
-                                                                kf);
-  return cudaGetLastError();
+cudaError_t launch_nd_begin(const Model& m, void* ws, cudaStream_t st) {
+  return launch_tables(make_axes(m.D, m.H, m.W, ws), m.D, st);
 }
 
 cudaError_t launch_nd_step(const NdStep& s, cudaStream_t st) {
   const Model& m = *s.m;
   const NdTab t = make_tab(m, s.dt_mode);
-  const size_t nw = (size_t)s.n_worlds, cells = (size_t)m.cells;
-  const int bpw = nd_blocks_per_world(m, (long)nw);
-  char* p = static_cast<char*>(s.ws);
-  float2* S = reinterpret_cast<float2*>(p);
-  p += al256(nw * m.C * cells * sizeof(float2));
-  float2* P = reinterpret_cast<float2*>(p);
-  p += al256(nw * m.K * cells * sizeof(float2));
-  float* U = reinterpret_cast<float*>(p);
-  p += al256(nw * m.K * cells * sizeof(float));
-  float* partial = reinterpret_cast<float*>(p);
-  float* pot = s.pot_out ? s.pot_out : U;
-  cudaError_t e = forward_real_head(t, (long)nw * m.C, s.state, S, st);
-  if (e != cudaSuccess) return e;
-  const int last = t.nd == 3 ? 2 : 1;  // the last world axis
-  if (conv_smem(t, false, (long)nw, nullptr) > 0) {
-    ConvArgs ca{};
-    ca.n_init = s.n_init;
-    ca.kf = s.kf;
-    ca.kf_sol_stride = s.kf_sol_stride;
-    ca.S = S;
-    ca.P = P;
-    if ((e = run_conv(false, t, (long)nw, ca, st)) != cudaSuccess) return e;
-  } else {
-    if ((e = run_pass(false, last, t, (long)nw * m.C, S, nullptr, nullptr, false, 1.f, st)) != cudaSuccess) return e;
-    nd_multiply_kernel<<<grid_for((long)nw * m.K * cells), kNT, 0, st>>>(t, s.n_worlds, s.n_init, S, s.kf,
-                                                                          s.kf_sol_stride, P);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = run_pass(true, last, t, (long)nw * m.K, P, nullptr, nullptr, false, 1.f, st)) != cudaSuccess) return e;
-  }
-  const bool fused = plane_epi_smem(t) > 0;
-  if (!fused && (e = inverse_real_tail(t, (long)nw * m.K, P, pot, false, 1.f, st)) != cudaSuccess) return e;
-  EpiArgs a;
+  const StepLayout L = step_layout(m, s.n_worlds);
+  char* base = static_cast<char*>(s.ws);
+  const NdAxes ax = make_axes(m.D, m.H, m.W, base + L.tables);
+  const long nw = s.n_worlds;
+  float2* S = reinterpret_cast<float2*>(base + L.S);
+  float2* P = reinterpret_cast<float2*>(base + L.P);
+  const bool plane = nd_plane_ok(t, ax);
+  cudaError_t e;
+  if (!s.spec_ready && (e = forward_head(t, ax, nw * m.C, s.state, S, st)) != cudaSuccess) return e;
+  ConvArgs ca{};
+  ca.n_init = s.n_init;
+  ca.kh = s.k_half;
+  ca.kh_sol_stride = s.k_sol_stride;
+  ca.S = S;
+  ca.P = P;
+  if ((e = nd_convolve(false, t, last_axis(t, ax), nw, ca, st)) != cudaSuccess) return e;
+  const bool columns = t.D > 1 && !plane;  // the y transforms are passes of their own
+  if (columns && (e = nd_columns(true, t, ax.y, nw * m.K, P, st)) != cudaSuccess) return e;
+  EpiArgs a{};
   a.n_worlds = s.n_worlds;
   a.n_init = s.n_init;
-  a.bpw = bpw;
   a.state = s.state;
   a.state_out = s.state_out;
-  a.pot = pot;
+  a.P = P;
+  a.S = s.emit_spec ? S : nullptr;
+  a.F = reinterpret_cast<float*>(base + L.field);
+  a.pot_out = s.pot_out;
   a.gf = s.gf;
   a.gf_sol_stride = s.gf_sol_stride;
   a.w = s.w;
@@ -1440,61 +556,71 @@ cudaError_t launch_nd_step(const NdStep& s, cudaStream_t st) {
   a.state_copy = s.state_copy;
   a.shift = s.shift;
   a.done = s.done;
-  a.partial = partial;
+  a.partial = reinterpret_cast<float*>(base + L.partial);
   a.raw = s.raw;
   a.raw_sol_stride = s.raw_sol_stride;
   a.raw_init_stride = s.raw_world_stride;
-  a.pot_out = s.pot_out;
-  if (fused) {
-    if ((e = allow_nd_smem()) != cudaSuccess) return e;
-    a.bpw = m.D;
-    nd_plane_epilogue_kernel<<<(unsigned)(nw * m.D), kNT, plane_epi_smem(t), st>>>(
-        t, a, P, make_plan(m.W), make_plan(m.H), make_fastdiv((unsigned)m.W));
-  } else {
-    nd_epilogue_kernel<<<(unsigned)(nw * bpw), kNT, 0, st>>>(t, a);
-  }
-  return cudaGetLastError();
+  a.scale = 1.f / (float)m.cells;
+  e = plane ? nd_plane_epilogue(t, ax, a, st) : nd_rows_epilogue(t, ax.x, a, st);
+  if (e == cudaSuccess && columns && s.emit_spec) e = nd_columns(false, t, ax.y, nw * m.C, S, st);
+  return e;
 }
 
-size_t nd_adjoint_workspace_bytes(const Model& m, int n_sols, int n_init) {
+namespace {
+struct AdjLayout {
+  size_t tables, A, Q, ar, bf, ff, lam, pacc, end;
+};
+AdjLayout adj_layout(const Model& m, int n_sols, int n_init) {
+  const NdTab t = make_tab(m, 2);
   const size_t nw = (size_t)n_sols * n_init, cells = (size_t)m.cells, KC = (size_t)(m.K + m.C);
-  return nd_prepared_bytes(m, n_sols) + al256(nw * KC * cells * sizeof(float2)) +  // kf, [A | S]
-         al256(nw * m.C * cells * sizeof(float2)) +                                // Q
-         al256(nw * KC * cells * sizeof(float)) +                                  // [a | state copy]
-         3 * al256(nw * m.C * cells * sizeof(float)) +                             // bf, ff, lambda ping-pong
-         al256(nw * m.K * nd_param_blocks(m, (long)nw) * (2 + m.C) * sizeof(float));  // parameter partials
+  AdjLayout L;
+  size_t off = 0;
+  L.tables = off;
+  off += table_bytes(m.D, m.H, m.W);
+  L.A = off;  // spectra of the K planes of a, then of the C planes of the state
+  off += al256(nw * KC * t.hcells * sizeof(float2));
+  L.Q = off;
+  off += al256(nw * m.C * t.hcells * sizeof(float2));
+  L.ar = off;  // a, then the state copy: one real input for the head passes
+  off += al256(nw * KC * cells * sizeof(float));
+  L.bf = off;
+  off += al256(nw * m.C * cells * sizeof(float));
+  L.ff = off;
+  off += al256(nw * m.C * cells * sizeof(float));
+  L.lam = off;
+  off += al256(nw * m.C * cells * sizeof(float));
+  L.pacc = off;
+  off += al256(nw * m.K * nd_param_blocks(m, (long)nw) * (2 + m.C) * sizeof(float));
+  L.end = off;
+  return L;
 }
+}  // namespace
+
+size_t nd_adjoint_workspace_bytes(const Model& m, int n_sols, int n_init) { return adj_layout(m, n_sols, n_init).end; }
 
 size_t nd_kernel_grad_acc_bytes(const Model& m, int n_sols, int n_init) {
-  return (size_t)n_sols * n_init * m.K * m.cells * sizeof(float2);
+  return (size_t)n_sols * n_init * m.K * m.D * m.H * (m.W / 2 + 1) * sizeof(float2);
 }
 
 cudaError_t launch_nd_adjoint(const Model& m, const NdAdjoint& j, void* ws, cudaStream_t st) {
   const NdTab t = make_tab(m, 2);
+  const AdjLayout L = adj_layout(m, j.n_sols, j.n_init);
   const int nw = j.n_sols * j.n_init;
   const size_t cells = (size_t)m.cells;
-  char* p = static_cast<char*>(ws);
-  float2* kf = reinterpret_cast<float2*>(p);
-  p += nd_prepared_bytes(m, j.n_sols);
+  char* base = static_cast<char*>(ws);
+  const NdAxes ax = make_axes(m.D, m.H, m.W, base + L.tables);
   const size_t KC = (size_t)(m.K + m.C);
-  float2* A = reinterpret_cast<float2*>(p);  // the K planes of a, then the C planes of the state
-  float2* S = A + (size_t)nw * m.K * cells;
-  p += al256((size_t)nw * KC * cells * sizeof(float2));
-  float2* Q = reinterpret_cast<float2*>(p);
-  p += al256((size_t)nw * m.C * cells * sizeof(float2));
-  float* ar = reinterpret_cast<float*>(p);  // a, then the state copy: one real input for the head passes
-  p += al256((size_t)nw * KC * cells * sizeof(float));
-  float* bf = reinterpret_cast<float*>(p);
-  p += al256((size_t)nw * m.C * cells * sizeof(float));
-  float* ff = reinterpret_cast<float*>(p);
-  p += al256((size_t)nw * m.C * cells * sizeof(float));
-  float* lam_tmp = reinterpret_cast<float*>(p);
-  p += al256((size_t)nw * m.C * cells * sizeof(float));
-  float* pacc = reinterpret_cast<float*>(p);
-  const long kf_sol = (long)m.C * m.max_k * m.cells;
+  float2* A = reinterpret_cast<float2*>(base + L.A);
+  float2* S = A + (size_t)nw * m.K * t.hcells;
+  float2* Q = reinterpret_cast<float2*>(base + L.Q);
+  float* ar = reinterpret_cast<float*>(base + L.ar);
+  float* bf = reinterpret_cast<float*>(base + L.bf);
+  float* ff = reinterpret_cast<float*>(base + L.ff);
+  float* lam_tmp = reinterpret_cast<float*>(base + L.lam);
+  float* pacc = reinterpret_cast<float*>(base + L.pacc);
   const int pb = nd_param_blocks(m, nw);
   const bool fused = m.K == 1 && m.C == 1;  // parameter partials inside the pointwise kernel
-  cudaError_t e = launch_nd_prepare(m, j.n_sols, j.k_half, kf, st);
+  cudaError_t e = launch_tables(ax, m.D, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(pacc, 0, (size_t)nw * m.K * pb * (2 + m.C) * sizeof(float), st);
   if (e != cudaSuccess) return e;
   const size_t plane_c = (size_t)m.C * cells, plane_k = (size_t)m.K * cells;
@@ -1527,25 +653,17 @@ cudaError_t launch_nd_adjoint(const Model& m, const NdAdjoint& j, void* ws, cuda
                                                                        j.weights, pacc);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    if ((e = forward_real_head(t, (long)nw * KC, ar, A, st)) != cudaSuccess) return e;
-    if (conv_smem(t, true, (long)nw, nullptr) > 0) {
-      ConvArgs ca{};
-      ca.n_init = j.n_init;
-      ca.kf = kf;
-      ca.kf_sol_stride = kf_sol;
-      ca.S = S;
-      ca.A = A;
-      ca.gk = j.gk;
-      ca.Q = Q;
-      if ((e = run_conv(true, t, (long)nw, ca, st)) != cudaSuccess) return e;
-    } else {
-      const int last = t.nd == 3 ? 2 : 1;
-      if ((e = run_pass(false, last, t, (long)nw * KC, A, nullptr, nullptr, false, 1.f, st)) != cudaSuccess) return e;
-      nd_adj_spectral_kernel<<<grid_for((long)nw * cells), kNT, 0, st>>>(t, nw, j.n_init, A, S, kf, kf_sol, j.gk, Q);
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      if ((e = run_pass(true, last, t, (long)nw * m.C, Q, nullptr, nullptr, false, 1.f, st)) != cudaSuccess) return e;
-    }
-    if ((e = inverse_real_tail(t, (long)nw * m.C, Q, lam_out, true, 1.f, st)) != cudaSuccess) return e;
+    if ((e = forward_head(t, ax, (long)nw * KC, ar, A, st)) != cudaSuccess) return e;
+    ConvArgs ca{};
+    ca.n_init = j.n_init;
+    ca.kh = j.k_half;
+    ca.kh_sol_stride = (long)m.C * m.max_k * t.hcells;
+    ca.S = S;
+    ca.A = A;
+    ca.gk = j.gk;
+    ca.Q = Q;
+    if ((e = nd_convolve(true, t, last_axis(t, ax), nw, ca, st)) != cudaSuccess) return e;
+    if ((e = inverse_tail(t, ax, (long)nw * m.C, Q, lam_out, true, 1.f / (float)m.cells, st)) != cudaSuccess) return e;
     lam_in = lam_out;
   }
   nd_param_reduce_kernel<<<grid_for((long)j.n_sols * (2 * m.K + m.C * m.K)), kNT, 0, st>>>(
@@ -1554,25 +672,27 @@ cudaError_t launch_nd_adjoint(const Model& m, const NdAdjoint& j, void* ws, cuda
 }
 
 size_t nd_kernel_grad_workspace_bytes(const Model& m, int n_sols) {
-  return al256((size_t)n_sols * m.K * m.cells * sizeof(float2));
+  return table_bytes(m.D, m.H, m.W) + al256((size_t)n_sols * m.K * m.D * m.H * (m.W / 2 + 1) * sizeof(float2));
 }
 
 cudaError_t launch_nd_kernel_grad(const Model& m, int n_sols, int n_init, const float2* gk, float* out, void* ws,
                                   cudaStream_t st) {
   const NdTab t = make_tab(m, 2);
-  float2* gsum = static_cast<float2*>(ws);
-  const long per = (long)m.K * m.cells;
-  nd_sum_inits_kernel<<<grid_for((long)n_sols * per), kNT, 0, st>>>(per, n_sols, n_init, gk, gsum);
-  cudaError_t e = cudaGetLastError();
+  const NdAxes ax = make_axes(m.D, m.H, m.W, ws);
+  float2* gsum = reinterpret_cast<float2*>(static_cast<char*>(ws) + table_bytes(m.D, m.H, m.W));
+  cudaError_t e = launch_tables(ax, m.D, st);
   if (e != cudaSuccess) return e;
+  const long per = (long)m.K * t.hcells, planes = (long)n_sols * m.K;
+  nd_sum_inits_kernel<<<grid_for((long)n_sols * per), kNT, 0, st>>>(per, n_sols, n_init, gk, gsum);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   // dL/dk = Re(IFFT(sum_t A_t conj(S_t))) = unnormalised inverse / cells
-  return inverse_real(t, (long)n_sols * m.K, gsum, out, false, 1.f / (float)m.cells, st);
+  if ((e = last_pass(true, t, ax, planes, gsum, st)) != cudaSuccess) return e;
+  return inverse_tail(t, ax, planes, gsum, out, false, 1.f / (float)m.cells, st);
 }
 
 size_t nd_spectrum_workspace_bytes(int nb_dims, const int* world, int planes) {
-  long cells = 1;
-  for (int i = 0; i < nb_dims; ++i) cells *= world[i];
-  return al256((size_t)planes * cells * sizeof(float2));
+  (void)planes;
+  return table_bytes(nb_dims == 3 ? world[0] : 1, world[nb_dims - 2], world[nb_dims - 1]);
 }
 
 cudaError_t launch_nd_spectrum(int nb_dims, const int* world, int planes, const float* k_real, float2* k_half,
@@ -1588,12 +708,10 @@ cudaError_t launch_nd_spectrum(int nb_dims, const int* world, int planes, const 
   m.state_fn = 0;
   m.cin[0] = m.slot[0] = m.gf[0] = 0;
   const NdTab t = make_tab(m, 0);
-  float2* full = static_cast<float2*>(ws);
-  cudaError_t e = forward_real(t, planes, k_real, full, st);
-  if (e != cudaSuccess) return e;
-  const long total = (long)planes * m.D * m.H * (m.W / 2 + 1);
-  nd_half_kernel<<<grid_for(total), kNT, 0, st>>>(planes, m.D, m.H, m.W, full, k_half);
-  return cudaGetLastError();
+  const NdAxes ax = make_axes(m.D, m.H, m.W, ws);
+  cudaError_t e = launch_tables(ax, m.D, st);
+  if (e == cudaSuccess) e = forward_head(t, ax, planes, k_real, k_half, st);
+  return e == cudaSuccess ? last_pass(false, t, ax, planes, k_half, st) : e;
 }
 
 }  // namespace lgx

@@ -1,0 +1,391 @@
+// Shared pieces of the general N-D engine (nd.cu, nd_rows.cu, nd_plane.cu,
+// nd_conv.cu): the model table, tile geometry and the epilogue of an Euler
+// step (growth, weighted field, state update, statistics moments).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "engine.h"
+#include "line_fft.cuh"
+
+namespace lgx {
+
+constexpr int kNdThreads = 320;        // most threads of a transform block
+constexpr int kNdBlocksPerSm = 3;      // register budget: 64 a thread
+constexpr int kNdMaxN = 4096;          // longest world axis (one 4096-point line per tile)
+constexpr int kBluesteinMaxN = 2048;   // longest axis with a prime factor above 7 (m <= 4096)
+constexpr int kMaxPts = 4096;          // complex points of one tile buffer
+constexpr int kMaxTileLines = 64;
+constexpr int kNdSmemMax = 227 * 1024;
+// Launches smaller than this many blocks (two on each of GB300's 152 SMs) get
+// smaller tiles so that one small world still spreads over the whole GPU.
+constexpr long kFillBlocks = 2 * 152;
+constexpr int kRawMax = RAW_CM + kMaxChannels;
+
+struct NdTab {  // kernel table and geometry of a model, passed by value
+  int C, K, max_k, mean, state_fn, dt_mode, nd;
+  int D, H, W, Wh;     // Wh = W / 2 + 1 columns of a half spectrum
+  long cells, hcells;  // D H W, D H Wh
+  int cin[kMaxKernels];
+  int slot[kMaxKernels];
+  int gf[kMaxKernels];
+};
+
+struct NdAxes {
+  LineAxis x, y, z;  // along W, H and D
+};
+
+inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// threads for `items` butterflies: one each up to kNdThreads, else whole rounds
+inline int nd_threads(long items) {
+  const long rounds = (items + kNdThreads - 1) / kNdThreads;
+  const long per = (items + rounds - 1) / std::max(1L, rounds);
+  return (int)std::min<long>(kNdThreads, std::max(32L, (per + 31) / 32 * 32));
+}
+// butterflies of an nl-line tile's widest end stage
+inline long line_items(const LineAxis& ax, int nl) {
+  const int last = ax.r[ax.stages - 1];
+  return (long)nl * (ax.m / std::min(ax.r[0], last > 1 ? last : ax.r[0]));
+}
+
+// Opt a kernel in to the full dynamic shared memory; the attribute belongs to
+// the CUDA context, so each context gets it once (nd.cu).
+cudaError_t nd_allow_smem(const void* kernel);
+
+// ------------------------------------------------------------------ epilogue
+struct EpiArgs {
+  int n_worlds, n_init, bpw;
+  const float* state;   // [nw, C, cells]
+  float* state_out;     // [nw, C, cells]
+  const float2* P;      // [nw, K, hcells] products, the last world axis inverse-transformed
+  float2* S;            // [nw, C, hcells] next step's row (2D) or plane (3D) spectra, or null
+  float* F;             // [nw, C, cells] weighted fields between the kernels when they do not fit shared memory
+  float* pot_out;       // [nw, K, cells] or null
+  const float* gf;      // [Ns, K, 2] (sol stride gf_sol_stride)
+  long gf_sol_stride;
+  const float* w;       // [Ns, C, K]
+  long w_sol_stride;
+  const float* dt;
+  float* field_out;     // [nw, C, cells] or null
+  float* state_copy;    // [nw, C, cells] copy of the entering state (trajectory), or null
+  int* shift;           // [nw, 3] read by every block, advanced by the world's last block
+  int* done;            // [nw] blocks finished this step (zero between steps)
+  float* partial;       // [nw, bpw, RAWS]
+  float* raw;           // the step's raw record, or null
+  long raw_sol_stride, raw_init_stride;
+  float scale;          // 1 / cells: the inverse transforms are unnormalised
+};
+
+// centred coordinate on one axis (statistics.py:64-81 on the world rolled by
+// the carried shift): ((i - shift) mod n) - n // 2, for 0 <= i, sh < n
+__device__ __forceinline__ float centred_in(int i, int sh, int n) {
+  const int d = i - sh;
+  return (float)((d < 0 ? d + n : d) - n / 2);
+}
+
+__device__ __forceinline__ float step_dt(const NdTab& t, const EpiArgs& a, int w, int sol) {
+  if (t.dt_mode == 0) return __ldg(a.dt);
+  if (t.dt_mode == 1) return __ldg(a.dt + w);
+  return 1.f / __ldg(a.dt + sol);
+}
+
+// Growth of one potential: the gaussian inline (the form of GrowthP: the
+// scale folds 1/s and sqrt(log2 e / 2)), the others out of line, so that an
+// unrolled butterfly's epilogue stays small.
+static __device__ __noinline__ float growth_any(int id, float u, float m, float s) { return growth_fn(id, u, m, s); }
+struct NdGrowth {
+  GrowthP p;
+  __device__ __forceinline__ NdGrowth(int id, float m, float s) {
+    p.id = id;
+    p.m = m;
+    p.s = s;
+    p.a = 0.84932180028801904272f / s;  // sqrt(log2(e) / 2) / s
+  }
+  __device__ __forceinline__ float operator()(float u) const {
+    if (p.id == LGX_GF_GAUSSIAN) return growth_cell<GF_FAST_GAUSSIAN>(p, u);
+    return growth_any(p.id, u, p.m, p.s);
+  }
+};
+
+// A packed pair of rows of a tile: row0 and, when the pair is whole, row0 + 1.
+struct RowPair {
+  long cell;         // first cell of row0 within the channel plane
+  float cz0, cy0, cz1, cy1;  // centred coordinates of the two rows
+  int rows;          // 0 (past the tile), 1 or 2
+  int edge;          // bit 0 / 1: the row lies on the outer layer of the un-centred world
+};
+
+__device__ __forceinline__ RowPair row_pair(const NdTab& t, int z0, int y0, int z1, int y1, int rows, int s0, int s1,
+                                            int s2) {
+  RowPair r;
+  r.cell = ((long)z0 * t.H + y0) * t.W;
+  r.rows = rows;
+  const int sz = t.nd == 3 ? s0 : 0, sy = t.nd == 3 ? s1 : s0;
+  r.cz0 = t.nd == 3 ? centred_in(z0, sz, t.D) : 0.f;
+  r.cz1 = t.nd == 3 ? centred_in(z1, sz, t.D) : 0.f;
+  r.cy0 = centred_in(y0, sy, t.H);
+  r.cy1 = centred_in(y1, sy, t.H);
+  const bool e0 = y0 == 0 || y0 == t.H - 1 || (t.nd == 3 && (z0 == 0 || z0 == t.D - 1));
+  const bool e1 = y1 == 0 || y1 == t.H - 1 || (t.nd == 3 && (z1 == 0 || z1 == t.D - 1));
+  r.edge = (e0 ? 1 : 0) | (e1 ? 2 : 0);
+  (void)s2;
+  return r;
+}
+
+// Per-thread statistics moments (statistics.py:64-100 in the centred frame).
+struct Moments {
+  float m00 = 0.f, g00 = 0.f, cpot = 0.f, cmass = 0.f, cgrow = 0.f;
+  float mz = 0.f, my = 0.f, mx = 0.f, gz = 0.f, gy = 0.f, gx = 0.f, qz = 0.f, qy = 0.f, qx = 0.f;
+  bool border = false;
+  // one cell of both rows of a pair: entering states, fields, centred x
+  __device__ __forceinline__ void add(const RowPair& r, float2 s, float2 f, float cx, bool xedge) {
+    const float2 g = make_float2(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
+    const float ss = s.x + s.y, gg = g.x + g.y;
+    m00 += ss;
+    g00 += gg;
+    mx = fmaf(ss, cx, mx);
+    qx = fmaf(ss * cx, cx, qx);
+    gx = fmaf(gg, cx, gx);
+    const float y0 = s.x * r.cy0, y1 = s.y * r.cy1, z0 = s.x * r.cz0, z1 = s.y * r.cz1;
+    my += y0 + y1;
+    mz += z0 + z1;
+    qy = fmaf(y0, r.cy0, fmaf(y1, r.cy1, qy));
+    qz = fmaf(z0, r.cz0, fmaf(z1, r.cz1, qz));
+    gy = fmaf(g.x, r.cy0, fmaf(g.y, r.cy1, gy));
+    gz = fmaf(g.x, r.cz0, fmaf(g.y, r.cz1, gz));
+    const bool l0 = s.x > kEps, l1 = s.y > kEps;
+    cmass += (l0 ? 1.f : 0.f) + (l1 ? 1.f : 0.f);
+    cgrow += (g.x > kEps ? 1.f : 0.f) + (g.y > kEps ? 1.f : 0.f);
+    border |= (l0 && (xedge || (r.edge & 1))) || (l1 && (xedge || (r.edge & 2)));
+  }
+  __device__ __forceinline__ void count_pot(float2 u, int rows) {
+    cpot += (u.x > kEps ? 1.f : 0.f) + (rows > 1 && u.y > kEps ? 1.f : 0.f);
+  }
+};
+
+struct EpiShared {
+  float red[kNdThreads / 32][kRawMax];
+  float tot[kRawMax];
+  int last;
+};
+
+// The warp's total of channel c's mass, kept for epi_finish.
+__device__ __forceinline__ void epi_channel_mass(EpiShared& sh, int c, float cm) {
+  cm = warp_sum(cm);
+  if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5][RAW_CM + c] = cm;
+}
+
+// The epilogue of the packed pairs of potentials in Z [nl][zp] (C = K = 1):
+// growth, state update, stores and moments, the new cells left in Z.  `lanes`
+// neighbouring threads take a row pair (the power of two that W wastes least
+// of), so the row coordinates multiply row sums and the cells of a pair go
+// through the packed FP32x2 pipe.  A rolled loop of its own rather than the
+// middle of the row transform's butterflies: inlined there it was unrolled
+// over every radix, and blocks that run the code once stalled on instruction
+// fetch.
+template <bool GAUSS, bool V1>
+__device__ __forceinline__ void epi_pairs(const NdTab& t, const EpiArgs& a, const RowPair* rp, float2* Z, int nl,
+                                          int zp, int lanes, int w, int sx, float dt, Moments& mo) {
+  const int W = t.W, sol = w / a.n_init;
+  const float* gf = a.gf + sol * a.gf_sol_stride;
+  const NdGrowth grow(t.gf[0], __ldg(gf), __ldg(gf + 1));
+  const float wk = __ldg(a.w + sol * a.w_sol_stride);
+  const float wf = t.mean ? wk / wk : wk;  // weighted_mean with one kernel: (w g) / w
+  const float wrap = (float)W, top = (float)(W - W / 2);
+  const int x0 = threadIdx.x & (lanes - 1);
+  const int per = __ffs(lanes) - 1;
+  float2 S2, G2;
+  for (int l = threadIdx.x >> per; l < nl; l += blockDim.x >> per) {
+    const RowPair r = rp[l];
+    if (r.rows == 0) continue;
+    const bool two = r.rows > 1;
+    const long off0 = (long)w * t.cells + r.cell;
+    S2 = G2 = make_float2(0.f, 0.f);
+    float2 most = make_float2(0.f, 0.f);  // largest cell of each row
+    bool lx = false;
+    float cx = centred_in(x0 < W ? x0 : 0, sx, W);
+    float2* z = Z + l * zp;
+    for (int x = x0; x < W; x += lanes) {
+      const long off = off0 + x;
+      const float2 s = make_float2(__ldg(a.state + off), two ? __ldg(a.state + off + W) : 0.f);
+      const float2 u = __fmul2_rn(z[x], make_float2(a.scale, a.scale));
+      float2 f;
+      if (GAUSS) f = weighted_growth2<GF_FAST_GAUSSIAN>(grow.p, u, wf);
+      else f = make_float2(grow(u.x) * wf, grow(u.y) * wf);
+      if (!two) f.y = 0.f;
+      float2 n;
+      if (V1) n = make_float2(__saturatef(fmaf(dt, f.x, s.x)), __saturatef(fmaf(dt, f.y, s.y)));
+      else n = make_float2(state_fn(t.state_fn, s.x, f.x, dt), state_fn(t.state_fn, s.y, f.y, dt));
+      z[x] = n;
+      a.state_out[off] = n.x;
+      if (two) a.state_out[off + W] = n.y;
+      if (a.field_out) {
+        a.field_out[off] = f.x;
+        if (two) a.field_out[off + W] = f.y;
+      }
+      if (a.state_copy) {
+        a.state_copy[off] = s.x;
+        if (two) a.state_copy[off + W] = s.y;
+      }
+      if (a.pot_out) {
+        a.pot_out[off] = u.x;
+        if (two) a.pot_out[off + W] = u.y;
+      }
+      mo.count_pot(u, r.rows);
+      const float2 g = make_float2(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
+      const float ss = s.x + s.y;
+      S2 = cadd(S2, s);
+      G2 = cadd(G2, g);
+      mo.mx = fmaf(ss, cx, mo.mx);
+      mo.qx = fmaf(ss * cx, cx, mo.qx);
+      mo.gx = fmaf(g.x + g.y, cx, mo.gx);
+      mo.cmass += (s.x > kEps ? 1.f : 0.f) + (s.y > kEps ? 1.f : 0.f);
+      mo.cgrow += (g.x > kEps ? 1.f : 0.f) + (g.y > kEps ? 1.f : 0.f);
+      most = make_float2(fmaxf(most.x, s.x), fmaxf(most.y, s.y));
+      if (x == 0 || x == W - 1) lx |= fmaxf(s.x, s.y) > kEps;
+      cx += (float)lanes;
+      while (cx >= top) cx -= wrap;  // past the centred frame's end
+    }
+    mo.border |= lx || (most.x > kEps && (r.edge & 1)) || (most.y > kEps && (r.edge & 2));
+    mo.m00 += S2.x + S2.y;
+    mo.g00 += G2.x + G2.y;
+    const float y0 = S2.x * r.cy0, y1 = S2.y * r.cy1, z0 = S2.x * r.cz0, z1 = S2.y * r.cz1;
+    mo.my += y0 + y1;
+    mo.mz += z0 + z1;
+    mo.qy = fmaf(y0, r.cy0, fmaf(y1, r.cy1, mo.qy));
+    mo.qz = fmaf(z0, r.cz0, fmaf(z1, r.cz1, mo.qz));
+    mo.gy = fmaf(G2.x, r.cy0, fmaf(G2.y, r.cy1, mo.gy));
+    mo.gz = fmaf(G2.x, r.cz0, fmaf(G2.y, r.cz1, mo.gz));
+  }
+}
+__device__ __forceinline__ void epi_single(const NdTab& t, const EpiArgs& a, const RowPair* rp, float2* Z, int nl,
+                                           int zp, int lanes, int w, int sx, float dt, Moments& mo) {
+  if (t.gf[0] == LGX_GF_GAUSSIAN && t.state_fn == LGX_STATE_V1)
+    epi_pairs<true, true>(t, a, rp, Z, nl, zp, lanes, w, sx, dt, mo);
+  else
+    epi_pairs<false, false>(t, a, rp, Z, nl, zp, lanes, w, sx, dt, mo);
+}
+// threads per row pair: the power of two in 8..32 that leaves the fewest idle
+inline int epi_lanes(int W) {
+  int best = 32;
+  for (int p : {16, 8})
+    if ((W + p - 1) / p * p < (W + best - 1) / best * best) best = p;
+  return best;
+}
+
+// Block b of world w: reduce the threads' moments into the block's partial;
+// the world's last block to finish (a ticket on the world's counter; no block
+// waits) reduces all of the world's block partials in a fixed order into the
+// step's raw record (with the shift s0..s2 that centred it), then advances
+// the carried shift by the integer part of the centred-frame centroid
+// (statistics.py:117-124).  Every thread of the block calls it, after
+// epi_channel_mass of every channel.
+__device__ __forceinline__ void epi_finish(const NdTab& t, const EpiArgs& a, EpiShared& sh, int w, int b,
+                                           const Moments& mo, int s0, int s1, int s2) {
+  const int NWARP = blockDim.x >> 5;
+  const int C = t.C, nd = t.nd, bpw = a.bpw;
+  const int sol = w / a.n_init, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // record order: 3D (z, y, x), 2D (y, x, 0)
+  const bool d3 = nd == 3;
+  float v[16] = {mo.m00, mo.g00, mo.cpot, mo.cmass, mo.cgrow,
+                 d3 ? mo.mz : mo.my, d3 ? mo.my : mo.mx, d3 ? mo.mx : 0.f,
+                 d3 ? mo.gz : mo.gy, d3 ? mo.gy : mo.gx, d3 ? mo.gx : 0.f,
+                 d3 ? mo.qz : mo.qy, d3 ? mo.qy : mo.qx, d3 ? mo.qx : 0.f, mo.border ? 1.f : 0.f, 0.f};
+  static_assert(RAW_M00 == 0 && RAW_G00 == 1 && RAW_CNT_POT == 2 && RAW_CNT_MASS == 3 && RAW_CNT_GROW == 4 &&
+                    RAW_MX == 5 && RAW_GX == 8 && RAW_MX2 == 11 && RAW_BORDER == 14 && RAW_SHIFT == 15,
+                "the order of v");
+  const float total = warp_sum16(v);  // lane L: value L >> 1
+  if ((lane & 1) == 0) sh.red[wid][lane >> 1] = total;  // slot 15 (shift) is written below
+  if (lane < 2) sh.red[wid][RAW_SHIFT + 1 + lane] = 0.f;
+  __syncthreads();
+  const int RAWS = raw_stride(C);
+  float* pw = a.partial + (long)w * bpw * RAWS;
+  for (int s = threadIdx.x; s < RAWS; s += blockDim.x) {
+    float acc = 0.f;
+    for (int i = 0; i < NWARP; ++i) acc += sh.red[i][s];
+    pw[(long)b * RAWS + s] = acc;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) sh.last = atomicAdd(a.done + w, 1) == bpw - 1;
+  __syncthreads();
+  if (!sh.last) return;
+  __threadfence();
+  for (int s = lane; s < RAWS; s += 32) {
+    float acc = 0.f;
+    for (int bb = wid; bb < bpw; bb += NWARP) acc += __ldcg(pw + (long)bb * RAWS + s);
+    sh.red[wid][s] = acc;
+  }
+  __syncthreads();
+  for (int s = threadIdx.x; s < RAWS; s += blockDim.x) {
+    float acc = 0.f;
+    for (int i = 0; i < NWARP; ++i) acc += sh.red[i][s];
+    if (s == RAW_BORDER) acc = acc > 0.f ? 1.f : 0.f;
+    if (s == RAW_SHIFT) acc = (float)s0;
+    if (s == RAW_SHIFT + 1) acc = (float)s1;
+    if (s == RAW_SHIFT + 2) acc = (float)s2;
+    sh.tot[s] = acc;
+    if (a.raw) a.raw[sol * a.raw_sol_stride + (w - sol * a.n_init) * a.raw_init_stride + s] = acc;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int n[3] = {nd == 2 ? t.H : t.D, nd == 2 ? t.W : t.H, t.W};
+    const int shf[3] = {s0, s1, s2};
+    for (int i = 0; i < nd; ++i)
+      a.shift[3 * w + i] = pmod(shf[i] + (int)(sh.tot[RAW_MX + i] / (sh.tot[RAW_M00] + kEps)), n[i]);
+    a.done[w] = 0;
+  }
+}
+
+// Point i of the packed inverse row transform: with row half spectra A and B
+// at column min(i, W - i), Z = A + i B for i < W/2 and conj(A) + i conj(B) past
+// it.  The real parts of the DC and Nyquist columns are what Re(IFFT) keeps.
+__device__ __forceinline__ float2 pack_rows(float2 a, float2 b, int i, int W) {
+  const float s = i == 0 || 2 * i == W ? 0.f : (2 * i > W ? -1.f : 1.f);
+  return make_float2(fmaf(-s, b.y, a.x), fmaf(s, a.y, b.x));
+}
+
+// Half spectra of two real rows from the transform Z of row0 + i row1, at
+// column k: (Z_k + conj Z_{W-k}) / 2 and (Z_k - conj Z_{W-k}) / 2i.
+__device__ __forceinline__ float2 unpack_row0(float2 zk, float2 zm) {
+  return make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+}
+__device__ __forceinline__ float2 unpack_row1(float2 zk, float2 zm) {
+  return make_float2(0.5f * (zk.y + zm.y), 0.5f * (zm.x - zk.x));
+}
+
+// ------------------------------------------------------------- launchers
+// nd_rows.cu.  `rows` rows of W cells per plane, paired within the plane.
+cudaError_t nd_rows_forward(const LineAxis& x, long planes, int rows, const float* src, float2* half, cudaStream_t st);
+cudaError_t nd_rows_inverse(const LineAxis& x, long planes, int rows, const float2* half, float* dst, bool accumulate,
+                            float scale, cudaStream_t st);
+// blocks per world, and the pair-cells [bpw][nr][W] per channel of EpiArgs::F (0: the fields stay on chip)
+int nd_rows_epi_blocks(const NdTab& t, const LineAxis& x, long n_worlds, long* field_pairs);
+cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& a, cudaStream_t st);
+// nd_conv.cu.  In-place transforms along y (H points, Wh lines per z-plane).
+cudaError_t nd_columns(bool inv, const NdTab& t, const LineAxis& y, long planes, float2* data, cudaStream_t st);
+struct ConvArgs {
+  int n_init;
+  const float2* kh;    // half spectra [Ns, C, max_k, hcells] as the caller gave them
+  long kh_sol_stride;
+  const float2* S;     // [nw, C, hcells], the other axes transformed
+  float2* P;           // forward: [nw, K, hcells] products out
+  const float2* A;     // adjoint: [nw, K, hcells] spectra of a = dL/du, the other axes transformed
+  float2* gk;          // adjoint: [nw, K, hcells] kernel-gradient spectra (accumulated)
+  float2* Q;           // adjoint: [nw, C, hcells] correlations out
+};
+cudaError_t nd_convolve(bool adjoint, const NdTab& t, const LineAxis& last, long nw, const ConvArgs& a,
+                        cudaStream_t st);
+// nd_plane.cu.  3D worlds whose z-planes fit a tile.
+bool nd_plane_ok(const NdTab& t, const NdAxes& ax);
+bool nd_plane_field_global(const NdTab& t, const NdAxes& ax);
+cudaError_t nd_plane_forward(const NdTab& t, const NdAxes& ax, long planes, const float* src, float2* half,
+                             cudaStream_t st);
+cudaError_t nd_plane_inverse(const NdTab& t, const NdAxes& ax, long planes, const float2* half, float* dst,
+                             bool accumulate, float scale, cudaStream_t st);
+cudaError_t nd_plane_epilogue(const NdTab& t, const NdAxes& ax, const EpiArgs& a, cudaStream_t st);
+
+}  // namespace lgx

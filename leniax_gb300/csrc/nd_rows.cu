@@ -1,0 +1,410 @@
+// Row transforms of the general N-D engine and the Euler step's row epilogue.
+//
+// Two real rows travel as one complex row (row0 + i row1), so a pass moves and
+// transforms half spectra of W/2 + 1 columns instead of full complex planes.
+// The epilogue block takes a tile of row pairs of one world through the
+// inverse row transform of every kernel's product, growth, the weighted field,
+// the state update and its statistics moments, and the next step's forward row
+// transform of the new rows: the potentials and the new rows never leave the
+// block (they are stored only as the new state and as requested trajectories).
+#include "nd.cuh"
+
+namespace lgx {
+namespace {
+
+struct RowsArgs {
+  const float* src;
+  float* dst;
+  float2* half;
+  const float2* half_in;
+  long pairs;       // planes * pp
+  int rows, W, Wh, pp, nr;
+  FastDivU ppd, whd;
+  int pitch, zp;    // exchange pitch; pitch of the Z rows
+  long buf;         // elements of one exchange buffer
+  FastDivU nrd;
+  float scale;
+  int accumulate;
+};
+
+// Row pair l of the block's tile: its first row (plane * rows + row), 0, 1 or 2 rows.
+__device__ __forceinline__ void tile_pair(const RowsArgs& a, int l, long* row, int* n) {
+  const long g = (long)blockIdx.x * a.nr + l;
+  *row = 0;
+  *n = 0;
+  if (g >= a.pairs) return;
+  const int plane = a.ppd.div((int)g), r0 = 2 * ((int)g - plane * a.pp);
+  *row = (long)plane * a.rows + r0;
+  *n = min(2, a.rows - r0);
+}
+
+template <bool BL>
+__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_fwd_kernel(RowsArgs a, LineAxis ax) {
+  extern __shared__ __align__(16) float2 sm[];
+  __shared__ long row[kMaxTileLines];
+  __shared__ int cnt[kMaxTileLines];
+  float2* tw = sm;
+  Tile t;
+  t.b[0] = tw + ax.m;
+  t.b[1] = t.b[0] + a.buf;
+  float2* Z = t.b[1] + a.buf;
+  t.lp = a.pitch;
+  t.nl = a.nr;
+  t.nld = a.nrd;
+  load_line_twiddles(tw, ax);
+  for (int l = threadIdx.x; l < a.nr; l += blockDim.x) tile_pair(a, l, row + l, cnt + l);
+  __syncthreads();
+  const float* __restrict__ src = a.src;
+  const int W = a.W, zp = a.zp;
+  line_fft<false, false, BL>(
+      ax, tw, t,
+      [&](int l, int i) {
+        const float* p = src + row[l] * W + i;
+        const int n = cnt[l];
+        return make_float2(n > 0 ? __ldg(p) : 0.f, n > 1 ? __ldg(p + W) : 0.f);
+      },
+      [=](int l, int k, float2 v) { Z[l * zp + k] = v; });
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < a.nr * a.Wh; idx += blockDim.x) {
+    const int l = a.whd.div(idx), k = idx - l * a.Wh;
+    const int n = cnt[l];
+    if (n == 0) continue;
+    const float2 zk = Z[l * zp + k], zm = Z[l * zp + (k == 0 ? 0 : W - k)];
+    float2* o = a.half + row[l] * a.Wh + k;
+    o[0] = unpack_row0(zk, zm);
+    if (n > 1) o[a.Wh] = unpack_row1(zk, zm);
+  }
+}
+
+template <bool BL>
+__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_inv_kernel(RowsArgs a, LineAxis ax) {
+  extern __shared__ __align__(16) float2 sm[];
+  __shared__ long row[kMaxTileLines];
+  __shared__ int cnt[kMaxTileLines];
+  float2* tw = sm;
+  Tile t;
+  t.b[0] = tw + ax.m;
+  t.b[1] = t.b[0] + a.buf;
+  t.lp = a.pitch;
+  t.nl = a.nr;
+  t.nld = a.nrd;
+  load_line_twiddles(tw, ax);
+  for (int l = threadIdx.x; l < a.nr; l += blockDim.x) tile_pair(a, l, row + l, cnt + l);
+  __syncthreads();
+  const float2* __restrict__ half = a.half_in;
+  const int W = a.W, Wh = a.Wh;
+  line_fft<true, false, BL>(
+      ax, tw, t,
+      [&](int l, int i) {
+        const bool mir = i >= Wh;
+        const float2* p = half + row[l] * Wh + (mir ? W - i : i);
+        const int n = cnt[l];
+        const float2 z = make_float2(0.f, 0.f);
+        return pack_rows(n > 0 ? __ldg(p) : z, n > 1 ? __ldg(p + Wh) : z, i, W);
+      },
+      [&](int l, int x, float2 v) {
+        const int n = cnt[l];
+        float* p = a.dst + row[l] * W + x;
+        if (a.accumulate) {
+          if (n > 0) p[0] = fmaf(v.x, a.scale, p[0]);
+          if (n > 1) p[W] = fmaf(v.y, a.scale, p[W]);
+        } else {
+          if (n > 0) p[0] = v.x * a.scale;
+          if (n > 1) p[W] = v.y * a.scale;
+        }
+      });
+}
+
+// Geometry of a row tile: nr pairs (all of `pairs` over the fill target, at
+// most a buffer's worth), their exchange buffers and threads.
+struct RowTile {
+  int nr, pitch, zp, threads;
+  long buf;
+};
+RowTile row_tile(const LineAxis& x, long pairs, long group_pairs) {
+  RowTile r;
+  const long fill = (pairs + kFillBlocks - 1) / kFillBlocks;
+  // one butterfly per thread at most twice over
+  const long by_items = std::max(1L, 2L * kNdThreads * std::min(x.r[0], std::max(x.r[x.stages - 1], 2)) / x.m);
+  const long cap = std::max(1L, std::min<long>(std::min<long>(kMaxTileLines, by_items), kMaxPts / x.m));
+  const long want = std::max(1L, std::min(std::min(cap, fill), group_pairs));
+  const long tiles = (group_pairs + want - 1) / want;
+  r.nr = (int)((group_pairs + tiles - 1) / tiles);  // even tiles over the group
+  r.pitch = line_pitch(false, x, r.nr);
+  r.buf = line_buf_elems(false, x, r.nr);
+  r.zp = x.n | 1;
+  r.threads = nd_threads(line_items(x, r.nr));
+  return r;
+}
+
+cudaError_t rows_args(const LineAxis& x, long planes, int rows, RowsArgs* a, RowTile* rt) {
+  a->rows = rows;
+  a->W = x.n;
+  a->Wh = x.n / 2 + 1;
+  a->pp = (rows + 1) / 2;
+  a->pairs = planes * a->pp;
+  if (a->pairs >= (1L << 31)) return cudaErrorInvalidConfiguration;
+  *rt = row_tile(x, a->pairs, a->pairs);
+  a->nr = rt->nr;
+  a->ppd = make_fastdiv((unsigned)a->pp);
+  a->whd = make_fastdiv((unsigned)a->Wh);
+  a->nrd = make_fastdiv((unsigned)a->nr);
+  a->pitch = rt->pitch;
+  a->zp = rt->zp;
+  a->buf = rt->buf;
+  return cudaSuccess;
+}
+
+// ------------------------------------------------------------------ epilogue
+struct RowsEpi {
+  int pp, nr, pitch, zp;  // pairs per world, pairs per tile, pitches
+  int lanes;              // threads per row pair of the epilogue
+  long buf;
+  FastDivU nrd, hd, whd;
+  int field_smem;         // the weighted fields live in shared memory
+};
+
+// SINGLE (C = K = 1): the epilogue works on the potentials in Z and leaves the
+// new cells there.  Otherwise the weighted fields of the tile accumulate over
+// the kernels in F, and the update is the load rule of each channel's forward
+// transform.
+template <bool SINGLE, bool BL>
+__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_epi_kernel(NdTab t, EpiArgs a, RowsEpi g, LineAxis ax) {
+  extern __shared__ __align__(16) float2 sm[];
+  __shared__ RowPair rp[kMaxTileLines];
+  __shared__ EpiShared sh;
+  float2* tw = sm;
+  Tile tl;
+  tl.b[0] = tw + ax.m;
+  tl.b[1] = tl.b[0] + g.buf;
+  float2* Z = tl.b[1] + g.buf;
+  tl.lp = g.pitch;
+  tl.nl = g.nr;
+  tl.nld = g.nrd;
+  const int w = blockIdx.x / a.bpw, b = blockIdx.x - w * a.bpw;
+  const int sol = w / a.n_init;
+  const int W = t.W, Wh = t.Wh, C = t.C, K = t.K, zp = g.zp;
+  const int s0 = a.shift[3 * w], s1 = a.shift[3 * w + 1], s2 = a.shift[3 * w + 2];
+  const int sx = t.nd == 3 ? s2 : s1;
+  const float dt = step_dt(t, a, w, sol);
+  const float* gf = a.gf + sol * a.gf_sol_stride;
+  const float* wt = a.w + sol * a.w_sol_stride;
+  load_line_twiddles(tw, ax);
+  for (int l = threadIdx.x; l < g.nr; l += blockDim.x) {
+    const int r0 = 2 * (b * g.nr + l), rows = max(0, min(2, t.D * t.H - r0));
+    const int q0 = rows > 0 ? r0 : 0, q1 = rows > 1 ? r0 + 1 : q0;
+    const int z0 = g.hd.div(q0), z1 = g.hd.div(q1);
+    rp[l] = row_pair(t, z0, q0 - z0 * t.H, z1, q1 - z1 * t.H, rows, s0, s1, s2);
+  }
+  __syncthreads();
+  Moments mo;
+  const long plane0 = (long)w * C * t.cells;  // the world's first cell
+  const float* __restrict__ state = a.state + plane0;
+  // the product rows of kernel k, packed
+  auto load_rows = [&](int k) {
+    const float2* __restrict__ src = a.P + ((long)w * K + k) * t.hcells + (long)2 * b * g.nr * Wh;
+    return [=](int l, int i) {
+      const bool mir = i >= Wh;
+      const float2* p = src + (long)2 * l * Wh + (mir ? W - i : i);
+      const int n = rp[l].rows;
+      const float2 z = make_float2(0.f, 0.f);
+      return pack_rows(n > 0 ? __ldg(p) : z, n > 1 ? __ldg(p + Wh) : z, i, W);
+    };
+  };
+  // both cells of a pair: state update, stores, moments; returns the new cells
+  auto update = [&](const RowPair& r, int c, int x, float2 s, float2 f) {
+    const long off = plane0 + (long)c * t.cells + r.cell + x;
+    float2 n = make_float2(state_fn(t.state_fn, s.x, f.x, dt), 0.f);
+    a.state_out[off] = n.x;
+    if (a.field_out) a.field_out[off] = f.x;
+    if (a.state_copy) a.state_copy[off] = s.x;
+    if (r.rows > 1) {
+      n.y = state_fn(t.state_fn, s.y, f.y, dt);
+      a.state_out[off + W] = n.y;
+      if (a.field_out) a.field_out[off + W] = f.y;
+      if (a.state_copy) a.state_copy[off + W] = s.y;
+    } else {
+      f.y = 0.f;
+    }
+    mo.add(r, s, f, centred_in(x, sx, W), x == 0 || x == W - 1);
+    return n;
+  };
+  auto load_state = [&](const RowPair& r, int c, int x) {
+    const float* p = state + (long)c * t.cells + r.cell + x;
+    return make_float2(__ldg(p), r.rows > 1 ? __ldg(p + W) : 0.f);
+  };
+  // half spectra of the tile's new rows (in Z) into S
+  auto store_spectra = [&](int c) {
+    float2* o = a.S + ((long)w * C + c) * t.hcells + (long)2 * b * g.nr * Wh;
+    for (int idx = threadIdx.x; idx < g.nr * Wh; idx += blockDim.x) {
+      const int l = g.whd.div(idx), k = idx - l * Wh, n = rp[l].rows;
+      if (n == 0) continue;
+      const float2 zk = Z[l * zp + k], zm = Z[l * zp + (k == 0 ? 0 : W - k)];
+      o[(long)2 * l * Wh + k] = unpack_row0(zk, zm);
+      if (n > 1) o[(long)(2 * l + 1) * Wh + k] = unpack_row1(zk, zm);
+    }
+  };
+  auto store_z = [=](int l, int k, float2 v) { Z[l * zp + k] = v; };
+  if constexpr (SINGLE) {
+    const auto rows0 = load_rows(0);
+    line_fft<true, false, BL>(ax, tw, tl, rows0, store_z);
+    __syncthreads();
+    epi_single(t, a, rp, Z, g.nr, zp, g.lanes, w, sx, dt, mo);
+    const bool emit = a.S != nullptr;
+    if (emit) {
+      __syncthreads();
+      line_fft<false, false, BL>(
+          ax, tw, tl, [=](int l, int i) { return rp[l].rows ? Z[l * zp + i] : make_float2(0.f, 0.f); }, store_z);
+    }
+    epi_channel_mass(sh, 0, mo.m00);
+    if (emit) {
+      __syncthreads();
+      store_spectra(0);
+    }
+  } else {
+    // [C][nr][W] pairs: fields of row0 and row1
+    float2* F = g.field_smem ? Z + (long)g.nr * zp
+                             : reinterpret_cast<float2*>(a.F) + (long)(w * a.bpw + b) * C * g.nr * W;
+    for (int i = threadIdx.x; i < C * g.nr * W; i += blockDim.x) F[i] = make_float2(0.f, 0.f);
+    __syncthreads();
+    for (int k = 0; k < K; ++k) {
+      const NdGrowth grow(t.gf[k], __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1));
+      line_fft<true, false, BL>(ax, tw, tl, load_rows(k), [&](int l, int x, float2 v) {
+        const int rows = rp[l].rows;
+        if (rows == 0) return;
+        const float2 u = make_float2(v.x * a.scale, v.y * a.scale);
+        if (a.pot_out) {
+          float* p = a.pot_out + ((long)w * K + k) * t.cells + rp[l].cell + x;
+          p[0] = u.x;
+          if (rows > 1) p[W] = u.y;
+        }
+        mo.count_pot(u, rows);
+        const float2 gr = make_float2(grow(u.x), grow(u.y));
+        for (int c = 0; c < C; ++c) {
+          const float wk = __ldg(wt + c * K + k);
+          if (wk == 0.f) continue;
+          float2* f = F + ((long)c * g.nr + l) * W + x;
+          *f = __ffma2_rn(gr, make_float2(wk, wk), *f);
+        }
+      });
+    }
+    __syncthreads();
+    for (int c = 0; c < C; ++c) {
+      float wsum = 0.f;
+      for (int k = 0; k < K; ++k) wsum += __ldg(wt + c * K + k);
+      const float before = mo.m00;
+      mo.m00 = 0.f;  // this channel's mass
+      auto new_cells = [&](int l, int x) {
+        const RowPair& r = rp[l];
+        if (r.rows == 0) return make_float2(0.f, 0.f);
+        float2 f = F[((long)c * g.nr + l) * W + x];
+        if (t.mean) f = make_float2(f.x / wsum, f.y / wsum);
+        return update(r, c, x, load_state(r, c, x), f);
+      };
+      if (a.S) {
+        line_fft<false, false, BL>(ax, tw, tl, new_cells, store_z);
+        __syncthreads();
+        store_spectra(c);
+        __syncthreads();  // Z is rewritten by the next channel
+      } else {
+        for (int i = threadIdx.x; i < g.nr * W; i += blockDim.x) new_cells(i / W, i % W);
+      }
+      epi_channel_mass(sh, c, mo.m00);
+      mo.m00 += before;
+    }
+  }
+  epi_finish(t, a, sh, w, b, mo, s0, s1, s2);
+}
+
+struct EpiTile {
+  RowTile rt;
+  int bpw;
+  bool field_smem;
+  size_t smem;
+};
+EpiTile epi_tile(const NdTab& t, const LineAxis& x, long n_worlds) {
+  EpiTile e;
+  const int pp = (t.D * t.H + 1) / 2;
+  e.rt = row_tile(x, n_worlds * pp, pp);
+  e.bpw = (pp + e.rt.nr - 1) / e.rt.nr;
+  const size_t base = (size_t)(x.m + 2 * e.rt.buf + (long)e.rt.nr * e.rt.zp) * sizeof(float2);
+  const size_t field = t.C == 1 && t.K == 1 ? 0 : (size_t)t.C * e.rt.nr * t.W * sizeof(float2);
+  // two blocks per SM keep the fields in shared memory; larger sets go through L2
+  e.field_smem = base + field <= (size_t)108 * 1024;
+  e.smem = base + (e.field_smem ? field : 0);
+  return e;
+}
+
+}  // namespace
+
+cudaError_t nd_rows_forward(const LineAxis& x, long planes, int rows, const float* src, float2* half,
+                            cudaStream_t st) {
+  RowsArgs a{};
+  RowTile rt;
+  cudaError_t e = rows_args(x, planes, rows, &a, &rt);
+  if (e != cudaSuccess) return e;
+  a.src = src;
+  a.half = half;
+  const size_t smem = (size_t)(x.m + 2 * rt.buf + (long)rt.nr * rt.zp) * sizeof(float2);
+  const bool bl = x.m != x.n;
+  const void* f = bl ? (const void*)nd_rows_fwd_kernel<true> : (const void*)nd_rows_fwd_kernel<false>;
+  if ((e = nd_allow_smem(f)) != cudaSuccess) return e;
+  const unsigned blocks = (unsigned)((a.pairs + a.nr - 1) / a.nr);
+  if (bl) nd_rows_fwd_kernel<true><<<blocks, rt.threads, smem, st>>>(a, x);
+  else nd_rows_fwd_kernel<false><<<blocks, rt.threads, smem, st>>>(a, x);
+  return cudaGetLastError();
+}
+
+cudaError_t nd_rows_inverse(const LineAxis& x, long planes, int rows, const float2* half, float* dst, bool accumulate,
+                            float scale, cudaStream_t st) {
+  RowsArgs a{};
+  RowTile rt;
+  cudaError_t e = rows_args(x, planes, rows, &a, &rt);
+  if (e != cudaSuccess) return e;
+  a.half_in = half;
+  a.dst = dst;
+  a.accumulate = accumulate ? 1 : 0;
+  a.scale = scale;
+  const size_t smem = (size_t)(x.m + 2 * rt.buf) * sizeof(float2);
+  const bool bl = x.m != x.n;
+  const void* f = bl ? (const void*)nd_rows_inv_kernel<true> : (const void*)nd_rows_inv_kernel<false>;
+  if ((e = nd_allow_smem(f)) != cudaSuccess) return e;
+  const unsigned blocks = (unsigned)((a.pairs + a.nr - 1) / a.nr);
+  if (bl) nd_rows_inv_kernel<true><<<blocks, rt.threads, smem, st>>>(a, x);
+  else nd_rows_inv_kernel<false><<<blocks, rt.threads, smem, st>>>(a, x);
+  return cudaGetLastError();
+}
+
+int nd_rows_epi_blocks(const NdTab& t, const LineAxis& x, long n_worlds, long* field_pairs) {
+  const EpiTile e = epi_tile(t, x, n_worlds);
+  if (field_pairs) *field_pairs = e.field_smem ? 0 : (long)e.bpw * e.rt.nr * t.W;
+  return e.bpw;
+}
+
+cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& args, cudaStream_t st) {
+  EpiArgs a = args;
+  const EpiTile e = epi_tile(t, x, a.n_worlds);
+  a.bpw = e.bpw;
+  RowsEpi g;
+  g.pp = (t.D * t.H + 1) / 2;
+  g.nr = e.rt.nr;
+  g.pitch = e.rt.pitch;
+  g.zp = e.rt.zp;
+  g.lanes = epi_lanes(t.W);
+  g.buf = e.rt.buf;
+  g.nrd = make_fastdiv((unsigned)g.nr);
+  g.hd = make_fastdiv((unsigned)t.H);
+  g.whd = make_fastdiv((unsigned)t.Wh);
+  g.field_smem = e.field_smem ? 1 : 0;
+  const long blocks = (long)a.n_worlds * a.bpw;
+  if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
+  const bool bl = x.m != x.n, single = t.C == 1 && t.K == 1;
+  auto f = single ? (bl ? nd_rows_epi_kernel<true, true> : nd_rows_epi_kernel<true, false>)
+                  : (bl ? nd_rows_epi_kernel<false, true> : nd_rows_epi_kernel<false, false>);
+  const cudaError_t err = nd_allow_smem((const void*)f);
+  if (err != cudaSuccess) return err;
+  f<<<(unsigned)blocks, e.rt.threads, e.smem, st>>>(t, a, g, x);
+  return cudaGetLastError();
+}
+
+}  // namespace lgx
