@@ -18,7 +18,9 @@ LIB = os.path.join(HERE, '_lgx.so')
 
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 NVCC_FLAGS = ['-O3', '-lineinfo', '-std=c++17', '--expt-relaxed-constexpr', '-Xcompiler', '-fPIC',
-              '-Xcompiler', '-fvisibility=hidden', '-Xptxas', '-warn-spills', '--split-compile=4']
+              '-Xcompiler', '-fvisibility=hidden', '-Xptxas', '-warn-spills']
+# the N-D engine's kernels hold one body per radix: their functions are compiled side by side
+SPLIT_FLAGS = ['--split-compile=4']
 
 
 def nvcc_path():
@@ -51,7 +53,8 @@ def build(verbose=False, force=False, extra_flags=()):
         obj = os.path.join(OBJ, os.path.basename(src)[:-3] + '.o')
         objs.append(obj)
         if force or _stale(obj, [src] + headers):
-            cmd = [nvcc] + ARCH + NVCC_FLAGS + list(extra_flags) + ['-c', src, '-o', obj]
+            split = SPLIT_FLAGS if os.path.basename(src).startswith('nd_') else []
+            cmd = [nvcc] + ARCH + NVCC_FLAGS + split + list(extra_flags) + ['-c', src, '-o', obj]
             jobs.append(cmd)
 
     def run(cmd):
