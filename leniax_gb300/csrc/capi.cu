@@ -217,7 +217,7 @@ StreamedBufs carve_streamed(const Model& m, int n_sols, int n_init, int steps, v
   b.spec = cv.take<float2>((size_t)nw * m.C * m.cells / 2);
   b.prod = cv.take<float2>((size_t)nw * m.K * m.cells / 2);
   b.kp = cv.take<float2>((size_t)n_sols * m.C * m.max_k * m.H * (m.W / 2 + 2));
-  b.partial = cv.take<float>((size_t)nw * streamed_blocks_per_world(m) * raw_stride(m.C));
+  b.partial = cv.take<float>(streamed_partial_floats(m, nw));
   b.shift = cv.take<int>((size_t)nw * 3);
   b.sa = cv.take<float>((size_t)nw * m.C * m.cells);
   b.sb = cv.take<float>((size_t)nw * m.C * m.cells);

@@ -141,7 +141,8 @@ cudaError_t launch_prepare_3d_spectrum(int N, long n, const float2* k_half, floa
 struct StreamedArgs;  // defined in streamed.cu
 bool streamed_supported(const Model& m);
 size_t streamed_workspace_bytes(const Model& m, int n_worlds, int n_sols);
-int streamed_blocks_per_world(const Model& m);
+// Floats of the row inverse's moment partials, for launches of up to n_worlds worlds.
+size_t streamed_partial_floats(const Model& m, int n_worlds);
 // One step of n_worlds worlds (all solutions): see streamed.cu.
 struct StreamedStep {
   const Model* m;

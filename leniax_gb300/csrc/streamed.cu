@@ -130,10 +130,10 @@ constexpr size_t col_conv_smem() {
          (size_t)CC::GPB * GE::SCR * sizeof(float2) + (size_t)N * sizeof(float2) + 16;
 }
 
-// Next kernel after k (or K) reading channel ch.
-__device__ __forceinline__ int next_kernel(const KTab& tab, int k, int ch) {
+// The n-th kernel after k (or K) reading channel ch.
+__device__ __forceinline__ int next_kernel(const KTab& tab, int k, int ch, int n) {
   for (++k; k < tab.K; ++k)
-    if (tab.cin[k] == ch) break;
+    if (tab.cin[k] == ch && --n == 0) break;
   return k;
 }
 
@@ -141,7 +141,9 @@ __device__ __forceinline__ int next_kernel(const KTab& tab, int k, int ch) {
 // arrives by TMA; per kernel reading the channel, the kernel's GPB spectrum
 // columns arrive by bulk copy (issued one kernel ahead), and the product
 // columns leave through the same swizzled tile by TMA stores, so the kernel's
-// global traffic bypasses the load/store pipe.
+// global traffic bypasses the load/store pipe.  gridDim.y blocks share a
+// tile's kernels (block y takes every gridDim.y-th of them, each repeating the
+// forward transform): see col_conv_split.
 template <int N>
 __global__ void __launch_bounds__(ColCfg<N>::T) col_conv_kernel(const __grid_constant__ CUtensorMap spec_map,
                                                                const __grid_constant__ CUtensorMap prod_map,
@@ -176,7 +178,9 @@ __global__ void __launch_bounds__(ColCfg<N>::T) col_conv_kernel(const __grid_con
     bulk_load(kb, kk + (size_t)j0 * N, main, &bar[1]);
     if (nyq) bulk_load(kb + GPB * N, kk + (size_t)(N / 2) * N, nyq, &bar[1]);
   };
-  const int k_first = next_kernel(tab, -1, ch);
+  const int ks = gridDim.y;
+  const int k_first = next_kernel(tab, -1, ch, blockIdx.y + 1);
+  if (k_first >= tab.K) return;
   if (threadIdx.x == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(ColCfg<N>::T) col_conv_kernel(const __grid_con
     mbar_arrive_expect_tx(&bar[0], CC::TILE_BYTES);
     for (int b = 0; b < CC::BOXES; ++b)
       tma_load_2d(tile + b * CC::BOX_BYTES, &spec_map, (j0 + 8 * b) * 4, plane * (N / 2), &bar[0]);
-    if (CC::KSTAGE && k_first < tab.K) issue_kernel(k_first);
+    if (CC::KSTAGE) issue_kernel(k_first);
   }
   init_twiddles<GE>(sm, sm + N, sm + 2 * N, threadIdx.x, blockDim.x);
   __syncthreads();
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(ColCfg<N>::T) col_conv_kernel(const __grid_con
     if (threadIdx.x == 0) {
       if (status) atomicExch(status, kStatusCopyTimeout);
       mbar_wait(&bar[0], 0);
-      if (CC::KSTAGE && k_first < tab.K) mbar_wait(&bar[1], 0);
+      if (CC::KSTAGE) mbar_wait(&bar[1], 0);
     }
     return;
   }
@@ -243,7 +247,7 @@ __global__ void __launch_bounds__(ColCfg<N>::T) col_conv_kernel(const __grid_con
     __syncwarp(gmask);
   }
   int it = 0;
-  for (int k = k_first; k < tab.K; k = next_kernel(tab, k, ch), ++it) {
+  for (int k = k_first; k < tab.K; k = next_kernel(tab, k, ch, ks), ++it) {
     bool ok = true;
     if constexpr (CC::KSTAGE) ok = mbar_wait(&bar[1], it & 1);
     float2 w[P];
@@ -273,7 +277,7 @@ __global__ void __launch_bounds__(ColCfg<N>::T) col_conv_kernel(const __grid_con
       }
       return;
     }
-    const int k_next = next_kernel(tab, k, ch);
+    const int k_next = next_kernel(tab, k, ch, ks);
     if (CC::KSTAGE && threadIdx.x == 0 && k_next < tab.K) issue_kernel(k_next);
     float2 u[Q][G];
     if constexpr (Q == 1) {
@@ -306,6 +310,24 @@ __global__ void __launch_bounds__(ColCfg<N>::T) col_conv_kernel(const __grid_con
     }
   }
   if (threadIdx.x == 0) bulk_wait_all();
+}
+
+// Q == 1: lane t needs Z[k], k = t + P*n2: one pair load each (k < N/2 for n2 < G/2)
+template <class GE>
+__device__ __forceinline__ void unpack_row_pair_q1(const float2* row, float2 (&v)[GE::Q][GE::G], int t) {
+  constexpr int N = GE::N, G = GE::G, P = GE::P;
+  const float4* p4 = reinterpret_cast<const float4*>(row);
+#pragma unroll
+  for (int n2 = 0; n2 < G; ++n2) {
+    const int k = t + P * n2;
+    if (n2 < G / 2) {
+      const float4 q = p4[k];  // k == 0: pair 0 = (DC, Nyquist)
+      v[0][n2] = k == 0 ? make_float2(q.x, q.z) : make_float2(q.x - q.w, q.y + q.z);
+    } else {
+      const float4 q = p4[k == N / 2 ? 0 : N - k];
+      v[0][n2] = k == N / 2 ? make_float2(q.y, q.w) : make_float2(q.x + q.w, q.z - q.y);
+    }
+  }
 }
 
 // ------------------------------------------------------------------ row_inv
@@ -482,19 +504,7 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
     float2* row = bufs + (i % NBUF) * RC::BUF + grp * ROWP;
     float2 v[Q][G];
     if constexpr (Q == 1) {
-      // lane t needs Z[k], k = t + P*n2: one pair load each (k < N/2 for n2 < G/2)
-      const float4* p4 = reinterpret_cast<const float4*>(row);
-#pragma unroll
-      for (int n2 = 0; n2 < G; ++n2) {
-        const int k = t + P * n2;
-        if (n2 < G / 2) {
-          const float4 q = p4[k];  // k == 0: pair 0 = (DC, Nyquist)
-          v[0][n2] = k == 0 ? make_float2(q.x, q.z) : make_float2(q.x - q.w, q.y + q.z);
-        } else {
-          const float4 q = p4[k == N / 2 ? 0 : N - k];
-          v[0][n2] = k == N / 2 ? make_float2(q.y, q.w) : make_float2(q.x + q.w, q.z - q.y);
-        }
-      }
+      unpack_row_pair_q1<GE>(row, v, t);
     } else {
       unpack_row_pair_pa<GE>(row, v, t);
     }
@@ -662,22 +672,279 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
   }
 }
 
-// ----------------------------------------------------------------- reduce
-// One warp per world: sum the block partials, write the step's raw moments,
-// update the carried torus shift with trunc(centroid) (statistics.py:117-119).
-__global__ void reduce_kernel(int n_worlds, int n_init, int bpw, int C, int H, int W, const float* __restrict__ partial,
-                              float* __restrict__ raw, long raw_sol_stride, long raw_init_stride, int* __restrict__ shift) {
-  const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+// ------------------------------------------------------------ row_inv_split
+// The row inverse for few worlds.  row_inv_kernel walks a world's C x K work
+// items one after another in N/2/GPB blocks, which leaves the chip idle and
+// the step as long as that chain.  Here a block owns the 32 / G packed rows of
+// one warp's transforms and one output channel, its warps take the channel's
+// kernels in turn (rows straight from L2 into the transform), the weighted
+// growths meet in shared memory, and the warps share the cells of the
+// epilogue; warp 0 then runs the fused forward transform of the new rows while
+// another sums the moments.  Bound by instruction issue of a lone block an SM
+// (48 blocks for one 128^2 world of three channels); 15 kernels of one 128^2
+// world: 43 us a step walking, 8.9 us split.
+template <int N>
+struct SplitCfg {
+  static constexpr int G = SCfg<N>::G;
+  static constexpr int RPB = 32 / G;          // packed rows per block
+  static constexpr int BPC = (N / 2) / RPB;   // blocks per world and channel
+  static constexpr int XCH = RPB * (N + G);   // float2 of exchange scratch per warp
+};
+constexpr int kSplitMinWarps = 4, kSplitMaxWarps = 8;
+
+template <int N>
+size_t row_inv_split_smem(int warps) {
+  return ((size_t)3 * N + (size_t)warps * SplitCfg<N>::XCH) * sizeof(float2) +
+         (size_t)warps * (RAW_CM + kMaxChannels) * sizeof(float);
+}
+
+template <int N, int GF>
+__global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
+    int n_worlds, int n_init, KTab tab, const float2* __restrict__ prod, const float* __restrict__ gfp,
+    long gf_sol_stride, const float* __restrict__ wts, long w_sol_stride, const float* __restrict__ dtp,
+    const float* __restrict__ state, float* __restrict__ state_out, float* __restrict__ field_out,
+    float* __restrict__ pot_out, const int* __restrict__ shift, float* __restrict__ partial,
+    float2* __restrict__ spec_next) {
+  using SC = SplitCfg<N>;
+  constexpr int G = SC::G, BPC = SC::BPC;
+  using GE = Geo<N, G>;
+  constexpr int P = GE::P, Q = GE::Q;
+  constexpr int RAWS_MAX = RAW_CM + kMaxChannels;
+  static_assert(SC::XCH >= P * 32, "a warp's scratch holds its weighted growths");
+  extern __shared__ __align__(16) float2 sm[];
+  const int warps = blockDim.x >> 5, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  float2* tw = sm;                      // 3N twiddles
+  float2* xch = tw + 3 * N;             // [warps][XCH]
+  float* red = reinterpret_cast<float*>(xch + warps * SC::XCH);  // [warps][RAWS_MAX]
+  const int C = tab.C, K = tab.K;
+  const int n = blockIdx.x / (BPC * C);
   if (n >= n_worlds) return;
+  const int co = blockIdx.x / BPC % C;
+  const int sol = n / n_init;
+  const int grp = lane / G, t = lane % G;
+  const int r = (blockIdx.x % BPC) * SC::RPB + grp;
+  const unsigned gmask = ((1u << G) - 1u) << (lane & ~(G - 1));
+  const float* gf = gfp + sol * gf_sol_stride;
+  const float* wt = wts + sol * w_sol_stride;
+  init_twiddles<GE>(tw, tw + N, tw + 2 * N, threadIdx.x, blockDim.x);
+
+  // bit k: kernel k feeds this channel / an earlier one / any channel
+  static_assert(kMaxKernels <= 64, "one bit per kernel");
+  unsigned long long fed = 0ull, before = 0ull, any = 0ull;
+  float wsum = 0.f;
+  for (int h = 0; h < K; h += 32) {
+    const int k = h + lane;
+    for (int c = 0; c < C; ++c) {
+      const float w = k < K ? __ldg(wt + c * K + k) : 0.f;
+      const unsigned long long b = (unsigned long long)__ballot_sync(0xffffffffu, w != 0.f) << h;
+      any |= b;
+      if (c < co) before |= b;
+      if (c == co) {
+        fed = fed | b;
+        wsum += w;
+      }
+    }
+  }
+  wsum = warp_sum(wsum);
+  // channel 0 also takes the kernels that feed no channel (their potentials count)
+  const unsigned long long all = K == 64 ? ~0ull : (1ull << K) - 1ull;
+  const unsigned long long mine = fed | (co == 0 ? all & ~any : 0ull);
+
+  float dt;
+  if (tab.dt_mode == 0) dt = __ldg(dtp);
+  else if (tab.dt_mode == 1) dt = __ldg(dtp + n);
+  else dt = 1.f / __ldg(dtp + sol);
+  const int sy = shift[3 * n], sx = shift[3 * n + 1];
+  const size_t base = ((size_t)n * C + co) * N * N + (size_t)(2 * r) * N;
+  float cpot = 0.f;
+  float2* scr = xch + wid * SC::XCH;
+  float2 acc[P];
+#pragma unroll
+  for (int k1 = 0; k1 < P; ++k1) acc[k1] = make_float2(0.f, 0.f);
+  __syncthreads();
+  int rank = 0;
+  for (unsigned long long todo = mine; todo; todo &= todo - 1) {
+    if (rank++ % warps != wid) continue;
+    const int k = __ffsll((long long)todo) - 1;
+    const float2* row = prod + (((size_t)n * K + k) * (N / 2) + r) * N;
+    float2 v[Q][G];
+    if constexpr (Q == 1) unpack_row_pair_q1<GE>(row, v, t);
+    else unpack_row_pair_pa<GE>(row, v, t);
+    float2 w[P];
+    __syncwarp();  // the previous item's exchange has been read
+    fft_mirrored<GE, true, true>(v, w, scr + grp * GE::SCR, tw + 2 * N, t, gmask);
+    if (!((before >> k) & 1ull)) {
+#pragma unroll
+      for (int k1 = 0; k1 < P; ++k1) cpot += (w[k1].x > kEps ? 1.f : 0.f) + (w[k1].y > kEps ? 1.f : 0.f);
+      if (pot_out) {
+        float* po = pot_out + ((size_t)n * K + k) * N * N + (size_t)(2 * r) * N;
+#pragma unroll
+        for (int k1 = 0; k1 < P; ++k1) {
+          po[t + G * k1] = w[k1].x;
+          po[N + t + G * k1] = w[k1].y;
+        }
+      }
+    }
+    if ((fed >> k) & 1ull) {
+      const float wk = __ldg(wt + co * K + k);
+      GrowthP g;
+      g.m = __ldg(gf + 2 * k);
+      g.s = __ldg(gf + 2 * k + 1);
+      g.a = GF == GF_FAST_GAUSSIAN ? 0.84932180028801904272f / g.s : (GF == GF_FAST_POLY4 ? 1.f / (9.f * (g.s * g.s)) : 0.f);
+      g.id = tab.gf[k];
+#pragma unroll
+      for (int k1 = 0; k1 < P; ++k1) {
+        if constexpr (GF == GF_GENERIC) {
+          acc[k1].x = fmaf(wk, growth_cell<GF>(g, w[k1].x), acc[k1].x);
+          acc[k1].y = fmaf(wk, growth_cell<GF>(g, w[k1].y), acc[k1].y);
+        } else {  // w (2 e - 1) summed as 2 w e here, minus the channel's weight sum below
+          acc[k1] = __ffma2_rn(make_float2(2.f * wk, 2.f * wk), growth_core2<GF>(g, w[k1]), acc[k1]);
+        }
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k1 = 0; k1 < P; ++k1) scr[k1 * 32 + lane] = acc[k1];
+  __syncthreads();
+
+  // field (weighted_sum / weighted_mean, core.py:202-242), state update,
+  // moments: warp w takes the cells k1 = w, w + warps, ...
+  const int nacc = rank < warps ? rank : warps;
+  const float cya = (float)(((2 * r - sy) & (N - 1)) - N / 2);
+  const float cyb = (float)(((2 * r + 1 - sy) & (N - 1)) - N / 2);
+  float Sa = 0.f, Sb = 0.f, Ga = 0.f, Gb = 0.f, cmass = 0.f, cgrow = 0.f, mxx = 0.f, gxx = 0.f, m2x = 0.f;
+  bool border = false;
+#pragma unroll 1
+  for (int k1 = wid; k1 < P; k1 += warps) {
+    const int x = t + G * k1;
+    const float sa = __ldg(state + base + x), sb = __ldg(state + base + N + x);
+    float fa = 0.f, fb = 0.f;
+    for (int q = 0; q < nacc; ++q) {
+      const float2 a = xch[q * SC::XCH + k1 * 32 + lane];
+      fa += a.x;
+      fb += a.y;
+    }
+    if constexpr (GF != GF_GENERIC) {
+      fa -= wsum;
+      fb -= wsum;
+    }
+    if (tab.mean) {
+      fa = fa / wsum;
+      fb = fb / wsum;
+    }
+    const float na = state_fn(tab.state_fn, sa, fa, dt), nb = state_fn(tab.state_fn, sb, fb, dt);
+    state_out[base + x] = na;
+    state_out[base + N + x] = nb;
+    if (field_out) {
+      field_out[base + x] = fa;
+      field_out[base + N + x] = fb;
+    }
+    xch[k1 * 32 + lane] = make_float2(na, nb);  // read above by this thread alone
+    const float fpa = fmaxf(fa, 0.f), fpb = fmaxf(fb, 0.f);
+    const float cx = (float)(((x - sx) & (N - 1)) - N / 2);
+    Sa += sa;
+    Sb += sb;
+    Ga += fpa;
+    Gb += fpb;
+    const float ss = sa + sb, gg = fpa + fpb;
+    mxx = fmaf(ss, cx, mxx);
+    gxx = fmaf(gg, cx, gxx);
+    m2x = fmaf(ss * cx, cx, m2x);
+    const bool la = sa > kEps, lb = sb > kEps;
+    cmass += (la ? 1.f : 0.f) + (lb ? 1.f : 0.f);
+    cgrow += (fpa > kEps ? 1.f : 0.f) + (fpb > kEps ? 1.f : 0.f);
+    border |= ((x == 0 || x == N - 1) && (la || lb)) || (r == 0 && la) || (r == N / 2 - 1 && lb);
+  }
+  float accm[11] = {Sa + Sb, Ga + Gb, cpot, cmass, cgrow, cya * Sa + cyb * Sb, mxx, cya * Ga + cyb * Gb, gxx,
+                    cya * cya * Sa + cyb * cyb * Sb, m2x};
+#pragma unroll
+  for (int q = 0; q < 11; ++q) accm[q] = warp_sum(accm[q]);
+  const bool anyb = __any_sync(0xffffffffu, border);
+  float* rd = red + wid * RAWS_MAX;
+  if (lane == 0) {
+    rd[RAW_M00] = accm[0];
+    rd[RAW_G00] = accm[1];
+    rd[RAW_CNT_POT] = accm[2];
+    rd[RAW_CNT_MASS] = accm[3];
+    rd[RAW_CNT_GROW] = accm[4];
+    rd[RAW_MX + 0] = accm[5];
+    rd[RAW_MX + 1] = accm[6];
+    rd[RAW_MX + 2] = 0.f;
+    rd[RAW_GX + 0] = accm[7];
+    rd[RAW_GX + 1] = accm[8];
+    rd[RAW_GX + 2] = 0.f;
+    rd[RAW_MX2 + 0] = accm[9];
+    rd[RAW_MX2 + 1] = accm[10];
+    rd[RAW_MX2 + 2] = 0.f;
+    rd[RAW_BORDER] = anyb ? 1.f : 0.f;
+    rd[RAW_SHIFT + 0] = rd[RAW_SHIFT + 1] = rd[RAW_SHIFT + 2] = 0.f;
+  }
+  if (lane < C) rd[RAW_CM + lane] = lane == co ? accm[0] : 0.f;
+  __syncthreads();
+  if (wid == warps - 1) {
+    const int RAWS = raw_stride(C);
+    for (int q = lane; q < RAWS; q += 32) {
+      float sum = 0.f;
+      for (int w = 0; w < warps; ++w) sum += red[w * RAWS_MAX + q];
+      if (q == RAW_BORDER) sum = sum > 0.f ? 1.f : 0.f;
+      partial[(size_t)blockIdx.x * RAWS + q] = sum;
+    }
+  }
+  if (wid == 0 && spec_next) {  // the next step's row pass: FFT of the packed new rows
+    float2 nsv[P];
+#pragma unroll
+    for (int k1 = 0; k1 < P; ++k1) nsv[k1] = xch[k1 * 32 + lane];
+    float2 u[Q][G];
+    fft_standard<GE, false, false>(nsv, u, xch + SC::XCH + grp * GE::SCR, tw, t, gmask);
+    float2* dst = spec_next + (((size_t)n * C + co) * (N / 2) + r) * N;
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int k1 = 0; k1 < G; ++k1) dst[pa_pos<N>(t + G * q + P * k1)] = u[q][k1];
+  }
+}
+
+// ----------------------------------------------------------------- reduce
+// Sum a world's block partials, write the step's raw moments, update the
+// carried torus shift with trunc(centroid) (statistics.py:117-119).  WPW warps
+// a world: one where a block of eight serves eight worlds, eight where one
+// warp would walk a long list of partials.
+constexpr int kReduceWarps = 8;
+
+template <int WPW>
+__global__ void __launch_bounds__(32 * kReduceWarps) reduce_kernel(
+    int n_worlds, int n_init, int bpw, int C, int H, int W, const float* __restrict__ partial, float* __restrict__ raw,
+    long raw_sol_stride, long raw_init_stride, int* __restrict__ shift) {
+  constexpr int RAWS_MAX = RAW_CM + kMaxChannels;
+  __shared__ float part[WPW > 1 ? WPW : 1][WPW > 1 ? RAWS_MAX : 1];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = blockIdx.x * (kReduceWarps / WPW) + wid / WPW;
+  if (n >= n_worlds) return;  // WPW > 1: one world a block, so whole blocks leave
   const int RAWS = raw_stride(C);
   const int sol = n / n_init, init = n - sol * n_init;
   float* rw = raw ? raw + sol * raw_sol_stride + init * raw_init_stride : nullptr;
+  if constexpr (WPW > 1) {
+    static_assert(WPW == kReduceWarps, "one world a block");
+    for (int s = lane; s < RAWS; s += 32) {
+      float v = 0.f;
+#pragma unroll 4
+      for (int b = wid; b < bpw; b += WPW) v += partial[((size_t)n * bpw + b) * RAWS + s];
+      part[wid][s] = v;
+    }
+    __syncthreads();
+    if (wid != 0) return;
+  }
   float m00 = 0.f, mxy = 0.f, mxx = 0.f;
   const int sh0 = shift[3 * n], sh1 = shift[3 * n + 1];
   for (int s = lane; s < RAWS; s += 32) {
     float v = 0.f;
-    for (int b = 0; b < bpw; ++b) v += partial[((size_t)n * bpw + b) * RAWS + s];
+    if constexpr (WPW > 1) {
+#pragma unroll
+      for (int w = 0; w < WPW; ++w) v += part[w][s];
+    } else {
+      for (int b = 0; b < bpw; ++b) v += partial[((size_t)n * bpw + b) * RAWS + s];
+    }
     if (s == RAW_BORDER) v = v > 0.f ? 1.f : 0.f;
     if (s == RAW_SHIFT) v = (float)sh0;
     if (s == RAW_SHIFT + 1) v = (float)sh1;
@@ -725,16 +992,70 @@ __global__ void prepare_streamed_kernel(long n_planes, const float2* __restrict_
   }
 }
 
+// Worlds up to which the row inverse is split over channels and kernels: as
+// many as the walking kernel gives less than a block an SM.  Measured, us for
+// a 16-step rollout with both kernels of 3 channels x 15 kernels (walking ->
+// split; the split column includes col_conv_split): 128^2: 1 world
+// 1037 -> 482, 16 1106 -> 814, 32 (128 blocks) 1143 -> 1077, 64 1383 -> 1745;
+// 64^2: 64 worlds 1235 -> 864, 256 1610 -> 1880; 256^2: 4 worlds 1090 -> 868,
+// 16 1406 -> 1842; one channel and kernel, 256^2: 8 worlds 535 -> 520, 16
+// 577 -> 646.  At 512^2 a lane holds 32 points and the lines cross earlier:
+// 3 x 9, 1 world 1198 -> 900, 2 (64 blocks) 1285 -> 1275, 4 1561 -> 2063.
+template <int N>
+constexpr int split_worlds() {
+  return (N == 512 ? 64 : 128) / RowInvCfg<N>::BPW;
+}
+
+template <int N>
+int partials_per_world(int C, int n_worlds) {
+  return n_worlds <= split_worlds<N>() ? SplitCfg<N>::BPC * C : RowInvCfg<N>::BPW;
+}
+
+// Floats of row-inverse partials for up to n_worlds worlds a launch.
+template <int N>
+size_t partial_floats(int C, int n_worlds) {
+  const size_t split = (size_t)std::min(n_worlds, split_worlds<N>()) * SplitCfg<N>::BPC * C;
+  return std::max(split, (size_t)n_worlds * RowInvCfg<N>::BPW) * raw_stride(C);
+}
+
 template <int N, int GF>
 cudaError_t launch_row_inv(const StreamedStep& s, const KTab& tab, cudaStream_t st) {
+  float2* spec_next = s.emit_spec ? s.spec : nullptr;
+  if (s.n_worlds <= split_worlds<N>()) {
+    const int warps = std::min(kSplitMaxWarps, std::max(kSplitMinWarps, tab.K));
+    const size_t smem = row_inv_split_smem<N>(warps);
+    cudaError_t e = cudaFuncSetAttribute(row_inv_split_kernel<N, GF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)row_inv_split_smem<N>(kSplitMaxWarps));
+    if (e != cudaSuccess) return e;
+    row_inv_split_kernel<N, GF><<<(unsigned)(s.n_worlds * tab.C * SplitCfg<N>::BPC), 32 * warps, smem, st>>>(
+        s.n_worlds, s.n_init, tab, s.prod, s.gf, s.gf_sol_stride, s.w, s.w_sol_stride, s.dt, s.state, s.state_out,
+        s.field_out, s.pot_out, s.shift, s.partial, spec_next);
+    return cudaGetLastError();
+  }
   using RC = RowInvCfg<N>;
   const size_t sm_inv = row_inv_smem<N>(tab.C, tab.K);
   cudaError_t e = cudaFuncSetAttribute(row_inv_kernel<N, GF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_inv);
   if (e != cudaSuccess) return e;
   row_inv_kernel<N, GF><<<(unsigned)((long)s.n_worlds * RC::BPW), RC::T, sm_inv, st>>>(
       s.n_worlds, s.n_init, tab, s.prod, s.gf, s.gf_sol_stride, s.w, s.w_sol_stride, s.dt, s.state, s.state_out,
-      s.field_out, s.pot_out, s.shift, s.partial, s.status, s.emit_spec ? s.spec : nullptr);
+      s.field_out, s.pot_out, s.shift, s.partial, s.status, spec_next);
   return cudaGetLastError();
+}
+
+// Blocks sharing one column tile's kernels (gridDim.y): as many as there are
+// kernels on a channel while the grid stays within two blocks an SM (more
+// would only repeat the forward transform).  Five kernels a channel, one
+// 128^2 world of three channels: 12 us on 12 blocks, 6.5 us on 60.
+constexpr long kColBlocks = 304;
+
+int col_conv_split(const Model& m, long blocks) {
+  int per_channel = 0;
+  for (int c = 0; c < m.C; ++c) {
+    int n = 0;
+    for (int k = 0; k < m.K; ++k) n += m.cin[k] == c ? 1 : 0;
+    per_channel = std::max(per_channel, n);
+  }
+  return (int)std::max(1L, std::min((long)per_channel, kColBlocks / blocks));
 }
 
 // cuTensorMapEncodeTiled, fetched once from the driver through the runtime.
@@ -800,9 +1121,9 @@ cudaError_t step_n(const StreamedStep& s, cudaStream_t st) {
   if (!encode_spec_map<N>(&prod_map, s.prod, (long)s.n_worlds * m.K)) return cudaErrorInvalidValue;
   if (!s.spec_ready)  // otherwise the previous step's row inverse already wrote this step's row spectra
     row_fwd_kernel<N><<<(unsigned)(planes * BPP), kThreads, sm_fwd, st>>>(s.n_worlds, m.C, s.state, s.spec);
-  col_conv_kernel<N><<<(unsigned)(planes * CC::BPP), CC::T, sm_col, st>>>(spec_map, prod_map, s.n_worlds, s.n_init,
-                                                                          tab, s.kp, s.kp_sol_stride, s.status);
-  using RC = RowInvCfg<N>;
+  const dim3 col_grid((unsigned)(planes * CC::BPP), (unsigned)col_conv_split(m, planes * CC::BPP));
+  col_conv_kernel<N><<<col_grid, CC::T, sm_col, st>>>(spec_map, prod_map, s.n_worlds, s.n_init, tab, s.kp,
+                                                      s.kp_sol_stride, s.status);
   bool all_gauss = true, all_poly = true;
   for (int k = 0; k < m.K; ++k) {
     all_gauss = all_gauss && m.gf[k] == LGX_GF_GAUSSIAN;
@@ -812,7 +1133,7 @@ cudaError_t step_n(const StreamedStep& s, cudaStream_t st) {
   else if (all_poly) e = launch_row_inv<N, GF_FAST_POLY4>(s, tab, st);
   else e = launch_row_inv<N, GF_GENERIC>(s, tab, st);
   if (e != cudaSuccess) return e;
-  return launch_streamed_reduce(s, RC::BPW, st);
+  return launch_streamed_reduce(s, partials_per_world<N>(m.C, s.n_worlds), st);
 }
 
 }  // namespace
@@ -824,15 +1145,15 @@ bool streamed_supported(const Model& m) {
   return true;
 }
 
-int streamed_blocks_per_world(const Model& m) {
+size_t streamed_partial_floats(const Model& m, int n_worlds) {
   switch (m.H) {
-    case 32: return RowInvCfg<32>::BPW;
-    case 64: return RowInvCfg<64>::BPW;
-    case 128: return RowInvCfg<128>::BPW;
-    case 256: return RowInvCfg<256>::BPW;
-    case 512: return RowInvCfg<512>::BPW;
+    case 32: return partial_floats<32>(m.C, n_worlds);
+    case 64: return partial_floats<64>(m.C, n_worlds);
+    case 128: return partial_floats<128>(m.C, n_worlds);
+    case 256: return partial_floats<256>(m.C, n_worlds);
+    case 512: return partial_floats<512>(m.C, n_worlds);
   }
-  return generic_blocks_per_world(m.H);  // generic sizes: a few packed rows per block
+  return (size_t)n_worlds * generic_blocks_per_world(m.H) * raw_stride(m.C);  // a few packed rows per block
 }
 
 size_t streamed_workspace_bytes(const Model& m, int n_worlds, int n_sols) {
@@ -842,16 +1163,19 @@ size_t streamed_workspace_bytes(const Model& m, int n_worlds, int n_sols) {
   b += al(plane * n_worlds * m.C);                                          // spec
   b += al(plane * n_worlds * m.K);                                          // prod
   b += al((size_t)n_sols * m.C * m.max_k * m.H * (m.W / 2 + 2) * sizeof(float2));  // kp
-  b += al((size_t)n_worlds * streamed_blocks_per_world(m) * raw_stride(m.C) * sizeof(float));  // partial
+  b += al(streamed_partial_floats(m, n_worlds) * sizeof(float));  // partial
   b += al((size_t)n_worlds * 3 * sizeof(int));                              // shift
   return b;
 }
 
 cudaError_t launch_streamed_reduce(const StreamedStep& s, int bpw, cudaStream_t st) {
-  const int wpb = 8;
-  reduce_kernel<<<(s.n_worlds + wpb - 1) / wpb, 32 * wpb, 0, st>>>(s.n_worlds, s.n_init, bpw, s.m->C, s.m->H, s.m->W,
-                                                                  s.partial, s.raw, s.raw_sol_stride,
-                                                                  s.raw_world_stride, s.shift);
+  const Model& m = *s.m;
+  if (bpw >= 2 * kReduceWarps)
+    reduce_kernel<kReduceWarps><<<s.n_worlds, 32 * kReduceWarps, 0, st>>>(
+        s.n_worlds, s.n_init, bpw, m.C, m.H, m.W, s.partial, s.raw, s.raw_sol_stride, s.raw_world_stride, s.shift);
+  else
+    reduce_kernel<1><<<(s.n_worlds + kReduceWarps - 1) / kReduceWarps, 32 * kReduceWarps, 0, st>>>(
+        s.n_worlds, s.n_init, bpw, m.C, m.H, m.W, s.partial, s.raw, s.raw_sol_stride, s.raw_world_stride, s.shift);
   return cudaGetLastError();
 }
 
