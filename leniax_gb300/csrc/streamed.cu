@@ -334,9 +334,9 @@ __device__ __forceinline__ void unpack_row_pair_q1(const float2* row, float2 (&v
 // Block = GPB groups = GPB packed rows of one world.  Work items are the
 // (output channel, kernel) pairs with a nonzero weight, channel by channel,
 // then the kernels that feed no channel (their potentials still count in
-// potential_volume).  Item i's GPB product rows are bulk-copied into buffer
-// i & 1 (row pitch N + G) while item i-1 is transformed; after unpacking its
-// row, a group reuses that row as its FFT exchange scratch.  The weighted
+// potential_volume).  A warp's product rows of item i are bulk-copied into its
+// buffer i & 1 (row pitch N + G) while item i-1 is transformed; after
+// unpacking its row, a group reuses that row as its FFT exchange scratch.  The weighted
 // field of the current channel stays in registers (2*P values per thread); a
 // kernel feeding several channels is transformed once per channel, its
 // potential counted (and written) at the first.
@@ -346,10 +346,20 @@ struct RowInvCfg {
   static constexpr int T = ((N / 2) * G < 128) ? (N / 2) * G : 128;  // threads per block
   static constexpr int GPB = T / G;
   static constexpr int BPW = (N / 2) / GPB;  // blocks per world
+  static constexpr int WROWS = 32 / G;       // packed rows per warp
   static constexpr int ROWP = N + G;         // staged row pitch (float2) == Geo<N, G>::SCR
-  static constexpr int BUF = GPB * ROWP;     // float2 per buffer
+  static constexpr int BUF = WROWS * ROWP;   // float2 per warp and ring slot
   static constexpr int NBUF = 2;             // staging ring depth (items in flight: NBUF - 1)
   static constexpr int SSTP = 2 * N + 16;    // staged state rows (2r, 2r+1) pitch per group (floats)
+  static constexpr int TABS = Geo<N, G>::Q == 1 ? 1 : 2;  // twiddle tables: std, rowi (the same one when Q == 1)
+  // resident blocks an SM asked of the compiler: 128 registers a thread and
+  // the 56 KB a block that four of them may have (a lane of 512^2 holds 32
+  // points and keeps what it needs).  Issue slots were 46% busy with three
+  // blocks and block barriers between the items; 8-step rollouts of 3 x 15
+  // kernels, us before -> now: 256 worlds of 256^2 5628 -> 5408, 128 of 128^2
+  // 1268 -> 1030, 2048 of 64^2 3744 -> 3333; one kernel, 64 of 256^2 551 -> 500.
+  // Three blocks without the block barriers: 5488, 1212, 3407, 537.
+  static constexpr int MINB = N == 512 ? 1 : 512 / T;
 };
 
 // item word: bit 16 = count the potential, bits 8..15 = output channel + 1 (0: none), bits 0..7 = kernel
@@ -360,15 +370,15 @@ __device__ __forceinline__ bool item_count(int it) { return (it >> 16) & 1; }
 template <int N>
 size_t row_inv_smem(int C, int K) {
   using RC = RowInvCfg<N>;
-  return (size_t)RC::NBUF * RC::BUF * sizeof(float2) + (size_t)RC::GPB * RC::SSTP * sizeof(float) +
-         (size_t)3 * N * sizeof(float2) +
+  return (size_t)(RC::T / 32) * RC::NBUF * RC::BUF * sizeof(float2) + (size_t)RC::GPB * RC::SSTP * sizeof(float) +
+         (size_t)RC::TABS * N * sizeof(float2) +
          (size_t)(RC::T / 32) * (RAW_CM + kMaxChannels) * sizeof(float) + 16 * sizeof(uint64_t) +
          (size_t)kMaxChannels * sizeof(float) + (size_t)(C * K + K + 1) * sizeof(int) +
          (size_t)(C * K + K + 1) * sizeof(float4) + (size_t)(C * K + 2 * K) * sizeof(float);
 }
 
 template <int N, int GF>
-__global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
+__global__ void __launch_bounds__(RowInvCfg<N>::T, RowInvCfg<N>::MINB) row_inv_kernel(
     int n_worlds, int n_init, KTab tab, const float2* __restrict__ prod, const float* __restrict__ gfp,
     long gf_sol_stride, const float* __restrict__ wts, long w_sol_stride, const float* __restrict__ dtp,
     const float* __restrict__ state, float* __restrict__ state_out, float* __restrict__ field_out,
@@ -382,12 +392,13 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
   constexpr int NWARPS = RC::T / 32;
   static_assert(ROWP == GE::SCR, "a staged row doubles as the group's FFT scratch");
   extern __shared__ __align__(16) float2 sm[];
-  float2* bufs = sm;                    // [NBUF][GPB][ROWP] staging ring
-  float* sst = reinterpret_cast<float*>(bufs + NBUF * RC::BUF);  // [GPB][SSTP] the channel's state rows
-  float2* tw = reinterpret_cast<float2*>(sst + GPB * RC::SSTP);  // 3N twiddles
-  float* red = reinterpret_cast<float*>(tw + 3 * N);  // [warps][RAWS_MAX]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(red + NWARPS * RAWS_MAX);  // NBUF ring + 1 state (16 reserved)
-  float* wsum_s = reinterpret_cast<float*>(bars + 16);  // [kMaxChannels]
+  static_assert(NWARPS * (NBUF + 1) <= 16, "mbarriers reserved");
+  float* sst = reinterpret_cast<float*>(sm + NWARPS * NBUF * RC::BUF);  // past the rings: [GPB][SSTP] state rows
+  float2* tw = reinterpret_cast<float2*>(sst + GPB * RC::SSTP);  // twiddle tables
+  float2* tw_rowi = tw + (RC::TABS - 1) * N;
+  float* red = reinterpret_cast<float*>(tw + RC::TABS * N);  // [warps][RAWS_MAX]
+  uint64_t* bars_all = reinterpret_cast<uint64_t*>(red + NWARPS * RAWS_MAX);  // [warps][ring, state] (16 reserved)
+  float* wsum_s = reinterpret_cast<float*>(bars_all + 16);  // [kMaxChannels]
   float4* ipar = reinterpret_cast<float4*>(wsum_s + kMaxChannels);  // [C*K + K + 1] per item: weight, m, s, a
   __shared__ int s_nitems;
 
@@ -398,6 +409,8 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
   const int r0 = (blockIdx.x % BPW) * GPB;
   const int r = r0 + grp;
   const unsigned gmask = ((1u << G) - 1u) << (lane & ~(G - 1));
+  float2* bufs = sm + wid * NBUF * RC::BUF;  // this warp's ring [NBUF][WROWS][ROWP]
+  uint64_t* bars = bars_all + wid * (NBUF + 1);
   const int C = tab.C, K = tab.K;
   const float* gf = gfp + sol * gf_sol_stride;
   const float* wt = wts + sol * w_sol_stride;
@@ -407,10 +420,10 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
   // the solution's weights and growth parameters, one coalesced pass
   for (int q = threadIdx.x; q < C * K + 2 * K; q += blockDim.x)
     wgf[q] = q < C * K ? __ldg(wt + q) : __ldg(gf + (q - C * K));
-  init_twiddles<GE>(tw, tw + N, tw + 2 * N, threadIdx.x, blockDim.x);
+  init_twiddles<GE>(tw, tw_rowi, tw_rowi, threadIdx.x, blockDim.x);
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int b = 0; b <= NBUF; ++b) mbar_init(&bars[b], 1);
+    for (int b = 0; b < NWARPS * (NBUF + 1); ++b) mbar_init(&bars_all[b], 1);
     fence_proxy_async();
     // work items with their growth parameters, and per-channel weight sums
     int ni = 0;
@@ -444,26 +457,27 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
   __syncthreads();
   const int nit = s_nitems;
 
-  // warp 0 stages item i's GPB product rows into ring slot i % NBUF
+  // the warp stages its rows of item i into ring slot i % NBUF
+  const float2* rows0 = prod + ((size_t)n * K * (N / 2) + r0 + wid * RC::WROWS) * N;
   auto issue = [&](int i) {
     const int b = i % NBUF;
-    const float2* src = prod + (((size_t)n * K + item_k(items[i])) * (N / 2) + r0) * N;
+    const float2* src = rows0 + (size_t)item_k(items[i]) * (N / 2) * N;
     float2* dst = bufs + b * RC::BUF;
-    if (lane == 0) mbar_arrive_expect_tx(&bars[b], (unsigned)(GPB * N * sizeof(float2)));
+    if (lane == 0) mbar_arrive_expect_tx(&bars[b], (unsigned)(RC::WROWS * N * sizeof(float2)));
     __syncwarp();
-    for (int g = lane; g < GPB; g += 32) bulk_load(dst + g * ROWP, src + (size_t)g * N, N * sizeof(float2), &bars[b]);
+    if (lane < RC::WROWS) bulk_load(dst + lane * ROWP, src + (size_t)lane * N, N * sizeof(float2), &bars[b]);
   };
-  // warp 0 stages channel co's state rows (2r, 2r+1) of every group into sst
+  // ... and channel co's state rows (2r, 2r+1) into sst
+  float* sst_w = sst + wid * RC::WROWS * RC::SSTP;
   auto issue_state = [&](int co) {
-    const float* src = state + (((size_t)n * C + co) * N + 2 * r0) * N;
-    if (lane == 0) mbar_arrive_expect_tx(&bars[NBUF], (unsigned)(GPB * 2 * N * sizeof(float)));
+    const float* src = state + (((size_t)n * C + co) * N + 2 * (r0 + wid * RC::WROWS)) * N;
+    if (lane == 0) mbar_arrive_expect_tx(&bars[NBUF], (unsigned)(RC::WROWS * 2 * N * sizeof(float)));
     __syncwarp();
-    for (int g = lane; g < GPB; g += 32)
-      bulk_load(sst + g * RC::SSTP, src + (size_t)g * 2 * N, 2 * N * sizeof(float), &bars[NBUF]);
+    if (lane < RC::WROWS)
+      bulk_load(sst_w + lane * RC::SSTP, src + (size_t)lane * 2 * N, 2 * N * sizeof(float), &bars[NBUF]);
   };
-  if (wid == 0)
-    for (int q = 0; q < NBUF - 1 && q < nit; ++q) issue(q);
-  int st_issued = 0, st_done = 0;  // state-row copies issued / waited for (block-uniform)
+  for (int q = 0; q < NBUF - 1 && q < nit; ++q) issue(q);
+  int st_issued = 0, st_done = 0;  // state-row copies issued / waited for (warp-uniform)
 
   float dt;
   if (tab.dt_mode == 0) dt = __ldg(dtp);
@@ -480,28 +494,27 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
   int failed_at = 0;
 
   // item i: wait for its rows, inverse row transform, count / write the
-  // potential, accumulate the weighted growth of channel co (co >= 0)
-  // One block barrier per item: past it, item i has landed for every thread
-  // and every group is done with slot (i - 1) % NBUF (item i - 1, or the
-  // fused row FFT's scratch), so warp 0 refills that slot with item
-  // i + NBUF - 1.
+  // potential, accumulate the weighted growth of channel co (co >= 0).  A warp
+  // stages, waits for and reuses its own rows, so no block barrier stands
+  // between the items: past the warp barrier every lane is done with slot
+  // (i - 1) % NBUF (item i - 1, or the fused row FFT's scratch), and the warp
+  // refills that slot with item i + NBUF - 1.
   auto process = [&](int i) {
-    if (__syncthreads_or(!mbar_wait(&bars[i % NBUF], (i / NBUF) & 1))) {
+    if (__any_sync(0xffffffffu, !mbar_wait(&bars[i % NBUF], (i / NBUF) & 1))) {
       failed = true;
       failed_at = i;
       return;
     }
     const int it = items[i], k = item_k(it), co = item_co(it);
+    fence_proxy_async();
+    if (i + NBUF - 1 < nit) issue(i + NBUF - 1);
     // a channel's first item: its state rows start moving (the previous
-    // channel's epilogue, the last reader of sst, is behind the barrier)
-    const bool first = co >= 0 && (i == 0 || item_co(items[i - 1]) != co);
-    st_issued += first ? 1 : 0;
-    if (wid == 0) {
-      fence_proxy_async();
-      if (i + NBUF - 1 < nit) issue(i + NBUF - 1);
-      if (first) issue_state(co);
+    // channel's epilogue, the last reader of sst, is behind the warp barrier)
+    if (co >= 0 && (i == 0 || item_co(items[i - 1]) != co)) {
+      ++st_issued;
+      issue_state(co);
     }
-    float2* row = bufs + (i % NBUF) * RC::BUF + grp * ROWP;
+    float2* row = bufs + (i % NBUF) * RC::BUF + (lane / G) * ROWP;
     float2 v[Q][G];
     if constexpr (Q == 1) {
       unpack_row_pair_q1<GE>(row, v, t);
@@ -510,7 +523,7 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
     }
     __syncwarp(gmask);
     float2 w[P];
-    fft_mirrored<GE, true, true>(v, w, row, tw + 2 * N, t, gmask);
+    fft_mirrored<GE, true, true>(v, w, row, tw_rowi, t, gmask);
     if (item_count(it)) {
 #pragma unroll
       for (int k1 = 0; k1 < P; ++k1) cpot += (w[k1].x > kEps ? 1.f : 0.f) + (w[k1].y > kEps ? 1.f : 0.f);
@@ -551,14 +564,12 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
     while (!failed && i < nit && item_co(items[i]) == co) process(i++);
     if (failed) break;
     if (i == i_begin) {  // a channel no kernel feeds: fetch its state rows here
-      __syncthreads();
+      __syncwarp();
       ++st_issued;
-      if (wid == 0) {
-        fence_proxy_async();
-        issue_state(co);
-      }
+      fence_proxy_async();
+      issue_state(co);
     }
-    if (__syncthreads_or(!mbar_wait(&bars[NBUF], (st_issued - 1) & 1))) {
+    if (__any_sync(0xffffffffu, !mbar_wait(&bars[NBUF], (st_issued - 1) & 1))) {
       failed = true;
       failed_at = i;
       break;
@@ -620,7 +631,8 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
       // (i - 1) % NBUF, the one slot with no copy in flight (items i ..
       // i + NBUF - 2 are); the next process() barrier orders it before reuse.
       float2 u[Q][G];
-      fft_standard<GE, false, false>(nsv, u, bufs + ((i + NBUF - 1) % NBUF) * RC::BUF + grp * ROWP, tw, t, gmask);
+      fft_standard<GE, false, false>(nsv, u, bufs + ((i + NBUF - 1) % NBUF) * RC::BUF + (lane / G) * ROWP, tw, t,
+                                     gmask);
       float2* dst = spec_next + (((size_t)n * C + co) * (N / 2) + r) * N;
 #pragma unroll
       for (int q = 0; q < Q; ++q)
@@ -630,13 +642,12 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T) row_inv_kernel(
   }
   while (!failed && i < nit) process(i++);  // kernels that feed no channel
   if (failed) {
-    // a staged copy never landed: record it, give the copies in flight a
-    // bounded time to drain, leave without writing moments
-    if (threadIdx.x == 0 && status) atomicExch(status, kStatusCopyTimeout);
+    // a staged copy never landed: record it and give the warp's copies in
+    // flight a bounded time to drain; the status word marks the step's results
+    if (lane == 0 && status) atomicExch(status, kStatusCopyTimeout);
     const int f = failed_at;
     for (int q = f; q < f + NBUF - 1 && q < nit; ++q) mbar_wait(&bars[q % NBUF], (q / NBUF) & 1);  // issued: <= f + NBUF - 2
     if (st_issued > st_done) mbar_wait(&bars[NBUF], (st_issued - 1) & 1);
-    return;
   }
   // block reduction: warp shuffles then shared memory
   float accm[11] = {m00, g00, cpot, cmass, cgrow, mxy, mxx, gxy, gxx, m2y, m2x};
