@@ -101,10 +101,10 @@ constexpr int kLineStages = 8;
 
 // One world axis: an n-point line transform of m-point transforms (m == n, or
 // the Bluestein length m >= 2n - 1).  r: radices of the forward transform, the
-// inverse runs them backwards.  The ends take radices up to 16, the middle
-// stages (m > 256) up to 8.
+// inverse runs them backwards.  The ends take radices up to 10, the middle
+// stages (m > 100) up to 8; a `wide` axis' ends are 8, 9, 10, 12, 14, 15 or 16.
 struct LineAxis {
-  int n, m, stages;
+  int n, m, stages, wide;
   int r[kLineStages];
   int st[kLineStages], ist[kLineStages];   // twiddle step m / (Ns r) of every forward / inverse stage
   int ns[kLineStages], ins[kLineStages];   // Ns: product of the radices before the stage
@@ -114,16 +114,19 @@ struct LineAxis {
   const float2 *chirp, *bhat;              // Bluestein tables (n and m entries), else null
 };
 
+inline bool wide_radix(int r) { return (r >= 8 && r <= 10) || r == 12 || (r >= 14 && r <= 16); }
 inline bool line_radix(int r, bool end) {
   if (end) return r >= 2 && r <= 10;
   return r == 2 || r == 3 || r == 4 || r == 5 || r == 7 || r == 8;
 }
 
 // The fewest stages, then the smallest sum of radices.  Depth-first over the
-// stage list first, last, middle...; returns the number of stages or 0.
-inline int line_radices(int m, int* out) {
+// stage list first, last, middle...; returns the number of stages or 0.  wide:
+// both ends from the wide radices, two stages at least.
+inline int line_radices(int m, int* out, bool wide = false) {
   int best = 0, best_sum = 1 << 30, cur[kLineStages] = {0};
-  if (m >= 2 && line_radix(m, true)) {
+  auto end_radix = [=](int r) { return wide ? wide_radix(r) : line_radix(r, true); };
+  if (!wide && m >= 2 && line_radix(m, true)) {
     out[0] = m;
     out[1] = 1;
     return 2;
@@ -146,10 +149,10 @@ inline int line_radices(int m, int* out) {
         self(self, left / r, depth + 1, sum + r, r);
       }
   };
-  for (int a = 10; a >= 2; --a) {
-    if (m % a || !line_radix(a, true)) continue;
-    for (int b = a; b <= 10; ++b) {  // the larger radix last: the smaller one writes the exchange
-      if ((m / a) % b || !line_radix(b, true)) continue;
+  for (int a = wide ? 16 : 10; a >= 2; --a) {
+    if (m % a || !end_radix(a)) continue;
+    for (int b = a; b <= 16; ++b) {  // the larger radix last: the smaller one writes the exchange
+      if ((m / a) % b || !end_radix(b)) continue;
       cur[0] = a;
       cur[1] = b;
       middle(middle, m / a / b, 2, a + b, 8);
@@ -159,12 +162,27 @@ inline int line_radices(int m, int* out) {
 }
 
 // Axis of n-point lines with m-point transforms; `tables` as laid out by
-// line_table_elems.  False when m has no plan.
-inline bool make_line_axis(int n, int m, float2* tables, LineAxis* ax) {
+// line_table_elems.  False when m has no plan.  allow_wide: take the wide
+// radices where they bring four stages down to three (1024 = 8 8 16, 768 =
+// 8 12 8): one exchange and one rounding of the twiddles less, at 96 registers
+// a thread and two blocks an SM instead of 64 and three.  8-step rollouts, us,
+// plain -> wide: 19 worlds of 100 x 768 478 -> 451, of 768 x 100 455 -> 450;
+// 14 of 100 x 1024 513 -> 478, of 1024 x 100 486 -> 468.  Bringing three
+// stages down to two does not pay for the blocks: 100 x 144 431 -> 516,
+// 100 x 192 426 -> 470, 100 x 256 387 -> 407, 192 x 100 426 -> 449.
+inline bool make_line_axis(int n, int m, float2* tables, LineAxis* ax, bool allow_wide) {
   ax->n = n;
   ax->m = m;
   ax->stages = line_radices(m, ax->r);
   if (ax->stages == 0) return false;
+  ax->wide = 0;
+  int r[kLineStages];
+  const int stages = allow_wide && n == m && ax->stages > 3 ? line_radices(m, r, true) : 0;
+  if (stages > 0 && stages < ax->stages) {
+    ax->wide = 1;
+    ax->stages = stages;
+    std::copy(r, r + stages, ax->r);
+  }
   int ns = 1, ins = 1;
   for (int s = 0; s < ax->stages; ++s) {
     const int r = ax->r[s], ri = ax->r[ax->stages - 1 - s];
@@ -307,6 +325,22 @@ __device__ __forceinline__ void center_stage(int m, FastDivU div, int nl, const 
 }
 
 #define LGX_END_RADICES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10)
+#define LGX_WIDE_RADICES(X) X(8) X(9) X(10) X(12) X(14) X(15) X(16)
+
+// Which lines a kernel is compiled for.
+enum LineKind { LINE_PLAIN = 0, LINE_BLUESTEIN = 1, LINE_WIDE = 2 };
+inline LineKind line_kind(const LineAxis& ax) {
+  return ax.m != ax.n ? LINE_BLUESTEIN : (ax.wide ? LINE_WIDE : LINE_PLAIN);
+}
+// kernel<KIND...>(line_kind(ax)): f(ic<KIND>) picks the instance
+template <class F>
+auto for_line_kind(const LineAxis& ax, F&& f) {
+  switch (line_kind(ax)) {
+    case LINE_BLUESTEIN: return f(ic<LINE_BLUESTEIN>{});
+    case LINE_WIDE: return f(ic<LINE_WIDE>{});
+    default: return f(ic<LINE_PLAIN>{});
+  }
+}
 
 // What stage s >= 1 of the INV or forward transform reads from t.b[0].
 template <bool INV, bool LINES>
@@ -345,52 +379,79 @@ __device__ __forceinline__ void line_middle(const LineAxis& ax, const float2* tw
 
 // Stages 0 .. S-2 of a transform: `in` through the first butterfly into the
 // exchange, then the middle ones; ends on a barrier with the points in t.b[0].
-template <bool INV, bool LINES, class In>
+template <bool INV, bool LINES, bool WIDE = false, class In>
 __device__ __forceinline__ void line_head(const LineAxis& ax, const float2* tw, Tile& t, const In& in) {
   const int S = ax.stages;
   const XWrite<LINES> out{t.b[0], t.lp};
   const int r = INV ? ax.r[S - 1] : ax.r[0];
   const FastDivU div = LINES ? t.nld : (INV ? ax.nbd[S - 1] : ax.nbd[0]);
-  switch (r) {
+  if constexpr (WIDE) {
+    switch (r) {
 #define LGX_CASE(R) \
   case R: line_stage<R, 0, INV, LINES>(ax.m, 1, 0, div, div, t.nl, tw, in, out); break;
-    LGX_END_RADICES(LGX_CASE)
+      LGX_WIDE_RADICES(LGX_CASE)
 #undef LGX_CASE
+    }
+  } else {
+    switch (r) {
+#define LGX_CASE(R) \
+  case R: line_stage<R, 0, INV, LINES>(ax.m, 1, 0, div, div, t.nl, tw, in, out); break;
+      LGX_END_RADICES(LGX_CASE)
+#undef LGX_CASE
+    }
   }
   __syncthreads();
   line_middle<INV, LINES>(ax, tw, t);
 }
 
 // The last stage, from t.b[0] to `out`; no barrier at its end.
-template <bool INV, bool LINES, class Out>
+template <bool INV, bool LINES, bool WIDE = false, class Out>
 __device__ __forceinline__ void line_tail(const LineAxis& ax, const float2* tw, Tile& t, const Out& out) {
   const int S = ax.stages;
   const XRead<LINES> rd = line_reads<INV, LINES>(ax, t, S - 1);
   const int r = INV ? ax.r[0] : ax.r[S - 1];
   const FastDivU div = LINES ? t.nld : (INV ? ax.nbd[0] : ax.nbd[S - 1]);
-  switch (r) {
+  if constexpr (WIDE) {
+    switch (r) {
 #define LGX_CASE(R) \
   case R: line_stage<R, 2, INV, LINES>(ax.m, 1, 0, div, div, t.nl, tw, rd, out); break;
-    LGX_END_RADICES(LGX_CASE)
+      LGX_WIDE_RADICES(LGX_CASE)
 #undef LGX_CASE
+    }
+  } else {
+    switch (r) {
+#define LGX_CASE(R) \
+  case R: line_stage<R, 2, INV, LINES>(ax.m, 1, 0, div, div, t.nl, tw, rd, out); break;
+      LGX_END_RADICES(LGX_CASE)
+#undef LGX_CASE
+    }
   }
   t.swap();
 }
 
 // line_tail, `mid`, then the opposite transform's first stage; ends on a
 // barrier with the points of that transform in t.b[0].
-template <bool INV, bool LINES, class Mid>
+template <bool INV, bool LINES, bool WIDE = false, class Mid>
 __device__ __forceinline__ void line_center(const LineAxis& ax, const float2* tw, Tile& t, const Mid& mid) {
   const int S = ax.stages;
   const XRead<LINES> rd = line_reads<INV, LINES>(ax, t, S - 1);
   const XWrite<LINES> wr{t.b[1], t.lp};
   const int r = INV ? ax.r[0] : ax.r[S - 1];
   const FastDivU div = LINES ? t.nld : (INV ? ax.nbd[0] : ax.nbd[S - 1]);
-  switch (r) {
+  if constexpr (WIDE) {
+    switch (r) {
 #define LGX_CASE(R) \
   case R: center_stage<R, INV, LINES>(ax.m, div, t.nl, tw, rd, mid, wr); break;
-    LGX_END_RADICES(LGX_CASE)
+      LGX_WIDE_RADICES(LGX_CASE)
 #undef LGX_CASE
+    }
+  } else {
+    switch (r) {
+#define LGX_CASE(R) \
+  case R: center_stage<R, INV, LINES>(ax.m, div, t.nl, tw, rd, mid, wr); break;
+      LGX_END_RADICES(LGX_CASE)
+#undef LGX_CASE
+    }
   }
   __syncthreads();
   t.swap();
@@ -471,15 +532,15 @@ __device__ __forceinline__ EachIn<F> each_in(const F& f) { return EachIn<F>{f}; 
 template <class F>
 __device__ __forceinline__ EachOut<F> each_out(const F& f) { return EachOut<F>{f}; }
 
-// in1(l, i) -> out1(l, k, X_k) point by point, either kind of line.
-template <bool INV, bool LINES, bool BL, class In, class Out>
+// in1(l, i) -> out1(l, k, X_k) point by point, any kind of line.
+template <bool INV, bool LINES, int KIND, class In, class Out>
 __device__ __forceinline__ void line_fft(const LineAxis& ax, const float2* tw, Tile& t, const In& in1,
                                          const Out& out1) {
-  if constexpr (BL) {
+  if constexpr (KIND == LINE_BLUESTEIN) {
     line_bluestein<INV, LINES>(ax, tw, t, in1, out1);
   } else {
-    line_head<INV, LINES>(ax, tw, t, each_in(in1));
-    line_tail<INV, LINES>(ax, tw, t, each_out(out1));
+    line_head<INV, LINES, KIND == LINE_WIDE>(ax, tw, t, each_in(in1));
+    line_tail<INV, LINES, KIND == LINE_WIDE>(ax, tw, t, each_out(out1));
   }
 }
 

@@ -107,15 +107,16 @@ size_t table_bytes(int D, int H, int W) {
   return axis_table_bytes(W) + axis_table_bytes(H) + (D > 1 ? axis_table_bytes(D) : 0);
 }
 
-// The axes of a D x H x W world with their tables at `ws`.
+// The axes of a D x H x W world with their tables at `ws`.  The x and y axes
+// of 3D worlds stay plain: plane tiles hold lines of at most a few dozen.
 NdAxes make_axes(int D, int H, int W, void* ws) {
   NdAxes a{};
   char* p = static_cast<char*>(ws);
-  make_line_axis(W, transform_len(W), reinterpret_cast<float2*>(p), &a.x);
+  make_line_axis(W, transform_len(W), reinterpret_cast<float2*>(p), &a.x, D == 1);
   p += axis_table_bytes(W);
-  make_line_axis(H, transform_len(H), reinterpret_cast<float2*>(p), &a.y);
+  make_line_axis(H, transform_len(H), reinterpret_cast<float2*>(p), &a.y, D == 1);
   p += axis_table_bytes(H);
-  if (D > 1) make_line_axis(D, transform_len(D), reinterpret_cast<float2*>(p), &a.z);
+  if (D > 1) make_line_axis(D, transform_len(D), reinterpret_cast<float2*>(p), &a.z, true);
   return a;
 }
 
@@ -256,6 +257,9 @@ __device__ __forceinline__ float growth_du(int id, float u, float m, float s, fl
 template <int FK, int FC>
 __global__ void __launch_bounds__(kNT) nd_adj_point_kernel(NdTab t, AdjArgs a, int pb, float* __restrict__ pacc) {
   constexpr bool kFused = FK > 0;
+  depend_wait();
+  a.lam = after_wait(a.lam);
+  pacc = after_wait(pacc);
   const int C = kFused ? FC : t.C, K = kFused ? FK : t.K;
   const int w = blockIdx.x / pb, b = blockIdx.x % pb;
   const long chunk = (t.cells + pb - 1) / pb;
@@ -644,11 +648,11 @@ cudaError_t launch_nd_adjoint(const Model& m, const NdAdjoint& j, void* ws, cuda
     a.T = j.T;
     a.s_copy = ar + (size_t)nw * m.K * cells;
     if (fused) {
-      nd_adj_point_kernel<1, 1><<<(unsigned)(nw * pb), kNT, 0, st>>>(t, a, pb, pacc);
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      e = launch_dependent(nd_adj_point_kernel<1, 1>, (unsigned)(nw * pb), kNT, 0, st, t, a, pb, pacc);
+      if (e != cudaSuccess) return e;
     } else {
-      nd_adj_point_kernel<0, 0><<<(unsigned)(nw * pb), kNT, 0, st>>>(t, a, pb, pacc);
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      e = launch_dependent(nd_adj_point_kernel<0, 0>, (unsigned)(nw * pb), kNT, 0, st, t, a, pb, pacc);
+      if (e != cudaSuccess) return e;
       nd_adj_param_kernel<<<(unsigned)(nw * m.K * pb), kNT, 0, st>>>(t, j.n_init, pb, a.u, ar, bf, ff, j.gf_params,
                                                                        j.weights, pacc);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;

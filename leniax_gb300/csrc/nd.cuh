@@ -8,12 +8,14 @@
 
 #include "common.cuh"
 #include "engine.h"
+#include "launch.cuh"
 #include "line_fft.cuh"
 
 namespace lgx {
 
 constexpr int kNdThreads = 320;        // most threads of a transform block
-constexpr int kNdBlocksPerSm = 3;      // register budget: 64 a thread
+constexpr int kNdBlocksPerSm = 3;      // register budget: 64 a thread ...
+__host__ __device__ constexpr int nd_blocks(int kind) { return kind == LINE_WIDE ? 2 : kNdBlocksPerSm; }  // ... 96 wide
 constexpr int kNdMaxN = 4096;          // longest world axis (one 4096-point line per tile)
 constexpr int kBluesteinMaxN = 2048;   // longest axis with a prime factor above 7 (m <= 4096)
 constexpr int kMaxPts = 4096;          // complex points of one tile buffer
@@ -171,6 +173,13 @@ struct EpiShared {
   float tot[kRawMax];
   int last;
 };
+
+// The epilogue's inputs that the launches before it write.
+__device__ __forceinline__ void epi_after_wait(EpiArgs& a) {
+  a.state = after_wait(a.state);
+  a.P = after_wait(a.P);
+  a.shift = after_wait(a.shift);
+}
 
 // The warp's total of channel c's mass, kept for epi_finish.
 __device__ __forceinline__ void epi_channel_mass(EpiShared& sh, int c, float cm) {

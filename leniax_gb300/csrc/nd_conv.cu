@@ -29,8 +29,9 @@ __device__ __forceinline__ void conv_tile_init(Tile& t, const ConvTile& g, float
 }
 
 // forward: P[w, k] = IFFT_axis(FFT_axis(S[w, c_in(k)]) * K[sol, c_in(k), slot(k)])
-template <bool BL>
-__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_conv_kernel(NdTab t, ConvArgs a, ConvTile g, LineAxis ax) {
+template <int KIND>
+__global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_conv_kernel(NdTab t, ConvArgs a, ConvTile g, LineAxis ax) {
+  constexpr bool BL = KIND == LINE_BLUESTEIN, WIDE = KIND == LINE_WIDE;
   extern __shared__ __align__(16) float2 sm[];
   float2* tw = sm;
   Tile tl;
@@ -42,6 +43,8 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_conv_kernel(NdT
   const int sol = w / a.n_init, sp = g.sp;
   const int I = (int)g.I;
   load_line_twiddles(tw, ax);
+  depend_wait();
+  a.S = after_wait(a.S);
   __syncthreads();
   const float2 zero = make_float2(0.f, 0.f);
   for (int c = 0; c < t.C; ++c) {
@@ -63,8 +66,8 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_conv_kernel(NdT
     };
     if (!BL && nk == 1) {
       const float2* __restrict__ kk = Kc + (long)t.slot[first] * t.hcells;
-      line_head<false, true>(ax, tw, tl, each_in(load));
-      line_center<false, true>(ax, tw, tl, [=](int l, int j, int nb, auto& v) {
+      line_head<false, true, WIDE>(ax, tw, tl, each_in(load));
+      line_center<false, true, WIDE>(ax, tw, tl, [=](int l, int j, int nb, auto& v) {
         constexpr int R = (int)(sizeof(v) / sizeof(float2));
         float2 s[R];
 #pragma unroll
@@ -75,14 +78,14 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_conv_kernel(NdT
       });
       line_middle<true, true>(ax, tw, tl);
       const auto store = store_to(first);
-      line_tail<true, true>(ax, tw, tl, each_out(store));
+      line_tail<true, true, WIDE>(ax, tw, tl, each_out(store));
     } else {
-      line_fft<false, true, BL>(ax, tw, tl, load, [=](int l, int i, float2 v) { Sc[i * sp + l] = v; });
+      line_fft<false, true, KIND>(ax, tw, tl, load, [=](int l, int i, float2 v) { Sc[i * sp + l] = v; });
       __syncthreads();
       for (int k = first; k < t.K; ++k) {
         if (t.cin[k] != c) continue;
         const float2* __restrict__ kk = Kc + (long)t.slot[k] * t.hcells;
-        line_fft<true, true, BL>(
+        line_fft<true, true, KIND>(
             ax, tw, tl,
             [=](int l, int i) { return l < lines ? cmul(Sc[i * sp + l], __ldg(kk + l + (long)i * I)) : zero; },
             store_to(k));
@@ -96,8 +99,9 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_conv_kernel(NdT
 // gk[w, k] += A_k conj(S_c_in(k)) and Q[w, c] = IFFT_axis(sum_{k: c_in(k) = c}
 // A_k conj(K_k)) -- the last forward passes of a and of the state, the
 // spectral products and the first inverse pass of Q in one launch.
-template <bool BL>
-__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_adj_conv_kernel(NdTab t, ConvArgs a, ConvTile g, LineAxis ax) {
+template <int KIND>
+__global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_adj_conv_kernel(NdTab t, ConvArgs a, ConvTile g, LineAxis ax) {
+  constexpr bool BL = KIND == LINE_BLUESTEIN, WIDE = KIND == LINE_WIDE;
   extern __shared__ __align__(16) float2 sm[];
   float2* tw = sm;
   Tile tl;
@@ -110,6 +114,10 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_adj_conv_kernel
   const int sol = w / a.n_init, sp = g.sp;
   const int I = (int)g.I;
   load_line_twiddles(tw, ax);
+  depend_wait();
+  a.S = after_wait(a.S);
+  a.A = after_wait(a.A);
+  a.gk = after_wait(a.gk);
   __syncthreads();
   const float2 zero = make_float2(0.f, 0.f);
   for (int c = 0; c < t.C; ++c) {
@@ -132,7 +140,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_adj_conv_kernel
       }
       continue;
     }
-    line_fft<false, true, BL>(
+    line_fft<false, true, KIND>(
         ax, tw, tl, [=](int l, int i) { return l < lines ? __ldg(S + l + (long)i * I) : zero; },
         [=](int l, int i, float2 v) {
           Sc[i * sp + l] = v;
@@ -146,8 +154,8 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_adj_conv_kernel
       float2* __restrict__ gk = a.gk + ((long)w * t.K + k) * t.hcells + i0;
       auto load = [=](int l, int i) { return l < lines ? __ldg(A + l + (long)i * I) : zero; };
       if (!BL && nk == 1) {
-        line_head<false, true>(ax, tw, tl, each_in(load));
-        line_center<false, true>(ax, tw, tl, [=](int l, int j, int nb, auto& v) {
+        line_head<false, true, WIDE>(ax, tw, tl, each_in(load));
+        line_center<false, true, WIDE>(ax, tw, tl, [=](int l, int j, int nb, auto& v) {
           constexpr int R = (int)(sizeof(v) / sizeof(float2));
           if (l >= lines) return true;  // zeros in, zeros out
           float2 s[R], o[R];
@@ -165,9 +173,9 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_adj_conv_kernel
           return true;
         });
         line_middle<true, true>(ax, tw, tl);
-        line_tail<true, true>(ax, tw, tl, each_out(store_q));
+        line_tail<true, true, WIDE>(ax, tw, tl, each_out(store_q));
       } else {
-        line_fft<false, true, BL>(ax, tw, tl, load, [=](int l, int i, float2 v) {
+        line_fft<false, true, KIND>(ax, tw, tl, load, [=](int l, int i, float2 v) {
           if (l >= lines) return;
           float2* gp = gk + l + (long)i * I;
           *gp = cadd(*gp, cmulc(v, Sc[i * sp + l]));
@@ -177,7 +185,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_adj_conv_kernel
     }
     __syncthreads();
     if (BL || nk > 1) {
-      line_fft<true, true, BL>(ax, tw, tl, [=](int l, int i) { return Qc[i * sp + l]; }, store_q);
+      line_fft<true, true, KIND>(ax, tw, tl, [=](int l, int i) { return Qc[i * sp + l]; }, store_q);
       __syncthreads();  // Sc and Qc are rewritten by the next channel
     }
   }
@@ -188,8 +196,8 @@ struct ColArgs {
   float2* data;
   ConvTile g;
 };
-template <bool INV, bool BL>
-__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_columns_kernel(ColArgs a, LineAxis ax) {
+template <bool INV, int KIND>
+__global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_columns_kernel(ColArgs a, LineAxis ax) {
   extern __shared__ __align__(16) float2 sm[];
   float2* tw = sm;
   Tile tl;
@@ -198,10 +206,13 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_columns_kernel(
   const long i0 = (long)(blockIdx.x - plane * a.g.tiles) * a.g.nl;
   const int lines = (int)min((long)a.g.nl, a.g.I - i0);
   const int I = (int)a.g.I;
+  depend_wait();
+  a.data = after_wait(a.data);
+  ax.tw = after_wait(ax.tw);
   load_line_twiddles(tw, ax);
   __syncthreads();
   float2* d = a.data + plane * a.g.I * ax.n + i0;
-  line_fft<INV, true, BL>(
+  line_fft<INV, true, KIND>(
       ax, tw, tl, [=](int l, int i) { return l < lines ? d[l + (long)i * I] : make_float2(0.f, 0.f); },
       [=](int l, int i, float2 v) {
         if (l < lines) d[l + (long)i * I] = v;
@@ -239,12 +250,12 @@ cudaError_t nd_convolve(bool adjoint, const NdTab& t, const LineAxis& ax, long n
   const size_t smem = (size_t)(ax.m + 2 * g.buf + keeps * g.keep) * sizeof(float2);
   const long blocks = nw * g.tiles;
   if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
-  auto f = adjoint ? (bl ? nd_adj_conv_kernel<true> : nd_adj_conv_kernel<false>)
-                   : (bl ? nd_conv_kernel<true> : nd_conv_kernel<false>);
+  auto f = for_line_kind(ax, [&](auto kind) {
+    return adjoint ? nd_adj_conv_kernel<decltype(kind)::value> : nd_conv_kernel<decltype(kind)::value>;
+  });
   const cudaError_t e = nd_allow_smem((const void*)f);
   if (e != cudaSuccess) return e;
-  f<<<(unsigned)blocks, nd_threads(line_items(ax, g.nl)), smem, st>>>(t, a, g, ax);
-  return cudaGetLastError();
+  return launch_dependent(f, (unsigned)blocks, nd_threads(line_items(ax, g.nl)), smem, st, t, a, g, ax);
 }
 
 cudaError_t nd_columns(bool inv, const NdTab& t, const LineAxis& y, long planes, float2* data, cudaStream_t st) {
@@ -252,16 +263,15 @@ cudaError_t nd_columns(bool inv, const NdTab& t, const LineAxis& y, long planes,
   a.data = data;
   const long groups = planes * t.D;
   a.g = conv_tile(y, groups, t.Wh);
-  const bool bl = y.m != y.n;
   const size_t smem = (size_t)(y.m + 2 * a.g.buf) * sizeof(float2);
   const long blocks = groups * a.g.tiles;
   if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
-  auto f = inv ? (bl ? nd_columns_kernel<true, true> : nd_columns_kernel<true, false>)
-               : (bl ? nd_columns_kernel<false, true> : nd_columns_kernel<false, false>);
+  auto f = for_line_kind(y, [&](auto kind) {
+    return inv ? nd_columns_kernel<true, decltype(kind)::value> : nd_columns_kernel<false, decltype(kind)::value>;
+  });
   const cudaError_t e = nd_allow_smem((const void*)f);
   if (e != cudaSuccess) return e;
-  f<<<(unsigned)blocks, nd_threads(line_items(y, a.g.nl)), smem, st>>>(a, y);
-  return cudaGetLastError();
+  return launch_dependent(f, (unsigned)blocks, nd_threads(line_items(y, a.g.nl)), smem, st, a, y);
 }
 
 }  // namespace lgx

@@ -99,6 +99,10 @@ struct PlaneArgs {
 __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_fwd_kernel(PlaneArgs a, PlaneGeo g, LineAxis ax,
                                                                      LineAxis ay) {
   extern __shared__ __align__(16) float2 sm[];
+  depend_wait();
+  a.src = after_wait(a.src);
+  ax.tw = after_wait(ax.tw);
+  ay.tw = after_wait(ay.tw);
   PlaneTile p = plane_init(g, ax, ay, sm);
   __syncthreads();
   const int H = a.H, W = a.W, Wh = a.Wh, zp = g.zp;
@@ -119,6 +123,11 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_fwd_kerne
 __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_inv_kernel(PlaneArgs a, PlaneGeo g, LineAxis ax,
                                                                      LineAxis ay) {
   extern __shared__ __align__(16) float2 sm[];
+  depend_wait();
+  a.half_in = after_wait(a.half_in);
+  a.dst = after_wait(a.dst);
+  ax.tw = after_wait(ax.tw);
+  ay.tw = after_wait(ay.tw);
   PlaneTile p = plane_init(g, ax, ay, sm);
   __syncthreads();
   const int H = a.H, W = a.W, Wh = a.Wh;
@@ -145,6 +154,8 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_epi_kerne
   __shared__ RowPair rp[kMaxTileLines];
   __shared__ EpiShared sh;
   PlaneTile p = plane_init(g, ax, ay, sm);
+  depend_wait();
+  epi_after_wait(a);
   const int w = blockIdx.x / t.D, z = blockIdx.x - w * t.D;
   const int sol = w / a.n_init;
   const int H = t.H, W = t.W, Wh = t.Wh, C = t.C, K = t.K, zp = g.zp;
@@ -305,8 +316,7 @@ cudaError_t nd_plane_forward(const NdTab& t, const NdAxes& ax, long planes, cons
   if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
   const cudaError_t e = nd_allow_smem((const void*)nd_plane_fwd_kernel);
   if (e != cudaSuccess) return e;
-  nd_plane_fwd_kernel<<<(unsigned)blocks, p.threads, p.smem, st>>>(a, p.g, ax.x, ax.y);
-  return cudaGetLastError();
+  return launch_dependent(nd_plane_fwd_kernel, (unsigned)blocks, p.threads, p.smem, st, a, p.g, ax.x, ax.y);
 }
 
 cudaError_t nd_plane_inverse(const NdTab& t, const NdAxes& ax, long planes, const float2* half, float* dst,
@@ -324,8 +334,7 @@ cudaError_t nd_plane_inverse(const NdTab& t, const NdAxes& ax, long planes, cons
   if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
   const cudaError_t e = nd_allow_smem((const void*)nd_plane_inv_kernel);
   if (e != cudaSuccess) return e;
-  nd_plane_inv_kernel<<<(unsigned)blocks, p.threads, p.smem, st>>>(a, p.g, ax.x, ax.y);
-  return cudaGetLastError();
+  return launch_dependent(nd_plane_inv_kernel, (unsigned)blocks, p.threads, p.smem, st, a, p.g, ax.x, ax.y);
 }
 
 cudaError_t nd_plane_epilogue(const NdTab& t, const NdAxes& ax, const EpiArgs& args, cudaStream_t st) {
@@ -339,8 +348,7 @@ cudaError_t nd_plane_epilogue(const NdTab& t, const NdAxes& ax, const EpiArgs& a
   auto f = t.C == 1 && t.K == 1 ? nd_plane_epi_kernel<true> : nd_plane_epi_kernel<false>;
   const cudaError_t e = nd_allow_smem((const void*)f);
   if (e != cudaSuccess) return e;
-  f<<<(unsigned)blocks, p.threads, smem, st>>>(t, a, p.g, ax.x, ax.y);
-  return cudaGetLastError();
+  return launch_dependent(f, (unsigned)blocks, p.threads, smem, st, t, a, p.g, ax.x, ax.y);
 }
 
 }  // namespace lgx

@@ -38,8 +38,8 @@ __device__ __forceinline__ void tile_pair(const RowsArgs& a, int l, long* row, i
   *n = min(2, a.rows - r0);
 }
 
-template <bool BL>
-__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_fwd_kernel(RowsArgs a, LineAxis ax) {
+template <int KIND>
+__global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_fwd_kernel(RowsArgs a, LineAxis ax) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ long row[kMaxTileLines];
   __shared__ int cnt[kMaxTileLines];
@@ -51,12 +51,15 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_fwd_kernel
   t.lp = a.pitch;
   t.nl = a.nr;
   t.nld = a.nrd;
+  depend_wait();
+  a.src = after_wait(a.src);
+  ax.tw = after_wait(ax.tw);
   load_line_twiddles(tw, ax);
   for (int l = threadIdx.x; l < a.nr; l += blockDim.x) tile_pair(a, l, row + l, cnt + l);
   __syncthreads();
   const float* __restrict__ src = a.src;
   const int W = a.W, zp = a.zp;
-  line_fft<false, false, BL>(
+  line_fft<false, false, KIND>(
       ax, tw, t,
       [&](int l, int i) {
         const float* p = src + row[l] * W + i;
@@ -76,8 +79,8 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_fwd_kernel
   }
 }
 
-template <bool BL>
-__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_inv_kernel(RowsArgs a, LineAxis ax) {
+template <int KIND>
+__global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_inv_kernel(RowsArgs a, LineAxis ax) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ long row[kMaxTileLines];
   __shared__ int cnt[kMaxTileLines];
@@ -88,12 +91,16 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_inv_kernel
   t.lp = a.pitch;
   t.nl = a.nr;
   t.nld = a.nrd;
+  depend_wait();
+  a.half_in = after_wait(a.half_in);
+  a.dst = after_wait(a.dst);
+  ax.tw = after_wait(ax.tw);
   load_line_twiddles(tw, ax);
   for (int l = threadIdx.x; l < a.nr; l += blockDim.x) tile_pair(a, l, row + l, cnt + l);
   __syncthreads();
   const float2* __restrict__ half = a.half_in;
   const int W = a.W, Wh = a.Wh;
-  line_fft<true, false, BL>(
+  line_fft<true, false, KIND>(
       ax, tw, t,
       [&](int l, int i) {
         const bool mir = i >= Wh;
@@ -168,8 +175,8 @@ struct RowsEpi {
 // new cells there.  Otherwise the weighted fields of the tile accumulate over
 // the kernels in F, and the update is the load rule of each channel's forward
 // transform.
-template <bool SINGLE, bool BL>
-__global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_epi_kernel(NdTab t, EpiArgs a, RowsEpi g, LineAxis ax) {
+template <bool SINGLE, int KIND>
+__global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kernel(NdTab t, EpiArgs a, RowsEpi g, LineAxis ax) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ RowPair rp[kMaxTileLines];
   __shared__ EpiShared sh;
@@ -184,12 +191,14 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_epi_kernel
   const int w = blockIdx.x / a.bpw, b = blockIdx.x - w * a.bpw;
   const int sol = w / a.n_init;
   const int W = t.W, Wh = t.Wh, C = t.C, K = t.K, zp = g.zp;
+  load_line_twiddles(tw, ax);
+  depend_wait();
+  epi_after_wait(a);
   const int s0 = a.shift[3 * w], s1 = a.shift[3 * w + 1], s2 = a.shift[3 * w + 2];
   const int sx = t.nd == 3 ? s2 : s1;
   const float dt = step_dt(t, a, w, sol);
   const float* gf = a.gf + sol * a.gf_sol_stride;
   const float* wt = a.w + sol * a.w_sol_stride;
-  load_line_twiddles(tw, ax);
   for (int l = threadIdx.x; l < g.nr; l += blockDim.x) {
     const int r0 = 2 * (b * g.nr + l), rows = max(0, min(2, t.D * t.H - r0));
     const int q0 = rows > 0 ? r0 : 0, q1 = rows > 1 ? r0 + 1 : q0;
@@ -247,13 +256,13 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_epi_kernel
   auto store_z = [=](int l, int k, float2 v) { Z[l * zp + k] = v; };
   if constexpr (SINGLE) {
     const auto rows0 = load_rows(0);
-    line_fft<true, false, BL>(ax, tw, tl, rows0, store_z);
+    line_fft<true, false, KIND>(ax, tw, tl, rows0, store_z);
     __syncthreads();
     epi_single(t, a, rp, Z, g.nr, zp, g.lanes, w, sx, dt, mo);
     const bool emit = a.S != nullptr;
     if (emit) {
       __syncthreads();
-      line_fft<false, false, BL>(
+      line_fft<false, false, KIND>(
           ax, tw, tl, [=](int l, int i) { return rp[l].rows ? Z[l * zp + i] : make_float2(0.f, 0.f); }, store_z);
     }
     epi_channel_mass(sh, 0, mo.m00);
@@ -269,7 +278,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_epi_kernel
     __syncthreads();
     for (int k = 0; k < K; ++k) {
       const NdGrowth grow(t.gf[k], __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1));
-      line_fft<true, false, BL>(ax, tw, tl, load_rows(k), [&](int l, int x, float2 v) {
+      line_fft<true, false, KIND>(ax, tw, tl, load_rows(k), [&](int l, int x, float2 v) {
         const int rows = rp[l].rows;
         if (rows == 0) return;
         const float2 u = make_float2(v.x * a.scale, v.y * a.scale);
@@ -302,7 +311,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_rows_epi_kernel
         return update(r, c, x, load_state(r, c, x), f);
       };
       if (a.S) {
-        line_fft<false, false, BL>(ax, tw, tl, new_cells, store_z);
+        line_fft<false, false, KIND>(ax, tw, tl, new_cells, store_z);
         __syncthreads();
         store_spectra(c);
         __syncthreads();  // Z is rewritten by the next channel
@@ -346,13 +355,10 @@ cudaError_t nd_rows_forward(const LineAxis& x, long planes, int rows, const floa
   a.src = src;
   a.half = half;
   const size_t smem = (size_t)(x.m + 2 * rt.buf + (long)rt.nr * rt.zp) * sizeof(float2);
-  const bool bl = x.m != x.n;
-  const void* f = bl ? (const void*)nd_rows_fwd_kernel<true> : (const void*)nd_rows_fwd_kernel<false>;
-  if ((e = nd_allow_smem(f)) != cudaSuccess) return e;
+  auto f = for_line_kind(x, [](auto kind) { return nd_rows_fwd_kernel<decltype(kind)::value>; });
+  if ((e = nd_allow_smem((const void*)f)) != cudaSuccess) return e;
   const unsigned blocks = (unsigned)((a.pairs + a.nr - 1) / a.nr);
-  if (bl) nd_rows_fwd_kernel<true><<<blocks, rt.threads, smem, st>>>(a, x);
-  else nd_rows_fwd_kernel<false><<<blocks, rt.threads, smem, st>>>(a, x);
-  return cudaGetLastError();
+  return launch_dependent(f, blocks, rt.threads, smem, st, a, x);
 }
 
 cudaError_t nd_rows_inverse(const LineAxis& x, long planes, int rows, const float2* half, float* dst, bool accumulate,
@@ -366,13 +372,10 @@ cudaError_t nd_rows_inverse(const LineAxis& x, long planes, int rows, const floa
   a.accumulate = accumulate ? 1 : 0;
   a.scale = scale;
   const size_t smem = (size_t)(x.m + 2 * rt.buf) * sizeof(float2);
-  const bool bl = x.m != x.n;
-  const void* f = bl ? (const void*)nd_rows_inv_kernel<true> : (const void*)nd_rows_inv_kernel<false>;
-  if ((e = nd_allow_smem(f)) != cudaSuccess) return e;
+  auto f = for_line_kind(x, [](auto kind) { return nd_rows_inv_kernel<decltype(kind)::value>; });
+  if ((e = nd_allow_smem((const void*)f)) != cudaSuccess) return e;
   const unsigned blocks = (unsigned)((a.pairs + a.nr - 1) / a.nr);
-  if (bl) nd_rows_inv_kernel<true><<<blocks, rt.threads, smem, st>>>(a, x);
-  else nd_rows_inv_kernel<false><<<blocks, rt.threads, smem, st>>>(a, x);
-  return cudaGetLastError();
+  return launch_dependent(f, blocks, rt.threads, smem, st, a, x);
 }
 
 int nd_rows_epi_blocks(const NdTab& t, const LineAxis& x, long n_worlds, long* field_pairs) {
@@ -398,13 +401,13 @@ cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& a
   g.field_smem = e.field_smem ? 1 : 0;
   const long blocks = (long)a.n_worlds * a.bpw;
   if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
-  const bool bl = x.m != x.n, single = t.C == 1 && t.K == 1;
-  auto f = single ? (bl ? nd_rows_epi_kernel<true, true> : nd_rows_epi_kernel<true, false>)
-                  : (bl ? nd_rows_epi_kernel<false, true> : nd_rows_epi_kernel<false, false>);
+  const bool single = t.C == 1 && t.K == 1;
+  auto f = for_line_kind(x, [&](auto kind) {
+    return single ? nd_rows_epi_kernel<true, decltype(kind)::value> : nd_rows_epi_kernel<false, decltype(kind)::value>;
+  });
   const cudaError_t err = nd_allow_smem((const void*)f);
   if (err != cudaSuccess) return err;
-  f<<<(unsigned)blocks, e.rt.threads, e.smem, st>>>(t, a, g, x);
-  return cudaGetLastError();
+  return launch_dependent(f, (unsigned)blocks, e.rt.threads, e.smem, st, t, a, g, x);
 }
 
 }  // namespace lgx

@@ -34,6 +34,7 @@
 #include "common.cuh"
 #include "engine.h"
 #include "fft.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace lgx {
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(kThreads) row_fwd_kernel(int n_worlds, int C, 
   constexpr int P = GE::P, Q = GE::Q, GPB = kThreads / G;  // groups per block
   constexpr int BPP = (N / 2 + GPB - 1) / GPB;             // blocks per plane
   extern __shared__ __align__(16) float2 sm[];
+  depend_trigger();  // an ordinary launch: all before it is complete
   float2* scr = init_tw<N>(sm);
   __syncthreads();
   const int plane = blockIdx.x / BPP;  // n*C + c
@@ -185,12 +187,16 @@ __global__ void __launch_bounds__(ColCfg<N>::T) col_conv_kernel(const __grid_con
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     fence_proxy_async();
-    mbar_arrive_expect_tx(&bar[0], CC::TILE_BYTES);
-    for (int b = 0; b < CC::BOXES; ++b)
-      tma_load_2d(tile + b * CC::BOX_BYTES, &spec_map, (j0 + 8 * b) * 4, plane * (N / 2), &bar[0]);
     if (CC::KSTAGE) issue_kernel(k_first);
   }
   init_twiddles<GE>(sm, sm + N, sm + 2 * N, threadIdx.x, blockDim.x);
+  depend_wait();
+  depend_trigger();
+  if (threadIdx.x == 0) {
+    mbar_arrive_expect_tx(&bar[0], CC::TILE_BYTES);
+    for (int b = 0; b < CC::BOXES; ++b)
+      tma_load_2d(tile + b * CC::BOX_BYTES, &spec_map, (j0 + 8 * b) * 4, plane * (N / 2), &bar[0]);
+  }
   __syncthreads();
   if (__syncthreads_or(!mbar_wait(&bar[0], 0))) {  // the tile never landed: record, drain, leave
     if (threadIdx.x == 0) {
@@ -456,6 +462,11 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T, RowInvCfg<N>::MINB) row_inv_k
   }
   __syncthreads();
   const int nit = s_nitems;
+  depend_wait();
+  depend_trigger();
+  prod = after_wait(prod);
+  state = after_wait(state);
+  shift = after_wait(shift);
 
   // the warp stages its rows of item i into ring slot i % NBUF
   const float2* rows0 = prod + ((size_t)n * K * (N / 2) + r0 + wid * RC::WROWS) * N;
@@ -761,6 +772,11 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
   const unsigned long long all = K == 64 ? ~0ull : (1ull << K) - 1ull;
   const unsigned long long mine = fed | (co == 0 ? all & ~any : 0ull);
 
+  depend_wait();
+  depend_trigger();
+  prod = after_wait(prod);
+  state = after_wait(state);
+  shift = after_wait(shift);
   float dt;
   if (tab.dt_mode == 0) dt = __ldg(dtp);
   else if (tab.dt_mode == 1) dt = __ldg(dtp + n);
@@ -931,6 +947,10 @@ __global__ void __launch_bounds__(32 * kReduceWarps) reduce_kernel(
   __shared__ float part[WPW > 1 ? WPW : 1][WPW > 1 ? RAWS_MAX : 1];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = blockIdx.x * (kReduceWarps / WPW) + wid / WPW;
+  depend_wait();
+  depend_trigger();
+  partial = after_wait(partial);
+  shift = after_wait(shift);
   if (n >= n_worlds) return;  // WPW > 1: one world a block, so whole blocks leave
   const int RAWS = raw_stride(C);
   const int sol = n / n_init, init = n - sol * n_init;
@@ -1038,19 +1058,17 @@ cudaError_t launch_row_inv(const StreamedStep& s, const KTab& tab, cudaStream_t 
     cudaError_t e = cudaFuncSetAttribute(row_inv_split_kernel<N, GF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)row_inv_split_smem<N>(kSplitMaxWarps));
     if (e != cudaSuccess) return e;
-    row_inv_split_kernel<N, GF><<<(unsigned)(s.n_worlds * tab.C * SplitCfg<N>::BPC), 32 * warps, smem, st>>>(
-        s.n_worlds, s.n_init, tab, s.prod, s.gf, s.gf_sol_stride, s.w, s.w_sol_stride, s.dt, s.state, s.state_out,
-        s.field_out, s.pot_out, s.shift, s.partial, spec_next);
-    return cudaGetLastError();
+    return launch_dependent(row_inv_split_kernel<N, GF>, (unsigned)(s.n_worlds * tab.C * SplitCfg<N>::BPC), 32 * warps,
+                            smem, st, s.n_worlds, s.n_init, tab, s.prod, s.gf, s.gf_sol_stride, s.w, s.w_sol_stride,
+                            s.dt, s.state, s.state_out, s.field_out, s.pot_out, s.shift, s.partial, spec_next);
   }
   using RC = RowInvCfg<N>;
   const size_t sm_inv = row_inv_smem<N>(tab.C, tab.K);
   cudaError_t e = cudaFuncSetAttribute(row_inv_kernel<N, GF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_inv);
   if (e != cudaSuccess) return e;
-  row_inv_kernel<N, GF><<<(unsigned)((long)s.n_worlds * RC::BPW), RC::T, sm_inv, st>>>(
-      s.n_worlds, s.n_init, tab, s.prod, s.gf, s.gf_sol_stride, s.w, s.w_sol_stride, s.dt, s.state, s.state_out,
-      s.field_out, s.pot_out, s.shift, s.partial, s.status, spec_next);
-  return cudaGetLastError();
+  return launch_dependent(row_inv_kernel<N, GF>, (unsigned)((long)s.n_worlds * RC::BPW), RC::T, sm_inv, st, s.n_worlds,
+                          s.n_init, tab, s.prod, s.gf, s.gf_sol_stride, s.w, s.w_sol_stride, s.dt, s.state,
+                          s.state_out, s.field_out, s.pot_out, s.shift, s.partial, s.status, spec_next);
 }
 
 // Blocks sharing one column tile's kernels (gridDim.y): as many as there are
@@ -1133,8 +1151,9 @@ cudaError_t step_n(const StreamedStep& s, cudaStream_t st) {
   if (!s.spec_ready)  // otherwise the previous step's row inverse already wrote this step's row spectra
     row_fwd_kernel<N><<<(unsigned)(planes * BPP), kThreads, sm_fwd, st>>>(s.n_worlds, m.C, s.state, s.spec);
   const dim3 col_grid((unsigned)(planes * CC::BPP), (unsigned)col_conv_split(m, planes * CC::BPP));
-  col_conv_kernel<N><<<col_grid, CC::T, sm_col, st>>>(spec_map, prod_map, s.n_worlds, s.n_init, tab, s.kp,
-                                                      s.kp_sol_stride, s.status);
+  e = launch_dependent(col_conv_kernel<N>, col_grid, CC::T, sm_col, st, spec_map, prod_map, s.n_worlds, s.n_init, tab,
+                       s.kp, s.kp_sol_stride, s.status);
+  if (e != cudaSuccess) return e;
   bool all_gauss = true, all_poly = true;
   for (int k = 0; k < m.K; ++k) {
     all_gauss = all_gauss && m.gf[k] == LGX_GF_GAUSSIAN;
@@ -1182,12 +1201,11 @@ size_t streamed_workspace_bytes(const Model& m, int n_worlds, int n_sols) {
 cudaError_t launch_streamed_reduce(const StreamedStep& s, int bpw, cudaStream_t st) {
   const Model& m = *s.m;
   if (bpw >= 2 * kReduceWarps)
-    reduce_kernel<kReduceWarps><<<s.n_worlds, 32 * kReduceWarps, 0, st>>>(
-        s.n_worlds, s.n_init, bpw, m.C, m.H, m.W, s.partial, s.raw, s.raw_sol_stride, s.raw_world_stride, s.shift);
-  else
-    reduce_kernel<1><<<(s.n_worlds + kReduceWarps - 1) / kReduceWarps, 32 * kReduceWarps, 0, st>>>(
-        s.n_worlds, s.n_init, bpw, m.C, m.H, m.W, s.partial, s.raw, s.raw_sol_stride, s.raw_world_stride, s.shift);
-  return cudaGetLastError();
+    return launch_dependent(reduce_kernel<kReduceWarps>, s.n_worlds, 32 * kReduceWarps, 0, st, s.n_worlds, s.n_init,
+                            bpw, m.C, m.H, m.W, s.partial, s.raw, s.raw_sol_stride, s.raw_world_stride, s.shift);
+  return launch_dependent(reduce_kernel<1>, (s.n_worlds + kReduceWarps - 1) / kReduceWarps, 32 * kReduceWarps, 0, st,
+                          s.n_worlds, s.n_init, bpw, m.C, m.H, m.W, s.partial, s.raw, s.raw_sol_stride,
+                          s.raw_world_stride, s.shift);
 }
 
 cudaError_t launch_streamed_step(const StreamedStep& s, cudaStream_t st) {
