@@ -102,6 +102,8 @@ def _engine_spectra(m, k_half: torch.Tensor) -> torch.Tensor:
     """Per-kernel half spectra ``[Ns, K, ...]`` placed at leniax's spectrum
     positions ``[Ns, C, max_k, ...]`` (kernels.py:122-152; padded slots zero)."""
     Ns = k_half.shape[0]
+    if [c * m.max_k + j for c, j in zip(m.cin, m.slot)] == list(range(m.C * m.max_k)):
+        return k_half.reshape((Ns, m.C, m.max_k) + tuple(k_half.shape[2:]))
     out = torch.zeros((Ns, m.C, m.max_k) + tuple(k_half.shape[2:]), dtype=k_half.dtype, device=k_half.device)
     for k, (c, j) in enumerate(zip(m.cin, m.slot)):
         out[:, c, j] = k_half[:, k]
@@ -184,10 +186,11 @@ class LeniaRolloutFunction(torch.autograd.Function):
         k = max(1, int(checkpoint_every))
         ckpts = [cells0.detach().contiguous()]
         cur = ckpts[0]
+        ws = _segment_workspace(m, Ns, Ni, min(k, steps), engine, dev) if steps else None
         done = 0
         while done < steps:
             n = min(k, steps - done)
-            cur = _segment(update_fn, cur, k_half, gf, w, Tt, n, traj=False, engine=engine)
+            cur = _segment(m, cur, k_half, gf, w, Tt, n, torch.empty_like(cur), ws, engine=engine)
             done += n
             if done < steps:
                 ckpts.append(cur)
@@ -224,71 +227,81 @@ class LeniaRolloutFunction(torch.autograd.Function):
         seg_starts = list(range(0, steps, k))
         # Segment j - 1's trajectory is recomputed on a side stream while
         # segment j's adjoint runs: the two launches take different SMs when
-        # a batch fills fewer than half of them.
+        # a batch fills fewer than half of them.  Two trajectory buffers serve
+        # all segments in turn (an allocation for each, freed across streams,
+        # cost the host more than its launches).
         main = torch.cuda.current_stream(dev)
         side = torch.cuda.Stream(device=dev)
+        slots = [(torch.empty((min(k, steps), Ns * Ni, m.C) + m.world, dtype=torch.float32, device=dev),
+                  torch.empty((min(k, steps), Ns * Ni, m.K) + m.world, dtype=torch.float32, device=dev))
+                 for _ in range(min(2, len(seg_starts)))]
+        read = [None, None]  # the adjoint that last read each slot
+        scratch = torch.empty_like(lam)
+        seg_ws = _segment_workspace(m, Ns, Ni, min(k, steps), ctx.engine, dev)
+        kh = torch.view_as_real(k_half.contiguous())
         side.wait_stream(main)
 
         def recompute(j):
+            slot = j % 2 if len(slots) > 1 else 0
+            if read[slot] is not None:
+                side.wait_event(read[slot])
             with torch.cuda.stream(side):
-                tr = _segment(update_fn, ckpts[j], k_half, gf, w, Tt, min(k, steps - seg_starts[j]), traj=True,
-                              engine=ctx.engine)
-                ev = torch.cuda.Event()
-                ev.record(side)
-            return tr, ev
+                _segment(m, ckpts[j], k_half, gf, w, Tt, min(k, steps - seg_starts[j]), scratch, seg_ws, slots[slot],
+                         engine=ctx.engine)
+            return slot, side.record_event()
 
-        kh = torch.view_as_real(k_half.contiguous())
-        nxt = recompute(len(seg_starts) - 1)
-        for j in reversed(range(len(seg_starts))):
-            n = min(k, steps - seg_starts[j])
-            (tc, tp), ready = nxt
-            if j > 0:
-                nxt = recompute(j - 1)
-            main.wait_event(ready)
-            tc.record_stream(main)
-            tp.record_stream(main)
-            job = AdjointJob()
-            job.n_sols, job.n_init, job.steps = Ns, Ni, n
-            job.k_half, job.gf_params, job.weights, job.T = (kh.data_ptr(), gf.data_ptr(), w.data_ptr(),
-                                                             Tt.data_ptr())
-            job.traj_cells, job.traj_potential = tc.data_ptr(), tp.data_ptr()
-            job.lambda_in, job.lambda_out = lam.data_ptr(), lam_out.data_ptr()
-            job.kernel_grad_acc = acc.data_ptr()
-            job.grad_gf, job.grad_weights = g_gf.data_ptr(), g_w.data_ptr()
-            job.clip_grad = ctx.clip
-            job.cells_after = after[j].data_ptr()
-            _lib.check(lib.lgx_adjoint(handle, job, ws.data_ptr(), ws.numel(), _stream_handle(dev)))
-            lam, lam_out = lam_out, lam
+        try:
+            nxt = recompute(len(seg_starts) - 1)
+            for j in reversed(range(len(seg_starts))):
+                n = min(k, steps - seg_starts[j])
+                slot, ready = nxt
+                if j > 0:
+                    nxt = recompute(j - 1)
+                main.wait_event(ready)
+                tc, tp = slots[slot]
+                job = AdjointJob()
+                job.n_sols, job.n_init, job.steps = Ns, Ni, n
+                job.k_half, job.gf_params, job.weights, job.T = (kh.data_ptr(), gf.data_ptr(), w.data_ptr(),
+                                                                 Tt.data_ptr())
+                job.traj_cells, job.traj_potential = tc.data_ptr(), tp.data_ptr()
+                job.lambda_in, job.lambda_out = lam.data_ptr(), lam_out.data_ptr()
+                job.kernel_grad_acc = acc.data_ptr()
+                job.grad_gf, job.grad_weights = g_gf.data_ptr(), g_w.data_ptr()
+                job.clip_grad = ctx.clip
+                job.cells_after = after[j].data_ptr()
+                _lib.check(lib.lgx_adjoint(handle, job, ws.data_ptr(), ws.numel(), _stream_handle(dev)))
+                if j > 1:
+                    read[slot] = main.record_event()
+                lam, lam_out = lam_out, lam
+        finally:
+            main.wait_stream(side)  # the side stream's buffers belong to this one
         g_k = torch.empty((Ns, m.K) + m.world, dtype=torch.float32, device=dev)
         _lib.check(lib.lgx_adjoint_kernel_grad(handle, Ns, Ni, acc.data_ptr(), g_k.data_ptr(), ws.data_ptr(),
                                                ws.numel(), _stream_handle(dev)))
         return lam, g_k.reshape(ctx.k_shape), g_gf, g_w, None, None, None, None, None, None
 
 
-def _segment(update_fn, cells, k_half, gf, w, Tt, n, traj, engine='auto'):
-    """n Euler steps from `cells` through lgx_run (no statistics needed)."""
-    m = update_fn.model_for(cells.shape[3:])
-    dev = cells.device
-    Ns, Ni = cells.shape[:2]
+def _segment_workspace(m, Ns, Ni, n, engine, dev):
+    """Workspace of :func:`_segment` for up to ``n`` steps."""
+    return workspace(_lib.load().lgx_run_workspace_bytes(m.plan.handle, Ns, Ni, n, _lib.ENGINES[engine]), dev)
+
+
+def _segment(m, cells, k_half, gf, w, Tt, n, final, ws, traj=None, engine='auto'):
+    """n Euler steps from `cells` into `final` through lgx_run (no statistics
+    needed); `traj`: buffers of at least n steps for the states and potentials."""
     lib = _lib.load()
-    final = torch.empty_like(cells)
     job = _lib.Rollout()
-    job.n_sols, job.n_init, job.steps = Ns, Ni, n
+    job.n_sols, job.n_init, job.steps = cells.shape[0], cells.shape[1], n
     kh = torch.view_as_real(k_half.contiguous())
     job.cells0, job.k_half, job.gf_params, job.weights, job.T = (cells.data_ptr(), kh.data_ptr(), gf.data_ptr(),
                                                                   w.data_ptr(), Tt.data_ptr())
     job.stats_R, job.stats_T = 1.0, 1.0
     job.final_cells = final.data_ptr()
-    tc = tp = None
-    if traj:
-        tc = torch.empty((n, Ns * Ni, m.C) + m.world, dtype=torch.float32, device=dev)
-        tp = torch.empty((n, Ns * Ni, m.K) + m.world, dtype=torch.float32, device=dev)
-        job.traj_cells, job.traj_potential = tc.data_ptr(), tp.data_ptr()
-    eng = _lib.ENGINES[engine]
-    ws = workspace(lib.lgx_run_workspace_bytes(m.plan.handle, Ns, Ni, n, eng), dev)
-    job.engine = eng
-    _lib.check(lib.lgx_run(m.plan.handle, job, ws.data_ptr(), ws.numel(), _stream_handle(dev)))
-    return (tc, tp) if traj else final
+    if traj is not None:
+        job.traj_cells, job.traj_potential = traj[0].data_ptr(), traj[1].data_ptr()
+    job.engine = _lib.ENGINES[engine]
+    _lib.check(lib.lgx_run(m.plan.handle, job, ws.data_ptr(), ws.numel(), _stream_handle(cells.device)))
+    return final
 
 
 def rollout(cells0, k_real, gf_params, weights, T, update_fn: UpdateFn, steps: int, checkpoint_every: int = 16,

@@ -38,10 +38,12 @@ def build_compute_stats_fn(world_params: Dict, render_params: Dict) -> ComputeSt
 
 
 def split_stats(packed: torch.Tensor, C: int) -> Dict[str, torch.Tensor]:
-    """Engine stats ``[..., C + 11]`` -> leniax's dict of arrays."""
-    out = {'channel_mass': packed[..., :C].contiguous()}
-    for i, k in enumerate(STAT_KEYS[1:]):
-        out[k] = packed[..., C + i].contiguous()
+    """Engine stats ``[..., C + 11]`` -> leniax's dict of arrays, contiguous
+    views of one transposed copy (a copy for each of the twelve was most of
+    what a rollout of a small batch spent outside the engine)."""
+    rows = packed.movedim(-1, 0).contiguous()
+    out = {'channel_mass': rows[0].unsqueeze(-1) if C == 1 else packed[..., :C].contiguous()}
+    out.update(zip(STAT_KEYS[1:], rows[C:].unbind(0)))
     return out
 
 
