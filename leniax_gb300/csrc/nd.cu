@@ -125,6 +125,14 @@ NdAxes make_axes(int D, int H, int W, void* ws) {
 // m-point spectrum of conj(c) wrapped around.  They are made once per call
 // and shared by all its launches; building them in every block of every pass
 // cost each block a sincospif per point, or a whole transform.
+// The twiddles of plain lines are rounded from double (an entry of tw_entry
+// carries the rounding of its argument as well); a block takes a slice of them.
+constexpr int kTableBlocks = 16;
+__device__ __forceinline__ float2 tw_rounded(int j, int m) {
+  double s, c;
+  sincospi(2.0 * (double)j / (double)m, &s, &c);
+  return make_float2((float)c, (float)-s);
+}
 struct TableArgs {
   float2* t[3];
   int n[3], m[3];
@@ -135,9 +143,10 @@ __global__ void __launch_bounds__(kNT) nd_tables_kernel(TableArgs a) {
   const int b = blockIdx.x, n = a.n[b], m = a.m[b];
   float2* out = a.t[b];
   if (m == n) {
-    for (int j = threadIdx.x; j < m; j += blockDim.x) out[j] = tw_entry(j, m);
+    for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < m; j += gridDim.y * blockDim.x) out[j] = tw_rounded(j, m);
     return;
   }
+  if (blockIdx.y > 0) return;
   float2 *tw = sm, *A = sm + m, *B = A + m;
   for (int j = threadIdx.x; j < m; j += blockDim.x) out[j] = tw[j] = tw_entry(j, m);
   for (int j = threadIdx.x; j < m; j += blockDim.x) {
@@ -167,7 +176,7 @@ cudaError_t launch_tables(const NdAxes& ax, int D, cudaStream_t st) {
     const cudaError_t e = nd_allow_smem((const void*)nd_tables_kernel);
     if (e != cudaSuccess) return e;
   }
-  nd_tables_kernel<<<naxes, kNT, smem, st>>>(a);
+  nd_tables_kernel<<<dim3(naxes, kTableBlocks), kNT, smem, st>>>(a);
   return cudaGetLastError();
 }
 
