@@ -503,9 +503,14 @@ StepLayout step_layout(const Model& m, int n_worlds) {
   const NdAxes ax = make_axes(m.D, m.H, m.W, nullptr);
   const size_t nw = (size_t)n_worlds;
   long field = 0;
-  int bpw = m.D;
-  if (!nd_plane_ok(t, ax)) bpw = nd_rows_epi_blocks(t, ax.x, (long)nw, &field);
-  else if (nd_plane_field_global(t, ax)) field = (long)m.D * ((m.H + 1) / 2) * m.W;
+  int bpw;
+  if (nd_plane_ok(t, ax)) {
+    bool global;
+    bpw = nd_plane_epi_blocks(t, ax, (long)nw, &global);
+    if (global) field = (long)m.D * ((m.H + 1) / 2) * m.W;
+  } else {
+    bpw = nd_rows_epi_blocks(t, ax.x, (long)nw, &field);
+  }
   StepLayout L;
   size_t off = 0;
   L.tables = off;

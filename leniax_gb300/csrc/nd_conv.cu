@@ -28,6 +28,7 @@ __device__ __forceinline__ void conv_tile_init(Tile& t, const ConvTile& g, float
   t.nld = g.nld;
 }
 
+// One channel of the tile a block (blockIdx.y): the channels share nothing.
 // forward: P[w, k] = IFFT_axis(FFT_axis(S[w, c_in(k)]) * K[sol, c_in(k), slot(k)])
 template <int KIND>
 __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_conv_kernel(NdTab t, ConvArgs a, ConvTile g, LineAxis ax) {
@@ -47,50 +48,48 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_conv_kernel(Nd
   a.S = after_wait(a.S);
   __syncthreads();
   const float2 zero = make_float2(0.f, 0.f);
-  for (int c = 0; c < t.C; ++c) {
-    int nk = 0, first = 0;
-    for (int k = t.K - 1; k >= 0; --k)
-      if (t.cin[k] == c) {
-        ++nk;
-        first = k;
-      }
-    if (nk == 0) continue;
-    const float2* __restrict__ S = a.S + ((long)w * t.C + c) * t.hcells + i0;
-    const float2* __restrict__ Kc = a.kh + sol * a.kh_sol_stride + (long)c * t.max_k * t.hcells + i0;
-    auto load = [=](int l, int i) { return l < lines ? __ldg(S + l + (long)i * I) : zero; };
-    auto store_to = [=](int k) {
-      float2* __restrict__ P = a.P + ((long)w * t.K + k) * t.hcells + i0;
-      return [=](int l, int i, float2 v) {
-        if (l < lines) P[l + (long)i * I] = v;
-      };
+  const int c = blockIdx.y;
+  int nk = 0, first = 0;
+  for (int k = t.K - 1; k >= 0; --k)
+    if (t.cin[k] == c) {
+      ++nk;
+      first = k;
+    }
+  if (nk == 0) return;
+  const float2* __restrict__ S = a.S + ((long)w * t.C + c) * t.hcells + i0;
+  const float2* __restrict__ Kc = a.kh + sol * a.kh_sol_stride + (long)c * t.max_k * t.hcells + i0;
+  auto load = [=](int l, int i) { return l < lines ? __ldg(S + l + (long)i * I) : zero; };
+  auto store_to = [=](int k) {
+    float2* __restrict__ P = a.P + ((long)w * t.K + k) * t.hcells + i0;
+    return [=](int l, int i, float2 v) {
+      if (l < lines) P[l + (long)i * I] = v;
     };
-    if (!BL && nk == 1) {
-      const float2* __restrict__ kk = Kc + (long)t.slot[first] * t.hcells;
-      line_head<false, true, WIDE>(ax, tw, tl, each_in(load));
-      line_center<false, true, WIDE>(ax, tw, tl, [=](int l, int j, int nb, auto& v) {
-        constexpr int R = (int)(sizeof(v) / sizeof(float2));
-        float2 s[R];
+  };
+  if (!BL && nk == 1) {
+    const float2* __restrict__ kk = Kc + (long)t.slot[first] * t.hcells;
+    line_head<false, true, WIDE>(ax, tw, tl, each_in(load));
+    line_center<false, true, WIDE>(ax, tw, tl, [=](int l, int j, int nb, auto& v) {
+      constexpr int R = (int)(sizeof(v) / sizeof(float2));
+      float2 s[R];
 #pragma unroll
-        for (int q = 0; q < R; ++q) s[q] = l < lines ? __ldg(kk + l + (long)(j + q * nb) * I) : zero;
+      for (int q = 0; q < R; ++q) s[q] = l < lines ? __ldg(kk + l + (long)(j + q * nb) * I) : zero;
 #pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = cmul(v[q], s[q]);
-        return true;
-      });
-      line_middle<true, true>(ax, tw, tl);
-      const auto store = store_to(first);
-      line_tail<true, true, WIDE>(ax, tw, tl, each_out(store));
-    } else {
-      line_fft<false, true, KIND>(ax, tw, tl, load, [=](int l, int i, float2 v) { Sc[i * sp + l] = v; });
-      __syncthreads();
-      for (int k = first; k < t.K; ++k) {
-        if (t.cin[k] != c) continue;
-        const float2* __restrict__ kk = Kc + (long)t.slot[k] * t.hcells;
-        line_fft<true, true, KIND>(
-            ax, tw, tl,
-            [=](int l, int i) { return l < lines ? cmul(Sc[i * sp + l], __ldg(kk + l + (long)i * I)) : zero; },
-            store_to(k));
-      }
-      __syncthreads();  // Sc is rewritten by the next channel
+      for (int q = 0; q < R; ++q) v[q] = cmul(v[q], s[q]);
+      return true;
+    });
+    line_middle<true, true>(ax, tw, tl);
+    const auto store = store_to(first);
+    line_tail<true, true, WIDE>(ax, tw, tl, each_out(store));
+  } else {
+    line_fft<false, true, KIND>(ax, tw, tl, load, [=](int l, int i, float2 v) { Sc[i * sp + l] = v; });
+    __syncthreads();
+    for (int k = first; k < t.K; ++k) {
+      if (t.cin[k] != c) continue;
+      const float2* __restrict__ kk = Kc + (long)t.slot[k] * t.hcells;
+      line_fft<true, true, KIND>(
+          ax, tw, tl,
+          [=](int l, int i) { return l < lines ? cmul(Sc[i * sp + l], __ldg(kk + l + (long)i * I)) : zero; },
+          store_to(k));
     }
   }
 }
@@ -120,74 +119,72 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_adj_conv_kerne
   a.gk = after_wait(a.gk);
   __syncthreads();
   const float2 zero = make_float2(0.f, 0.f);
-  for (int c = 0; c < t.C; ++c) {
-    int nk = 0, first = t.K;
-    for (int k = t.K - 1; k >= 0; --k)
-      if (t.cin[k] == c) {
-        ++nk;
-        first = k;
-      }
-    const float2* __restrict__ S = a.S + ((long)w * t.C + c) * t.hcells + i0;
-    const float2* __restrict__ Kc = a.kh + sol * a.kh_sol_stride + (long)c * t.max_k * t.hcells + i0;
-    float2* __restrict__ Q = a.Q + ((long)w * t.C + c) * t.hcells + i0;
-    auto store_q = [=](int l, int i, float2 v) {
-      if (l < lines) Q[l + (long)i * I] = v;
-    };
-    if (nk == 0) {
-      for (int i = threadIdx.x; i < lines * ax.n; i += blockDim.x) {
-        const int j = i / lines;
-        Q[i - j * lines + (long)j * I] = zero;
-      }
-      continue;
+  const int c = blockIdx.y;
+  int nk = 0, first = t.K;
+  for (int k = t.K - 1; k >= 0; --k)
+    if (t.cin[k] == c) {
+      ++nk;
+      first = k;
     }
-    line_fft<false, true, KIND>(
-        ax, tw, tl, [=](int l, int i) { return l < lines ? __ldg(S + l + (long)i * I) : zero; },
-        [=](int l, int i, float2 v) {
-          Sc[i * sp + l] = v;
-          if (BL || nk > 1) Qc[i * sp + l] = zero;
-        });
-    __syncthreads();
-    for (int k = first; k < t.K; ++k) {
-      if (t.cin[k] != c) continue;
-      const float2* __restrict__ A = a.A + ((long)w * t.K + k) * t.hcells + i0;
-      const float2* __restrict__ kk = Kc + (long)t.slot[k] * t.hcells;
-      float2* __restrict__ gk = a.gk + ((long)w * t.K + k) * t.hcells + i0;
-      auto load = [=](int l, int i) { return l < lines ? __ldg(A + l + (long)i * I) : zero; };
-      if (!BL && nk == 1) {
-        line_head<false, true, WIDE>(ax, tw, tl, each_in(load));
-        line_center<false, true, WIDE>(ax, tw, tl, [=](int l, int j, int nb, auto& v) {
-          constexpr int R = (int)(sizeof(v) / sizeof(float2));
-          if (l >= lines) return true;  // zeros in, zeros out
-          float2 s[R], o[R];
+  const float2* __restrict__ S = a.S + ((long)w * t.C + c) * t.hcells + i0;
+  const float2* __restrict__ Kc = a.kh + sol * a.kh_sol_stride + (long)c * t.max_k * t.hcells + i0;
+  float2* __restrict__ Q = a.Q + ((long)w * t.C + c) * t.hcells + i0;
+  auto store_q = [=](int l, int i, float2 v) {
+    if (l < lines) Q[l + (long)i * I] = v;
+  };
+  if (nk == 0) {
+    for (int i = threadIdx.x; i < lines * ax.n; i += blockDim.x) {
+      const int j = i / lines;
+      Q[i - j * lines + (long)j * I] = zero;
+    }
+    return;
+  }
+  line_fft<false, true, KIND>(
+      ax, tw, tl, [=](int l, int i) { return l < lines ? __ldg(S + l + (long)i * I) : zero; },
+      [=](int l, int i, float2 v) {
+        Sc[i * sp + l] = v;
+        if (BL || nk > 1) Qc[i * sp + l] = zero;
+      });
+  __syncthreads();
+  for (int k = first; k < t.K; ++k) {
+    if (t.cin[k] != c) continue;
+    const float2* __restrict__ A = a.A + ((long)w * t.K + k) * t.hcells + i0;
+    const float2* __restrict__ kk = Kc + (long)t.slot[k] * t.hcells;
+    float2* __restrict__ gk = a.gk + ((long)w * t.K + k) * t.hcells + i0;
+    auto load = [=](int l, int i) { return l < lines ? __ldg(A + l + (long)i * I) : zero; };
+    if (!BL && nk == 1) {
+      line_head<false, true, WIDE>(ax, tw, tl, each_in(load));
+      line_center<false, true, WIDE>(ax, tw, tl, [=](int l, int j, int nb, auto& v) {
+        constexpr int R = (int)(sizeof(v) / sizeof(float2));
+        if (l >= lines) return true;  // zeros in, zeros out
+        float2 s[R], o[R];
 #pragma unroll
-          for (int q = 0; q < R; ++q) {
-            s[q] = __ldg(kk + l + (long)(j + q * nb) * I);
-            o[q] = gk[l + (long)(j + q * nb) * I];
-          }
+        for (int q = 0; q < R; ++q) {
+          s[q] = __ldg(kk + l + (long)(j + q * nb) * I);
+          o[q] = gk[l + (long)(j + q * nb) * I];
+        }
 #pragma unroll
-          for (int q = 0; q < R; ++q) {
-            const int i = j + q * nb;
-            gk[l + (long)i * I] = cadd(o[q], cmulc(v[q], Sc[i * sp + l]));
-            v[q] = cmulc(v[q], s[q]);
-          }
-          return true;
-        });
-        line_middle<true, true>(ax, tw, tl);
-        line_tail<true, true, WIDE>(ax, tw, tl, each_out(store_q));
-      } else {
-        line_fft<false, true, KIND>(ax, tw, tl, load, [=](int l, int i, float2 v) {
-          if (l >= lines) return;
-          float2* gp = gk + l + (long)i * I;
-          *gp = cadd(*gp, cmulc(v, Sc[i * sp + l]));
-          Qc[i * sp + l] = cadd(Qc[i * sp + l], cmulc(v, __ldg(kk + l + (long)i * I)));
-        });
-      }
+        for (int q = 0; q < R; ++q) {
+          const int i = j + q * nb;
+          gk[l + (long)i * I] = cadd(o[q], cmulc(v[q], Sc[i * sp + l]));
+          v[q] = cmulc(v[q], s[q]);
+        }
+        return true;
+      });
+      line_middle<true, true>(ax, tw, tl);
+      line_tail<true, true, WIDE>(ax, tw, tl, each_out(store_q));
+    } else {
+      line_fft<false, true, KIND>(ax, tw, tl, load, [=](int l, int i, float2 v) {
+        if (l >= lines) return;
+        float2* gp = gk + l + (long)i * I;
+        *gp = cadd(*gp, cmulc(v, Sc[i * sp + l]));
+        Qc[i * sp + l] = cadd(Qc[i * sp + l], cmulc(v, __ldg(kk + l + (long)i * I)));
+      });
     }
-    __syncthreads();
-    if (BL || nk > 1) {
-      line_fft<true, true, KIND>(ax, tw, tl, [=](int l, int i) { return Qc[i * sp + l]; }, store_q);
-      __syncthreads();  // Sc and Qc are rewritten by the next channel
-    }
+  }
+  __syncthreads();
+  if (BL || nk > 1) {
+    line_fft<true, true, KIND>(ax, tw, tl, [=](int l, int i) { return Qc[i * sp + l]; }, store_q);
   }
 }
 
@@ -242,7 +239,7 @@ ConvTile conv_tile(const LineAxis& ax, long groups, long I) {
 
 cudaError_t nd_convolve(bool adjoint, const NdTab& t, const LineAxis& ax, long nw, const ConvArgs& a,
                         cudaStream_t st) {
-  const ConvTile g = conv_tile(ax, nw, t.hcells / ax.n);
+  const ConvTile g = conv_tile(ax, nw * t.C, t.hcells / ax.n);
   const bool bl = ax.m != ax.n;
   int per[kMaxChannels] = {0}, most = 0;
   for (int k = 0; k < t.K; ++k) most = std::max(most, ++per[t.cin[k]]);
@@ -255,7 +252,7 @@ cudaError_t nd_convolve(bool adjoint, const NdTab& t, const LineAxis& ax, long n
   });
   const cudaError_t e = nd_allow_smem((const void*)f);
   if (e != cudaSuccess) return e;
-  return launch_dependent(f, (unsigned)blocks, nd_threads(line_items(ax, g.nl)), smem, st, t, a, g, ax);
+  return launch_dependent(f, dim3((unsigned)blocks, (unsigned)t.C), nd_threads(line_items(ax, g.nl)), smem, st, t, a, g, ax);
 }
 
 cudaError_t nd_columns(bool inv, const NdTab& t, const LineAxis& y, long planes, float2* data, cudaStream_t st) {

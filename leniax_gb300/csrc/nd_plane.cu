@@ -218,34 +218,39 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_epi_kerne
     }
     epi_channel_mass(sh, 0, mo.m00);
   } else {
-    float2* F = g.field_smem ? p.keep + g.keep : reinterpret_cast<float2*>(a.F) + (long)blockIdx.x * C * g.pp * W;
-    for (int i = threadIdx.x; i < C * g.pp * W; i += blockDim.x) F[i] = make_float2(0.f, 0.f);
+    const EpiChannels ch = epi_channels(t, a, wt);
+    float2* F = g.field_smem ? p.keep + g.keep
+                             : reinterpret_cast<float2*>(a.F) + ((long)blockIdx.x * C + ch.lo) * g.pp * W;
+    for (int i = threadIdx.x; i < (ch.hi - ch.lo) * g.pp * W; i += blockDim.x) F[i] = make_float2(0.f, 0.f);
+    __syncthreads();
     for (int k = 0; k < K; ++k) {
+      if (!((ch.todo >> k) & 1ull)) continue;
+      const bool count = (ch.count >> k) & 1ull;
       const NdGrowth grow(t.gf[k], __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1));
       columns_inverse(p, g, ay, Wh, a.P + ((long)w * K + k) * t.hcells + z * hplane);
       as_rows(p.t, g);
       line_fft<true, false, false>(ax, p.twx, p.t, kept, [&](int l, int x, float2 v) {
         const RowPair& r = rp[l];
         const float2 u = make_float2(v.x * a.scale, v.y * a.scale);
-        store_pot(r, k, x, u);
+        if (count) store_pot(r, k, x, u);
         const float2 gr = make_float2(grow(u.x), grow(u.y));
-        for (int c = 0; c < C; ++c) {
+        for (int c = ch.lo; c < ch.hi; ++c) {
           const float wk = __ldg(wt + c * K + k);
           if (wk == 0.f) continue;
-          float2* f = F + ((long)c * g.pp + l) * W + x;
+          float2* f = F + ((long)(c - ch.lo) * g.pp + l) * W + x;
           *f = __ffma2_rn(gr, make_float2(wk, wk), *f);
         }
       });
       __syncthreads();  // the half plane is rewritten by the next kernel
     }
-    for (int c = 0; c < C; ++c) {
+    for (int c = ch.lo; c < ch.hi; ++c) {
       float wsum = 0.f;
       for (int k = 0; k < K; ++k) wsum += __ldg(wt + c * K + k);
       const float before = mo.m00;
       mo.m00 = 0.f;  // this channel's mass
       auto new_cells = [&](int l, int x) {
         const RowPair& r = rp[l];
-        float2 f = F[((long)c * g.pp + l) * W + x];
+        float2 f = F[((long)(c - ch.lo) * g.pp + l) * W + x];
         if (t.mean) f = make_float2(f.x / wsum, f.y / wsum);
         return update(r, c, x, load_state(r, c, x), f);
       };
@@ -261,8 +266,10 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_epi_kerne
       epi_channel_mass(sh, c, mo.m00);
       mo.m00 += before;
     }
+    for (int c = 0; c < C; ++c)
+      if (c < ch.lo || c >= ch.hi) epi_channel_mass(sh, c, 0.f);
   }
-  epi_finish(t, a, sh, w, z, mo, s0, s1, s2);
+  epi_finish(t, a, sh, w, z + blockIdx.y * a.tiles, mo, s0, s1, s2);
 }
 
 struct PlanePlan {
@@ -288,8 +295,8 @@ PlanePlan plane_plan(const NdTab& t, const NdAxes& ax) {
   p.smem = (size_t)(t.W + t.H + 2 * g.buf + g.keep) * sizeof(float2);
   return p;
 }
-size_t plane_field_bytes(const NdTab& t, const PlanePlan& p) {
-  return t.C == 1 && t.K == 1 ? 0 : (size_t)t.C * p.g.pp * t.W * sizeof(float2);
+size_t plane_field_bytes(const NdTab& t, const PlanePlan& p, bool split) {
+  return t.C == 1 && t.K == 1 ? 0 : (size_t)(split ? 1 : t.C) * p.g.pp * t.W * sizeof(float2);
 }
 
 }  // namespace
@@ -298,9 +305,11 @@ bool nd_plane_ok(const NdTab& t, const NdAxes& ax) {
   return t.D > 1 && (long)t.H * t.W <= kMaxPts && ax.x.m == t.W && ax.y.m == t.H && (t.H + 1) / 2 <= kMaxTileLines;
 }
 
-bool nd_plane_field_global(const NdTab& t, const NdAxes& ax) {
+int nd_plane_epi_blocks(const NdTab& t, const NdAxes& ax, long n_worlds, bool* field_global) {
   const PlanePlan p = plane_plan(t, ax);
-  return p.smem + plane_field_bytes(t, p) > (size_t)108 * 1024;
+  const bool split = epi_split(t, n_worlds * t.D);
+  if (field_global) *field_global = p.smem + plane_field_bytes(t, p, split) > (size_t)108 * 1024;
+  return t.D * (split ? t.C : 1);
 }
 
 cudaError_t nd_plane_forward(const NdTab& t, const NdAxes& ax, long planes, const float* src, float2* half,
@@ -340,15 +349,18 @@ cudaError_t nd_plane_inverse(const NdTab& t, const NdAxes& ax, long planes, cons
 cudaError_t nd_plane_epilogue(const NdTab& t, const NdAxes& ax, const EpiArgs& args, cudaStream_t st) {
   EpiArgs a = args;
   PlanePlan p = plane_plan(t, ax);
-  a.bpw = t.D;
-  p.g.field_smem = nd_plane_field_global(t, ax) ? 0 : 1;
-  const size_t smem = p.smem + (p.g.field_smem ? plane_field_bytes(t, p) : 0);
+  bool field_global;
+  a.tiles = t.D;
+  a.bpw = nd_plane_epi_blocks(t, ax, a.n_worlds, &field_global);
+  a.split = a.bpw > a.tiles ? 1 : 0;
+  p.g.field_smem = field_global ? 0 : 1;
+  const size_t smem = p.smem + (p.g.field_smem ? plane_field_bytes(t, p, a.split) : 0);
   const long blocks = (long)a.n_worlds * t.D;
   if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
   auto f = t.C == 1 && t.K == 1 ? nd_plane_epi_kernel<true> : nd_plane_epi_kernel<false>;
   const cudaError_t e = nd_allow_smem((const void*)f);
   if (e != cudaSuccess) return e;
-  return launch_dependent(f, (unsigned)blocks, p.threads, smem, st, t, a, p.g, ax.x, ax.y);
+  return launch_dependent(f, dim3((unsigned)blocks, a.split ? t.C : 1), p.threads, smem, st, t, a, p.g, ax.x, ax.y);
 }
 
 }  // namespace lgx

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
   tl.lp = g.pitch;
   tl.nl = g.nr;
   tl.nld = g.nrd;
-  const int w = blockIdx.x / a.bpw, b = blockIdx.x - w * a.bpw;
+  const int w = blockIdx.x / a.tiles, b = blockIdx.x - w * a.tiles;
   const int sol = w / a.n_init;
   const int W = t.W, Wh = t.Wh, C = t.C, K = t.K, zp = g.zp;
   load_line_twiddles(tw, ax);
@@ -271,34 +271,37 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
       store_spectra(0);
     }
   } else {
-    // [C][nr][W] pairs: fields of row0 and row1
+    const EpiChannels ch = epi_channels(t, a, wt);
+    // [channel][nr][W] pairs: fields of row0 and row1
     float2* F = g.field_smem ? Z + (long)g.nr * zp
-                             : reinterpret_cast<float2*>(a.F) + (long)(w * a.bpw + b) * C * g.nr * W;
-    for (int i = threadIdx.x; i < C * g.nr * W; i += blockDim.x) F[i] = make_float2(0.f, 0.f);
+                             : reinterpret_cast<float2*>(a.F) + ((long)(w * a.tiles + b) * C + ch.lo) * g.nr * W;
+    for (int i = threadIdx.x; i < (ch.hi - ch.lo) * g.nr * W; i += blockDim.x) F[i] = make_float2(0.f, 0.f);
     __syncthreads();
     for (int k = 0; k < K; ++k) {
+      if (!((ch.todo >> k) & 1ull)) continue;
+      const bool count = (ch.count >> k) & 1ull;
       const NdGrowth grow(t.gf[k], __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1));
       line_fft<true, false, KIND>(ax, tw, tl, load_rows(k), [&](int l, int x, float2 v) {
         const int rows = rp[l].rows;
         if (rows == 0) return;
         const float2 u = make_float2(v.x * a.scale, v.y * a.scale);
-        if (a.pot_out) {
+        if (count && a.pot_out) {
           float* p = a.pot_out + ((long)w * K + k) * t.cells + rp[l].cell + x;
           p[0] = u.x;
           if (rows > 1) p[W] = u.y;
         }
-        mo.count_pot(u, rows);
+        if (count) mo.count_pot(u, rows);
         const float2 gr = make_float2(grow(u.x), grow(u.y));
-        for (int c = 0; c < C; ++c) {
+        for (int c = ch.lo; c < ch.hi; ++c) {
           const float wk = __ldg(wt + c * K + k);
           if (wk == 0.f) continue;
-          float2* f = F + ((long)c * g.nr + l) * W + x;
+          float2* f = F + ((long)(c - ch.lo) * g.nr + l) * W + x;
           *f = __ffma2_rn(gr, make_float2(wk, wk), *f);
         }
       });
     }
     __syncthreads();
-    for (int c = 0; c < C; ++c) {
+    for (int c = ch.lo; c < ch.hi; ++c) {
       float wsum = 0.f;
       for (int k = 0; k < K; ++k) wsum += __ldg(wt + c * K + k);
       const float before = mo.m00;
@@ -306,7 +309,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
       auto new_cells = [&](int l, int x) {
         const RowPair& r = rp[l];
         if (r.rows == 0) return make_float2(0.f, 0.f);
-        float2 f = F[((long)c * g.nr + l) * W + x];
+        float2 f = F[((long)(c - ch.lo) * g.nr + l) * W + x];
         if (t.mean) f = make_float2(f.x / wsum, f.y / wsum);
         return update(r, c, x, load_state(r, c, x), f);
       };
@@ -321,23 +324,27 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
       epi_channel_mass(sh, c, mo.m00);
       mo.m00 += before;
     }
+    for (int c = 0; c < C; ++c)
+      if (c < ch.lo || c >= ch.hi) epi_channel_mass(sh, c, 0.f);
   }
-  epi_finish(t, a, sh, w, b, mo, s0, s1, s2);
+  epi_finish(t, a, sh, w, b + blockIdx.y * a.tiles, mo, s0, s1, s2);
 }
 
 struct EpiTile {
   RowTile rt;
-  int bpw;
-  bool field_smem;
+  int tiles;
+  bool split, field_smem;
   size_t smem;
 };
 EpiTile epi_tile(const NdTab& t, const LineAxis& x, long n_worlds) {
   EpiTile e;
   const int pp = (t.D * t.H + 1) / 2;
-  e.rt = row_tile(x, n_worlds * pp, pp);
-  e.bpw = (pp + e.rt.nr - 1) / e.rt.nr;
+  const long whole = row_tile(x, kFillBlocks * (long)pp, pp).nr;
+  e.split = epi_split(t, n_worlds * ((pp + whole - 1) / whole));
+  e.rt = row_tile(x, n_worlds * pp * (e.split ? t.C : 1), pp);
+  e.tiles = (pp + e.rt.nr - 1) / e.rt.nr;
   const size_t base = (size_t)(x.m + 2 * e.rt.buf + (long)e.rt.nr * e.rt.zp) * sizeof(float2);
-  const size_t field = t.C == 1 && t.K == 1 ? 0 : (size_t)t.C * e.rt.nr * t.W * sizeof(float2);
+  const size_t field = t.C == 1 && t.K == 1 ? 0 : (size_t)(e.split ? 1 : t.C) * e.rt.nr * t.W * sizeof(float2);
   // two blocks per SM keep the fields in shared memory; larger sets go through L2
   e.field_smem = base + field <= (size_t)108 * 1024;
   e.smem = base + (e.field_smem ? field : 0);
@@ -380,14 +387,16 @@ cudaError_t nd_rows_inverse(const LineAxis& x, long planes, int rows, const floa
 
 int nd_rows_epi_blocks(const NdTab& t, const LineAxis& x, long n_worlds, long* field_pairs) {
   const EpiTile e = epi_tile(t, x, n_worlds);
-  if (field_pairs) *field_pairs = e.field_smem ? 0 : (long)e.bpw * e.rt.nr * t.W;
-  return e.bpw;
+  if (field_pairs) *field_pairs = e.field_smem ? 0 : (long)e.tiles * e.rt.nr * t.W;
+  return e.tiles * (e.split ? t.C : 1);
 }
 
 cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& args, cudaStream_t st) {
   EpiArgs a = args;
   const EpiTile e = epi_tile(t, x, a.n_worlds);
-  a.bpw = e.bpw;
+  a.tiles = e.tiles;
+  a.split = e.split ? 1 : 0;
+  a.bpw = e.tiles * (e.split ? t.C : 1);
   RowsEpi g;
   g.pp = (t.D * t.H + 1) / 2;
   g.nr = e.rt.nr;
@@ -399,7 +408,7 @@ cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& a
   g.hd = make_fastdiv((unsigned)t.H);
   g.whd = make_fastdiv((unsigned)t.Wh);
   g.field_smem = e.field_smem ? 1 : 0;
-  const long blocks = (long)a.n_worlds * a.bpw;
+  const long blocks = (long)a.n_worlds * a.tiles;
   if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
   const bool single = t.C == 1 && t.K == 1;
   auto f = for_line_kind(x, [&](auto kind) {
@@ -407,7 +416,7 @@ cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& a
   });
   const cudaError_t err = nd_allow_smem((const void*)f);
   if (err != cudaSuccess) return err;
-  return launch_dependent(f, (unsigned)blocks, e.rt.threads, e.smem, st, t, a, g, x);
+  return launch_dependent(f, dim3((unsigned)blocks, e.split ? t.C : 1), e.rt.threads, e.smem, st, t, a, g, x);
 }
 
 }  // namespace lgx
