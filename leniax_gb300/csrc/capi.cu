@@ -200,6 +200,54 @@ NdLayout nd_layout(const Model& m, int n_sols, int n_init, int steps) {
   return L;
 }
 
+// 3D worlds of 32^3 and 64^3 so few that one CTA a world leaves most of the
+// chip idle: their default engine (LGX_ENGINE_CTA) runs them by N-D steps,
+// each step spread over all SMs.  A CTA round is as long for one world as for
+// one a SM; an N-D step grows with the worlds.  8-step rollouts on 152 SMs,
+// us, one CTA a world / N-D steps: 64^3, 1 world 3135 / 346, 16 3148 / 726,
+// 64 3229 / 2130, 128 3244 / 3827, 256 (two rounds) 6303 / 7197; 32^3, 1 world
+// 532 / 302, 16 522 / 327, 64 526 / 574, 256 915 / 1623.
+bool few_3d_worlds(const Model& m, long nw) {
+  if (!cta_supported(m) || !nd_supported(m)) return false;
+  const long sms = sm_count_now(), rounds = (nw + sms - 1) / sms;
+  return m.H == 64 ? 152 * nw <= 104 * sms * rounds : 152 * nw <= 48 * sms;
+}
+
+// The engine whose kernels lgx_run runs for a batch of nw worlds.
+int run_engine(const Model& m, int requested, long nw) {
+  const int e = select_engine(m, requested);
+  return requested == LGX_ENGINE_AUTO && e == LGX_ENGINE_CTA && few_3d_worlds(m, nw) ? LGX_ENGINE_ND : e;
+}
+
+size_t run_workspace(const Model& m, int n_sols, int n_init, int steps, int e) {
+  if (e == LGX_ENGINE_RESIDENT) return resident_ws(m, n_sols, n_init, steps);
+  if (e == LGX_ENGINE_STREAMED || e == LGX_ENGINE_PLAIN_STREAMED) return streamed_ws(m, n_sols, n_init, steps, true);
+  if (e == LGX_ENGINE_PLAIN) return plain_ws(m, n_sols, n_init, steps);
+  if (e == LGX_ENGINE_ND) return nd_layout(m, n_sols, n_init, steps).end;
+  if (e == LGX_ENGINE_CTA) return cta_layout(m, n_sols, n_init, steps).end;
+  return 0;
+}
+
+// The engine of one lgx_update step: a streamed step for 2D powers of two
+// (resident sizes included), one world per CTA for 3D batches that fill the
+// chip, else an N-D step.  `general`: the engine taken where the workspace has
+// no room for the N-D step's.  Other even squares run the mixed-radix streamed
+// step only for one or two planes; a step, us, streamed / N-D: 100^2, 1 plane
+// 40 / 44, 64 86 / 39, 8 worlds of 3 channels x 9 kernels 98 / 73, 64 of them
+// 342 / 139; 360^2, 1 plane 61 / 73, 8 96 / 61, one world of 3 x 9 156 / 100;
+// 48^2, 1 plane 41 / 37, one world of 3 x 9 89 / 67.
+int update_engine(const Model& m, long n, bool general = false) {
+  if (streamed_supported(m))
+    return !general && generic_size(m.H) && n * m.C > 2 && nd_supported(m) ? LGX_ENGINE_ND : LGX_ENGINE_STREAMED;
+  if (cta_supported(m)) return !general && few_3d_worlds(m, n) ? LGX_ENGINE_ND : LGX_ENGINE_CTA;
+  return nd_supported(m) ? LGX_ENGINE_ND : -1;
+}
+
+size_t update_workspace(const Model& m, int n, int e) {
+  if (e == LGX_ENGINE_STREAMED) return streamed_ws(m, 1, n, 1, false);
+  return e < 0 ? 0 : run_workspace(m, 1, n, 1, e);
+}
+
 struct StreamedBufs {
   float2 *spec, *prod, *kp;
   float* partial;
@@ -303,14 +351,7 @@ int lgx_select_engine(const lgx_plan* plan, int n_sols, int n_init, int requeste
 
 size_t lgx_run_workspace_bytes(const lgx_plan* plan, int n_sols, int n_init, int steps, int engine) {
   if (!plan || n_sols < 1 || n_init < 1 || steps < 0) return 0;
-  const int e = select_engine(plan->m, engine);
-  if (e == LGX_ENGINE_RESIDENT) return resident_ws(plan->m, n_sols, n_init, steps);
-  if (e == LGX_ENGINE_STREAMED || e == LGX_ENGINE_PLAIN_STREAMED)
-    return streamed_ws(plan->m, n_sols, n_init, steps, true);
-  if (e == LGX_ENGINE_PLAIN) return plain_ws(plan->m, n_sols, n_init, steps);
-  if (e == LGX_ENGINE_ND) return nd_layout(plan->m, n_sols, n_init, steps).end;
-  if (e == LGX_ENGINE_CTA) return cta_layout(plan->m, n_sols, n_init, steps).end;
-  return 0;
+  return run_workspace(plan->m, n_sols, n_init, steps, run_engine(plan->m, engine, (long)n_sols * n_init));
 }
 
 int lgx_run(const lgx_plan* plan, const lgx_rollout* j, void* ws, size_t ws_bytes, void* stream) {
@@ -321,11 +362,13 @@ int lgx_run(const lgx_plan* plan, const lgx_rollout* j, void* ws, size_t ws_byte
   if (!j->cells0 || !j->k_half || !j->gf_params || !j->weights || !j->T)
     return fail(LGX_ERR_INVALID, "lgx_run: null input tensor");
   if (!(j->stats_R > 0.f) || !(j->stats_T > 0.f)) return fail(LGX_ERR_INVALID, "lgx_run: stats_R and stats_T must be > 0");
-  const int e = select_engine(m, j->engine);
+  int e = run_engine(m, j->engine, (long)j->n_sols * j->n_init);
   if (e < 0) return fail(LGX_ERR_UNSUPPORTED, "lgx_run: no engine for this model (engine=%d, C=%d, K=%d, size=%d)",
                          j->engine, m.C, m.K, m.H);
-  const size_t need = lgx_run_workspace_bytes(plan, j->n_sols, j->n_init, j->steps, e);
-  if (!ws || ws_bytes < need) return fail(LGX_ERR_WORKSPACE, "lgx_run: workspace %zu < %zu bytes", ws_bytes, need);
+  const size_t need = run_workspace(m, j->n_sols, j->n_init, j->steps, e);
+  const int other = select_engine(m, j->engine);  // a workspace that holds this engine's layout alone is taken too
+  if (ws && ws_bytes < need && other != e && ws_bytes >= run_workspace(m, j->n_sols, j->n_init, j->steps, other)) e = other;
+  else if (!ws || ws_bytes < need) return fail(LGX_ERR_WORKSPACE, "lgx_run: workspace %zu < %zu bytes", ws_bytes, need);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int nw = j->n_sols * j->n_init;
   const size_t plane = (size_t)m.C * m.cells;
@@ -621,12 +664,7 @@ int lgx_run(const lgx_plan* plan, const lgx_rollout* j, void* ws, size_t ws_byte
 size_t lgx_update_workspace_bytes(const lgx_plan* plan, int n) {
   if (!plan || n < 1) return 0;
   const Model& m = plan->m;
-  // lgx_update runs one streamed step for every 2D model (resident sizes
-  // included) and a one-step one-world-per-CTA rollout for 3D models
-  if (streamed_supported(m)) return streamed_ws(m, 1, n, 1, false);
-  if (cta_supported(m)) return cta_layout(m, 1, n, 1).end;
-  if (nd_supported(m)) return nd_layout(m, 1, n, 1).end;
-  return 0;
+  return update_workspace(m, n, update_engine(m, n));
 }
 
 int lgx_update(const lgx_plan* plan, int n, const float* state, const float* k_half, const float* gf_params,
@@ -637,12 +675,15 @@ int lgx_update(const lgx_plan* plan, int n, const float* state, const float* k_h
   if (n < 1) return fail(LGX_ERR_INVALID, "lgx_update: n must be >= 1");
   if (!state || !k_half || !gf_params || !weights || !dt || !state_out)
     return fail(LGX_ERR_INVALID, "lgx_update: null tensor");
-  const size_t need = lgx_update_workspace_bytes(plan, n);
+  int e = update_engine(m, n);
+  const size_t need = update_workspace(m, n, e);
   if (need == 0) return fail(LGX_ERR_UNSUPPORTED, "lgx_update: no engine for this model");
-  if (!ws || ws_bytes < need) return fail(LGX_ERR_WORKSPACE, "lgx_update: workspace %zu < %zu bytes", ws_bytes, need);
+  const int other = update_engine(m, n, true);  // a workspace that holds this engine's layout alone is taken too
+  if (ws && ws_bytes < need && other != e && ws_bytes >= update_workspace(m, n, other)) e = other;
+  else if (!ws || ws_bytes < need) return fail(LGX_ERR_WORKSPACE, "lgx_update: workspace %zu < %zu bytes", ws_bytes, need);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t ce;
-  if (cta_supported(m)) {
+  if (e == LGX_ENGINE_CTA) {
     // 3D: one step of the plane-fused item, field and potential as its step-0 trajectory
     const CtaLayout L = cta_layout(m, 1, n, 1);
     char* base = static_cast<char*>(ws);
@@ -677,8 +718,10 @@ int lgx_update(const lgx_plan* plan, int n, const float* state, const float* k_h
     g_err.clear();
     return LGX_OK;
   }
-  if (!streamed_supported(m) && nd_supported(m)) {
+  if (e == LGX_ENGINE_ND) {
     // one step of the general N-D engine, scalar or per-world dt
+    if (streamed_supported(m) && (reinterpret_cast<uintptr_t>(state) & 15u) != 0)  // as the streamed step asks
+      return cuda_fail(cudaErrorMisalignedAddress, "update step");
     const NdLayout L = nd_layout(m, 1, n, 1);
     char* base = static_cast<char*>(ws);
     int* shift = reinterpret_cast<int*>(base + L.shift);
