@@ -101,14 +101,36 @@ __device__ __forceinline__ float step_dt(const NdTab& t, const EpiArgs& a, int w
 static __device__ __noinline__ float growth_any(int id, float u, float m, float s) { return growth_fn(id, u, m, s); }
 struct NdGrowth {
   GrowthP p;
+  // the exponent's coefficient log2(e) / (2 s^2) as an unevaluated sum c + dc:
+  // rounded to one float its error is the same in every cell of a world, and a
+  // world's growth shows it where cells' roundings average out
+  float c, dc;
   __device__ __forceinline__ NdGrowth(int id, float m, float s) {
     p.id = id;
     p.m = m;
     p.s = s;
-    p.a = 0.84932180028801904272f / s;  // sqrt(log2(e) / 2) / s
+    const float q = s * s, dq = fmaf(s, s, -q);  // s^2 = q + dq
+    c = kC / q;
+    dc = (fmaf(-c, q, kC) + (kDc - c * dq)) / q;
+  }
+  static constexpr double kLog2E2 = 0.72134752044448170368;  // log2(e) / 2
+  static constexpr float kC = (float)kLog2E2, kDc = (float)(kLog2E2 - (double)kC);
+  // the gaussian's exponential at both cells
+  __device__ __forceinline__ float2 gauss(float2 u) const {
+    const float2 d = __fadd2_rn(u, make_float2(-p.m, -p.m));
+    const float2 d2 = __fmul2_rn(d, d);
+    const float2 x = __ffma2_rn(d2, make_float2(-c, -c), __fmul2_rn(d2, make_float2(-dc, -dc)));
+    return make_float2(fast_exp2(x.x), fast_exp2(x.y));
+  }
+  // weighted growth of a pair: w (2 e - 1)
+  __device__ __forceinline__ float2 gauss_weighted(float2 u, float w) const {
+    return __ffma2_rn(make_float2(2.f * w, 2.f * w), gauss(u), make_float2(-w, -w));
   }
   __device__ __forceinline__ float operator()(float u) const {
-    if (p.id == LGX_GF_GAUSSIAN) return growth_cell<GF_FAST_GAUSSIAN>(p, u);
+    if (p.id == LGX_GF_GAUSSIAN) {
+      const float d = u - p.m, d2 = d * d;
+      return fmaf(2.f, fast_exp2(fmaf(d2, -c, d2 * -dc)), -1.f);
+    }
     return growth_any(p.id, u, p.m, p.s);
   }
 };
@@ -256,7 +278,7 @@ __device__ __forceinline__ void epi_pairs(const NdTab& t, const EpiArgs& a, cons
       const float2 s = make_float2(__ldg(a.state + off), two ? __ldg(a.state + off + W) : 0.f);
       const float2 u = __fmul2_rn(z[x], make_float2(a.scale, a.scale));
       float2 f;
-      if (GAUSS) f = weighted_growth2<GF_FAST_GAUSSIAN>(grow.p, u, wf);
+      if (GAUSS) f = grow.gauss_weighted(u, wf);
       else f = make_float2(grow(u.x) * wf, grow(u.y) * wf);
       if (!two) f.y = 0.f;
       float2 n;
