@@ -128,13 +128,21 @@ struct RowTile {
   int nr, pitch, zp, threads;
   long buf;
 };
-RowTile row_tile(const LineAxis& x, long pairs, long group_pairs) {
+RowTile row_tile(const LineAxis& x, long pairs, long group_pairs, bool three = false) {
   RowTile r;
+  // `three`: no more lines than leave room for three blocks an SM, as many as
+  // the registers allow (the plain epilogue of one kernel; tiles of several
+  // kernels and of wide lines measured slower when cut: 8 worlds of 360 x 480,
+  // 3 x 15 kernels 4169 -> 5438 us).  12-step rollouts, us, larger tiles ->
+  // these: 32 worlds of 128 x 512 771 -> 580, 512 of 80^2 782 -> 708, 128 of
+  // 144^2 819 -> 792; 100^2 and 250^2 as before.
+  const long pts = 74 * 1024L / (long)sizeof(float2) - x.m;
+  const long by_smem = three ? std::max(1L, pts / (2 * line_pitch(false, x, 1) + (x.n | 1))) : kMaxTileLines;
   const long fill = (pairs + kFillBlocks - 1) / kFillBlocks;
   // one butterfly per thread at most twice over
   const long by_items = std::max(1L, 2L * kNdThreads * std::min(x.r[0], std::max(x.r[x.stages - 1], 2)) / x.m);
   const long cap = std::max(1L, std::min<long>(std::min<long>(kMaxTileLines, by_items), kMaxPts / x.m));
-  const long want = std::max(1L, std::min(std::min(cap, fill), group_pairs));
+  const long want = std::max(1L, std::min(std::min(cap, by_smem), std::min(fill, group_pairs)));
   const long tiles = (group_pairs + want - 1) / want;
   r.nr = (int)((group_pairs + tiles - 1) / tiles);  // even tiles over the group
   r.pitch = line_pitch(false, x, r.nr);
@@ -341,7 +349,7 @@ EpiTile epi_tile(const NdTab& t, const LineAxis& x, long n_worlds) {
   const int pp = (t.D * t.H + 1) / 2;
   const long whole = row_tile(x, kFillBlocks * (long)pp, pp).nr;
   e.split = epi_split(t, n_worlds * ((pp + whole - 1) / whole));
-  e.rt = row_tile(x, n_worlds * pp * (e.split ? t.C : 1), pp);
+  e.rt = row_tile(x, n_worlds * pp * (e.split ? t.C : 1), pp, t.C == 1 && t.K == 1 && !x.wide);
   e.tiles = (pp + e.rt.nr - 1) / e.rt.nr;
   const size_t base = (size_t)(x.m + 2 * e.rt.buf + (long)e.rt.nr * e.rt.zp) * sizeof(float2);
   const size_t field = t.C == 1 && t.K == 1 ? 0 : (size_t)(e.split ? 1 : t.C) * e.rt.nr * t.W * sizeof(float2);
