@@ -53,6 +53,9 @@ struct Big3D {
   static constexpr int PITCH = N + G;
   static constexpr int BUF = (N / 2) * PITCH, CSCR = (N / 2) * GE::SCR;
   static constexpr int XS = N * HW;               // one half-spectrum plane, staged per slice (phase C)
+  static constexpr int SP = 2 * N + 4;            // pitch (floats) of the row pairs of a staged state plane:
+                                                  // a warp's groups read distinct banks
+  static_assert((N / 2) * SP <= 2 * XS && (N / 2) * SP <= 2 * CSCR, "a state plane fits either staging area");
   static constexpr int XSOFF = SL * (BUF + CSCR);
   static constexpr int PLANES = XSOFF + SL * XS;
   static constexpr int ZSCR = (512 / LG) * GZ::SCR;
@@ -60,7 +63,7 @@ struct Big3D {
   static_assert(NT % 32 == 0 && 512 % NT == 0 && N % SL == 0, "plane slices");
 };
 
-constexpr int kBigBars = 8;  // mbarriers after the reduction area (one per plane slice)
+constexpr int kBigBars = 16;  // mbarriers after the reduction area (two per plane slice)
 
 template <int N, int LG>
 constexpr size_t big3d_smem() {
@@ -280,8 +283,9 @@ __device__ __noinline__ void big2d_item(const BigArgs& a, int world, const float
 //      column inverse (DC and Nyquist columns re-packed as DC + i Nyquist),
 //      row inverse -> potential, growth, update, moments, and the run_scan
 //      trajectories when asked.
-// The next state plane (A, C) and the z pass's next round of lines (B) are
-// prefetched into L2 with bulk prefetches.
+// State planes are staged too (A: one ahead; C: during the row inverse, the new
+// states leaving from the same buffer).  The next state plane (C) and the z
+// pass's next round of lines (B) are prefetched into L2 with bulk prefetches.
 template <int N, int LG, int GF>
 __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float2* tw4, const float2* twz,
                                         float2* work) {
@@ -303,7 +307,11 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
   int* shv = reinterpret_cast<int*>(red + 16 * 16);
   uint64_t* xbar = reinterpret_cast<uint64_t*>(red + kBigRed) + sub;  // this slice's plane copies
   float2* xs = work + B3::XSOFF + sub * B3::XS;                       // this slice's staged plane
-  static_assert(SL <= kBigBars, "one mbarrier per slice");
+  static_assert(2 * SL <= kBigBars, "two mbarriers per slice");
+  uint64_t* sbar = xbar + SL;                                         // its state plane copies (phase C)
+  float* sxs = reinterpret_cast<float*>(xs);                          // staged state plane, phase A
+  float* scs = reinterpret_cast<float*>(buf + B3::BUF);               // ... phase C: the column pass' scratch
+  constexpr int SP = B3::SP;
   float2* X = a.scratch + (size_t)blockIdx.x * a.scratch_per_cta;
   const int sol = world / a.n_init;
   const float2* kp = a.kp + (size_t)sol * N * PLANE;  // [N][N][HW], scaled by 1/N^3
@@ -318,9 +326,29 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
   if (threadIdx.x == 0) shv[0] = shv[1] = shv[2] = 0;
   if (tid == 0) {
     mbar_init(xbar, 1);
+    mbar_init(sbar, 1);
     fence_proxy_async();
   }
-  unsigned xph = 0;  // phase parity of this slice's next plane copy
+  unsigned xph = 0, sph = 0;  // phase parities of this slice's next copies
+  // State planes move by bulk copies of row pairs where their addresses allow
+  // (torch allocations do): a group's own loads and stores, 16 bytes of a row
+  // each, cost a warp a tag lookup for every one of its eight rows.  152 worlds
+  // of 64^3, 8 steps: 3247 -> 2706 us; 1024 of 32^3 2848 -> 2504.
+  const bool staged = ((reinterpret_cast<uintptr_t>(c0) | reinterpret_cast<uintptr_t>(st)) & 15u) == 0;
+  auto landed = [&](uint64_t* bar, unsigned& phase) {
+    if (!mbar_wait(bar, phase)) {  // the copy never landed: record it, give it a bounded second wait
+      if (tid == 0 && a.status) atomicExch(a.status, kStatusCopyTimeout);
+      mbar_wait(bar, phase);
+    }
+    phase ^= 1u;
+  };
+  // the slice's first warp copies state plane z into dst
+  auto stage_state = [&](float* dst, const float* src, int z, uint64_t* bar) {
+    fence_proxy_async();
+    if (tid == 0) mbar_arrive_expect_tx(bar, (unsigned)(N * N * sizeof(float)));
+    __syncwarp();
+    if (tid < N / 2) bulk_load(dst + tid * SP, src + ((size_t)z * N + 2 * tid) * N, 2 * N * sizeof(float), bar);
+  };
   // bulk copy of spectrum plane z into the slice's staging buffer
   auto stage_plane = [&](int z) {
     mbar_arrive_expect_tx(xbar, (unsigned)(PLANE * sizeof(float2)));
@@ -330,15 +358,18 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
   for (int step = 0; step < a.steps; ++step) {
     const float* src = step == 0 ? c0 : st;
     // ---------------------------------------------------------- A. planes forward
+    if (staged && tid < 32) stage_state(sxs, src, sub, xbar);
     for (int zb = 0; zb < N; zb += SL) {
       const int z = zb + sub;
-      if (tid == 0 && z + SL < N) prefetch_l2(src + (size_t)(z + SL) * N * N, N * N * sizeof(float));
       {
-        const float* pl = src + (size_t)z * N * N;
+        const float* pl = src + ((size_t)z * N + 2 * grp) * N;  // rows 2 grp, 2 grp + 1
+        if (staged) {
+          landed(xbar, xph);
+          pl = sxs + grp * SP;
+        }
         float2 v[P];
 #pragma unroll
-        for (int n2 = 0; n2 < P; ++n2)
-          v[n2] = make_float2(pl[(2 * grp) * N + t + G * n2], pl[(2 * grp + 1) * N + t + G * n2]);
+        for (int n2 = 0; n2 < P; ++n2) v[n2] = make_float2(pl[t + G * n2], pl[N + t + G * n2]);
         float2 u[Q][G];
         fft_standard<GE, false, false>(v, u, rowbuf, tw_std, t, gmask);
 #pragma unroll
@@ -347,6 +378,7 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
           for (int k1 = 0; k1 < G; ++k1) rowbuf[t + G * q + P * k1] = u[q][k1];
       }
       named_bar(bar_id, NT);
+      if (staged && tid < 32 && z + SL < N) stage_state(sxs, src, z + SL, xbar);  // the slice is done with sxs
       {
         float2 v[Q][G];
 #pragma unroll
@@ -450,12 +482,8 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
     const int sz = shv[0], sy = shv[1], sx = shv[2];
     for (int zb = 0; zb < N; zb += SL) {
       const int z = zb + sub;
-      if (tid == 0 && z + SL < N) prefetch_l2(src + (size_t)(z + SL) * N * N, N * N * sizeof(float));
-      if (!mbar_wait(xbar, xph)) {  // the plane never landed: record it, give it a bounded second wait
-        if (tid == 0 && a.status) atomicExch(a.status, kStatusCopyTimeout);
-        mbar_wait(xbar, xph);
-      }
-      xph ^= 1u;
+      if (staged && tid == 0 && z + SL < N) prefetch_l2(src + (size_t)(z + SL) * N * N, N * N * sizeof(float));
+      landed(xbar, xph);
       {
         const float2* xz = xs;
         float2 w[P];
@@ -468,6 +496,10 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
             const float2 a0 = xz[ky * HW], an = xz[ky * HW + N / 2];
             w[k1] = make_float2(a0.x - an.y, a0.y + an.x);  // DC + i Nyquist
           }
+        }
+        if (staged) {  // the last plane's new states have left the column scratch
+          if (tid < 32) bulk_wait_read_all();
+          named_bar(bar_id, NT);
         }
         float2 u[Q][G];
         fft_standard<GE, true, true>(w, u, cs, tw_std, t, gmask);
@@ -484,6 +516,7 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
         fence_proxy_async();
         stage_plane(z + SL);
       }
+      if (staged && tid < 32) stage_state(scs, src, z, sbar);  // lands during the row inverse
       {
         const int r = grp;
         float2 v[Q][G];
@@ -496,6 +529,10 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
         const float cyb = (float)(((2 * r + 1 - sy) & (N - 1)) - N / 2);
         const float* sra = src + ((size_t)z * N + 2 * r) * N;
         float* dsa = st + ((size_t)z * N + 2 * r) * N;
+        if (staged) {
+          landed(sbar, sph);
+          sra = dsa = scs + grp * SP;
+        }
         float Sa = 0.f, Sb = 0.f, Ga = 0.f, Gb = 0.f;
 #pragma unroll
         for (int k1 = 0; k1 < P; ++k1) {
@@ -547,12 +584,21 @@ __device__ __noinline__ void big3d_item(const BigArgs& a, int world, const float
         acc[RAW_GX + 1] += cya * Ga + cyb * Gb;
         acc[RAW_MX2 + 1] += cya * cya * Sa + cyb * cyb * Sb;
       }
+      if (staged) fence_proxy_async();  // the new states in scs, before they leave
       named_bar(bar_id, NT);
+      if (staged && tid < 32) {
+        if (tid < N / 2) bulk_store(st + ((size_t)z * N + 2 * tid) * N, scs + tid * SP, 2 * N * sizeof(float));
+        bulk_commit();
+      }
     }
+    if (staged && tid < 32) bulk_wait_all();  // the next step's copies read them
     big_finish_step(a, world, step, 3, sizes, acc, border, red, shv);
   }
   __syncthreads();
-  if (tid == 0) mbar_inval(xbar);  // the area holds other items' data next
+  if (tid == 0) {  // the area holds other items' data next
+    mbar_inval(xbar);
+    mbar_inval(sbar);
+  }
 }
 
 template <int N, int G, int GF>

@@ -204,13 +204,13 @@ NdLayout nd_layout(const Model& m, int n_sols, int n_init, int steps) {
 // chip idle: their default engine (LGX_ENGINE_CTA) runs them by N-D steps,
 // each step spread over all SMs.  A CTA round is as long for one world as for
 // one a SM; an N-D step grows with the worlds.  8-step rollouts on 152 SMs,
-// us, one CTA a world / N-D steps: 64^3, 1 world 3135 / 346, 16 3148 / 726,
-// 64 3229 / 2130, 128 3244 / 3827, 256 (two rounds) 6303 / 7197; 32^3, 1 world
-// 532 / 302, 16 522 / 327, 64 526 / 574, 256 915 / 1623.
+// us, one CTA a world / N-D steps: 64^3, 64 worlds 2680 / 2140, 128 2696 /
+// 3853, 256 (two rounds) 5179 / 7233, and 343 for one world, 730 for 16; 32^3,
+// 64 worlds 474 / 571, 256 822 / 1628, and 300 for one world, 325 for 16.
 bool few_3d_worlds(const Model& m, long nw) {
   if (!cta_supported(m) || !nd_supported(m)) return false;
   const long sms = sm_count_now(), rounds = (nw + sms - 1) / sms;
-  return m.H == 64 ? 152 * nw <= 104 * sms * rounds : 152 * nw <= 48 * sms;
+  return m.H == 64 ? 152 * nw <= 84 * sms * rounds : 152 * nw <= 40 * sms;
 }
 
 // The engine whose kernels lgx_run runs for a batch of nw worlds.

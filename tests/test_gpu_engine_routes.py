@@ -28,7 +28,7 @@ def _model(cuda, world, C=1, per=1, R=5.0):
     return kp, K, mp, helpers.build_update_fn(K.shape, mp)
 
 
-@pytest.mark.parametrize('side,n', [(32, 1), (32, 48), (32, 49), (64, 1), (64, 104), (64, 105), (64, 153)])
+@pytest.mark.parametrize('side,n', [(32, 1), (32, 40), (32, 41), (64, 1), (64, 84), (64, 85), (64, 153)])
 def test_3d_batches_match_both_engines(cuda, side, n):
     _, K, mp, upd = _model(cuda, [side] * 3)
     g = torch.Generator(device='cpu').manual_seed(side + n)
@@ -46,7 +46,25 @@ def test_3d_batches_match_both_engines(cuda, side, n):
         torch.testing.assert_close(out['auto'][0]['mass'], out[other][0]['mass'], rtol=1e-5, atol=0)
 
 
-@pytest.mark.parametrize('side,n', [(32, 1), (32, 49), (64, 2)])
+@pytest.mark.parametrize('side', [32, 64])
+def test_3d_states_off_the_16_byte_grid_match_those_on_it(cuda, side):
+    # one world per CTA: state planes by bulk copies where their addresses
+    # allow, by the lanes' own loads elsewhere; the arithmetic is the same
+    _, K, mp, upd = _model(cuda, [side] * 3)
+    g = torch.Generator(device='cpu').manual_seed(side)
+    flat = torch.rand(2 * side**3 + 1, generator=g).to(cuda)
+    on = flat[1:].clone().view(1, 2, 1, side, side, side)
+    off = flat[1:].view(1, 2, 1, side, side, side)
+    assert on.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 4
+    stats_fn = statistics.ComputeStatsFn([side] * 3, 5.0, 10.0)
+    a, b = (runner.run_scan_mem_optimized(None, c, K[None], mp.get_gf_params(cuda)[None],
+                                          mp.get_kernels_weight_per_channel(cuda)[None], torch.tensor([10.0]), 3, 5.0,
+                                          upd, stats_fn, engine='cta') for c in (on, off))
+    assert torch.equal(a[1], b[1])
+    assert all(torch.equal(a[0][k], b[0][k]) for k in a[0])
+
+
+@pytest.mark.parametrize('side,n', [(32, 1), (32, 41), (64, 2)])
 @pytest.mark.parametrize('per_world', [False, True])
 def test_3d_update_matches_the_oracle(cuda, side, n, per_world):
     kp, K, mp, upd = _model(cuda, [side] * 3)
