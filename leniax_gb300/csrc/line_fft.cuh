@@ -568,9 +568,11 @@ __device__ __forceinline__ void line_fft(const LineAxis& ax, const float2* tw, T
   }
 }
 
-// The axis' twiddles into shared memory (m entries), without a barrier.
-__device__ __forceinline__ void load_line_twiddles(float2* tw, const LineAxis& ax) {
-  for (int i = threadIdx.x; i < ax.m; i += blockDim.x) tw[i] = __ldg(ax.tw + i);
+// An axis' twiddles into shared memory (m entries), without a barrier.  The
+// table is a parameter of its own: a kernel that writes to its LineAxis, whose
+// radices are indexed, keeps all of it in local memory.
+__device__ __forceinline__ void load_line_twiddles(float2* tw, const float2* table, int m) {
+  for (int i = threadIdx.x; i < m; i += blockDim.x) tw[i] = __ldg(table + i);
 }
 
 }  // namespace lgx

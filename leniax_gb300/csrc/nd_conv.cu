@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_conv_kernel(Nd
   const int lines = (int)min((long)g.nl, g.I - i0);
   const int sol = w / a.n_init, sp = g.sp;
   const int I = (int)g.I;
-  load_line_twiddles(tw, ax);
+  load_line_twiddles(tw, ax.tw, ax.m);
   depend_wait();
   a.S = after_wait(a.S);
   __syncthreads();
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_adj_conv_kerne
   const int lines = (int)min((long)g.nl, g.I - i0);
   const int sol = w / a.n_init, sp = g.sp;
   const int I = (int)g.I;
-  load_line_twiddles(tw, ax);
+  load_line_twiddles(tw, ax.tw, ax.m);
   depend_wait();
   a.S = after_wait(a.S);
   a.A = after_wait(a.A);
@@ -205,8 +205,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_columns_kernel
   const int I = (int)a.g.I;
   depend_wait();
   a.data = after_wait(a.data);
-  ax.tw = after_wait(ax.tw);
-  load_line_twiddles(tw, ax);
+  load_line_twiddles(tw, after_wait(ax.tw), ax.m);
   __syncthreads();
   float2* d = a.data + plane * a.g.I * ax.n + i0;
   line_fft<INV, true, KIND>(

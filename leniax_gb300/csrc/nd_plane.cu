@@ -25,15 +25,15 @@ struct PlaneTile {
 };
 
 __device__ __forceinline__ PlaneTile plane_init(const PlaneGeo& g, const LineAxis& ax, const LineAxis& ay,
-                                                float2* sm) {
+                                                const float2* tabx, const float2* taby, float2* sm) {
   PlaneTile p;
   p.twx = sm;
   p.twy = sm + ax.m;
   p.t.b[0] = p.twy + ay.m;
   p.t.b[1] = p.t.b[0] + g.buf;
   p.keep = p.t.b[1] + g.buf;
-  load_line_twiddles(p.twx, ax);
-  load_line_twiddles(p.twy, ay);
+  load_line_twiddles(p.twx, tabx, ax.m);
+  load_line_twiddles(p.twy, taby, ay.m);
   return p;
 }
 __device__ __forceinline__ void as_rows(Tile& t, const PlaneGeo& g) {
@@ -101,9 +101,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_fwd_kerne
   extern __shared__ __align__(16) float2 sm[];
   depend_wait();
   a.src = after_wait(a.src);
-  ax.tw = after_wait(ax.tw);
-  ay.tw = after_wait(ay.tw);
-  PlaneTile p = plane_init(g, ax, ay, sm);
+  PlaneTile p = plane_init(g, ax, ay, after_wait(ax.tw), after_wait(ay.tw), sm);
   __syncthreads();
   const int H = a.H, W = a.W, Wh = a.Wh, zp = g.zp;
   const float* __restrict__ src = a.src + (long)blockIdx.x * H * W;
@@ -126,9 +124,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_inv_kerne
   depend_wait();
   a.half_in = after_wait(a.half_in);
   a.dst = after_wait(a.dst);
-  ax.tw = after_wait(ax.tw);
-  ay.tw = after_wait(ay.tw);
-  PlaneTile p = plane_init(g, ax, ay, sm);
+  PlaneTile p = plane_init(g, ax, ay, after_wait(ax.tw), after_wait(ay.tw), sm);
   __syncthreads();
   const int H = a.H, W = a.W, Wh = a.Wh;
   columns_inverse(p, g, ay, Wh, a.half_in + (long)blockIdx.x * H * Wh);
@@ -153,7 +149,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_epi_kerne
   extern __shared__ __align__(16) float2 sm[];
   __shared__ RowPair rp[kMaxTileLines];
   __shared__ EpiShared sh;
-  PlaneTile p = plane_init(g, ax, ay, sm);
+  PlaneTile p = plane_init(g, ax, ay, ax.tw, ay.tw, sm);
   depend_wait();
   epi_after_wait(a);
   const int w = blockIdx.x / t.D, z = blockIdx.x - w * t.D;

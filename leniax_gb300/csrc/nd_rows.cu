@@ -53,8 +53,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_fwd_kerne
   t.nld = a.nrd;
   depend_wait();
   a.src = after_wait(a.src);
-  ax.tw = after_wait(ax.tw);
-  load_line_twiddles(tw, ax);
+  load_line_twiddles(tw, after_wait(ax.tw), ax.m);
   for (int l = threadIdx.x; l < a.nr; l += blockDim.x) tile_pair(a, l, row + l, cnt + l);
   __syncthreads();
   const float* __restrict__ src = a.src;
@@ -94,8 +93,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_inv_kerne
   depend_wait();
   a.half_in = after_wait(a.half_in);
   a.dst = after_wait(a.dst);
-  ax.tw = after_wait(ax.tw);
-  load_line_twiddles(tw, ax);
+  load_line_twiddles(tw, after_wait(ax.tw), ax.m);
   for (int l = threadIdx.x; l < a.nr; l += blockDim.x) tile_pair(a, l, row + l, cnt + l);
   __syncthreads();
   const float2* __restrict__ half = a.half_in;
@@ -199,7 +197,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
   const int w = blockIdx.x / a.tiles, b = blockIdx.x - w * a.tiles;
   const int sol = w / a.n_init;
   const int W = t.W, Wh = t.Wh, C = t.C, K = t.K, zp = g.zp;
-  load_line_twiddles(tw, ax);
+  load_line_twiddles(tw, ax.tw, ax.m);
   depend_wait();
   epi_after_wait(a);
   const int s0 = a.shift[3 * w], s1 = a.shift[3 * w + 1], s2 = a.shift[3 * w + 2];
