@@ -164,10 +164,18 @@ __device__ __noinline__ void big2d_item(const BigArgs& a, int world, const float
       for (int n2 = 0; n2 < P; ++n2) v[n2] = make_float2(src[(2 * r) * N + t + G * n2], src[(2 * r + 1) * N + t + G * n2]);
       float2 u[Q][G];
       fft_standard<GE, false, false>(v, u, scr, tw_std, t, gmask);
+      __syncwarp(gmask);
+      // the row leaves in order, 128 bytes a group and store, by way of the
+      // scratch: its pair-adjacent positions are 16 bytes apart across lanes
 #pragma unroll
       for (int q = 0; q < Q; ++q)
 #pragma unroll
-        for (int k1 = 0; k1 < G; ++k1) spec[r * N + pa_pos<N>(t + G * q + P * k1)] = u[q][k1];
+        for (int k1 = 0; k1 < G; ++k1) scr[pa_pos<N>(t + G * q + P * k1)] = u[q][k1];
+      __syncwarp(gmask);
+      float4* out = reinterpret_cast<float4*>(spec + r * N);
+#pragma unroll
+      for (int i = 0; i < N / 2 / G; ++i) out[t + G * i] = reinterpret_cast<const float4*>(scr)[t + G * i];
+      __syncwarp(gmask);
     }
     __syncthreads();
     for (int c = grp; c < N / 2; c += NG) {  // column pass
