@@ -95,43 +95,55 @@ __device__ __forceinline__ float step_dt(const NdTab& t, const EpiArgs& a, int w
   return 1.f / __ldg(a.dt + sol);
 }
 
-// Growth of one potential: the gaussian inline (the form of GrowthP: the
-// scale folds 1/s and sqrt(log2 e / 2)), the others out of line, so that an
-// unrolled butterfly's epilogue stays small.
+// Growth of one potential: the gaussian inline, the others out of line, so that
+// an unrolled butterfly's epilogue stays small.
 static __device__ __noinline__ float growth_any(int id, float u, float m, float s) { return growth_fn(id, u, m, s); }
 struct NdGrowth {
-  GrowthP p;
+  int id;
+  bool inl;  // the inline form holds: gaussian, its coefficient within float32's normal range
+  float m, s;
   // the exponent's coefficient log2(e) / (2 s^2) as an unevaluated sum c + dc:
   // rounded to one float its error is the same in every cell of a world, and a
-  // world's growth shows it where cells' roundings average out
+  // world's growth shows it where cells' roundings average out.  c is rounded
+  // down and dc > 0, so that both parts of the exponent of an infinite square
+  // are -inf (growth -1), not inf - inf.
   float c, dc;
-  __device__ __forceinline__ NdGrowth(int id, float m, float s) {
-    p.id = id;
-    p.m = m;
-    p.s = s;
+  // Widths whose square, coefficient and remainder are all normal floats; for
+  // the others (0, tiny, huge, infinite, NaN) growth_fn's quotient is exact
+  // where the sum c + dc is infinite or NaN.
+  __device__ __forceinline__ static bool regular(float s) { return fabsf(s) >= 0x1p-50f && fabsf(s) <= 0x1p50f; }
+  __device__ __forceinline__ NdGrowth(int id, float m, float s)
+      : id(id), inl(id == LGX_GF_GAUSSIAN && regular(s)), m(m), s(s), c(0.f), dc(0.f) {
+    if (!inl) return;
     const float q = s * s, dq = fmaf(s, s, -q);  // s^2 = q + dq
+    const auto rest = [=](float c) { return (fmaf(-c, q, kC) + (kDc - c * dq)) / q; };
     c = kC / q;
-    dc = (fmaf(-c, q, kC) + (kDc - c * dq)) / q;
+    dc = rest(c);
+    if (!(dc > 0.f)) {
+      c = __int_as_float(__float_as_int(c) - 1);
+      dc = rest(c);
+    }
   }
   static constexpr double kLog2E2 = 0.72134752044448170368;  // log2(e) / 2
   static constexpr float kC = (float)kLog2E2, kDc = (float)(kLog2E2 - (double)kC);
   // the gaussian's exponential at both cells
   __device__ __forceinline__ float2 gauss(float2 u) const {
-    const float2 d = __fadd2_rn(u, make_float2(-p.m, -p.m));
+    const float2 d = __fadd2_rn(u, make_float2(-m, -m));
     const float2 d2 = __fmul2_rn(d, d);
     const float2 x = __ffma2_rn(d2, make_float2(-c, -c), __fmul2_rn(d2, make_float2(-dc, -dc)));
     return make_float2(fast_exp2(x.x), fast_exp2(x.y));
   }
-  // weighted growth of a pair: w (2 e - 1)
+  // weighted growth of a pair: w (2 e - 1), for weights whose double is finite
   __device__ __forceinline__ float2 gauss_weighted(float2 u, float w) const {
     return __ffma2_rn(make_float2(2.f * w, 2.f * w), gauss(u), make_float2(-w, -w));
   }
+  __device__ __forceinline__ static bool foldable(float w) { return fabsf(w) <= 0x1p126f; }
   __device__ __forceinline__ float operator()(float u) const {
-    if (p.id == LGX_GF_GAUSSIAN) {
-      const float d = u - p.m, d2 = d * d;
+    if (inl) {
+      const float d = u - m, d2 = d * d;
       return fmaf(2.f, fast_exp2(fmaf(d2, -c, d2 * -dc)), -1.f);
     }
-    return growth_any(p.id, u, p.m, p.s);
+    return growth_any(id, u, m, s);
   }
 };
 
@@ -253,12 +265,9 @@ __device__ __forceinline__ void epi_channel_mass(EpiShared& sh, int c, float cm)
 // fetch.
 template <bool GAUSS, bool V1>
 __device__ __forceinline__ void epi_pairs(const NdTab& t, const EpiArgs& a, const RowPair* rp, float2* Z, int nl,
-                                          int zp, int lanes, int w, int sx, float dt, Moments& mo) {
-  const int W = t.W, sol = w / a.n_init;
-  const float* gf = a.gf + sol * a.gf_sol_stride;
-  const NdGrowth grow(t.gf[0], __ldg(gf), __ldg(gf + 1));
-  const float wk = __ldg(a.w + sol * a.w_sol_stride);
-  const float wf = t.mean ? wk / wk : wk;  // weighted_mean with one kernel: (w g) / w
+                                          int zp, int lanes, int w, int sx, float dt, const NdGrowth& grow, float wf,
+                                          Moments& mo) {
+  const int W = t.W;
   const float wrap = (float)W, top = (float)(W - W / 2);
   const int x0 = threadIdx.x & (lanes - 1);
   const int per = __ffs(lanes) - 1;
@@ -328,10 +337,15 @@ __device__ __forceinline__ void epi_pairs(const NdTab& t, const EpiArgs& a, cons
 }
 __device__ __forceinline__ void epi_single(const NdTab& t, const EpiArgs& a, const RowPair* rp, float2* Z, int nl,
                                            int zp, int lanes, int w, int sx, float dt, Moments& mo) {
-  if (t.gf[0] == LGX_GF_GAUSSIAN && t.state_fn == LGX_STATE_V1)
-    epi_pairs<true, true>(t, a, rp, Z, nl, zp, lanes, w, sx, dt, mo);
+  const int sol = w / a.n_init;
+  const float* gf = a.gf + sol * a.gf_sol_stride;
+  const NdGrowth grow(t.gf[0], __ldg(gf), __ldg(gf + 1));
+  const float wk = __ldg(a.w + sol * a.w_sol_stride);
+  const float wf = t.mean ? wk / wk : wk;  // weighted_mean with one kernel: (w g) / w
+  if (grow.inl && grow.foldable(wf) && t.state_fn == LGX_STATE_V1)
+    epi_pairs<true, true>(t, a, rp, Z, nl, zp, lanes, w, sx, dt, grow, wf, mo);
   else
-    epi_pairs<false, false>(t, a, rp, Z, nl, zp, lanes, w, sx, dt, mo);
+    epi_pairs<false, false>(t, a, rp, Z, nl, zp, lanes, w, sx, dt, grow, wf, mo);
 }
 // threads per row pair: the power of two in 8..32 that leaves the fewest idle
 inline int epi_lanes(int W) {
