@@ -111,8 +111,7 @@ struct LineAxis {
   int ns[kLineStages], ins[kLineStages];   // Ns: product of the radices before the stage
   FastDivU nbd[kLineStages];               // by the stage's butterflies m / r
   FastDivU nsd[kLineStages], insd[kLineStages];
-  const float2* tw;                        // W_m^j, j < m
-  const float2 *chirp, *bhat;              // Bluestein tables (n and m entries), else null
+  const float2* tw;                        // W_m^j, j < m; Bluestein lines: then the chirp (n) and its filter (m)
 };
 
 inline bool wide_radix(int r) { return (r >= 8 && r <= 10) || r == 12 || (r >= 14 && r <= 16); }
@@ -221,8 +220,6 @@ inline bool make_line_axis(int n, int m, float2* tables, LineAxis* ax, bool allo
     ins *= ri;
   }
   ax->tw = tables;
-  ax->chirp = m != n ? tables + m : nullptr;
-  ax->bhat = m != n ? tables + m + n : nullptr;
   return true;
 }
 inline size_t line_table_elems(int n, int m) { return (size_t)m + (m != n ? (size_t)n + m : 0); }
@@ -235,6 +232,9 @@ inline size_t line_table_elems(int n, int m) { return (size_t)m + (m != n ? (siz
 // innermost (`lp` lines, odd, per point); otherwise a line is `lp` points.
 struct Tile {
   float2* b[2];  // every transform's last exchange leaves b[1] free for the next one's first
+  // the axis' tables, for Bluestein lines: after_wait(LineAxis::tw), as the
+  // kernel may depend on the launch that writes them
+  const float2* tab;
   int lp;
   int nl;
   FastDivU nld;  // by nl
@@ -493,8 +493,8 @@ __device__ __forceinline__ void line_center(const LineAxis& ax, const float2* tw
 template <bool INV, bool LINES, class In, class Out>
 __device__ __forceinline__ void line_bluestein(const LineAxis& ax, const float2* tw, Tile& t, const In& in1,
                                                const Out& out1) {
-  const float2 *chirp = ax.chirp, *bhat = ax.bhat;
   const int n = ax.n;
+  const float2 *chirp = t.tab + ax.m, *bhat = chirp + n;
   const float inv_m = 1.f / (float)ax.m;
   line_head<false, LINES>(ax, tw, t, [&](int l, int j, int nb, auto& v) {
     constexpr int R = (int)(sizeof(v) / sizeof(float2));

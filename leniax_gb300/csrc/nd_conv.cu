@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_conv_kernel(Nd
   const int I = (int)g.I;
   load_line_twiddles(tw, ax.tw, ax.m);
   depend_wait();
+  tl.tab = after_wait(ax.tw);
   a.S = after_wait(a.S);
   __syncthreads();
   const float2 zero = make_float2(0.f, 0.f);
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_adj_conv_kerne
   const int I = (int)g.I;
   load_line_twiddles(tw, ax.tw, ax.m);
   depend_wait();
+  tl.tab = after_wait(ax.tw);
   a.S = after_wait(a.S);
   a.A = after_wait(a.A);
   a.gk = after_wait(a.gk);
@@ -205,7 +207,8 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_columns_kernel
   const int I = (int)a.g.I;
   depend_wait();
   a.data = after_wait(a.data);
-  load_line_twiddles(tw, after_wait(ax.tw), ax.m);
+  tl.tab = after_wait(ax.tw);
+  load_line_twiddles(tw, tl.tab, ax.m);
   __syncthreads();
   float2* d = a.data + plane * a.g.I * ax.n + i0;
   line_fft<INV, true, KIND>(

@@ -53,7 +53,8 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_fwd_kerne
   t.nld = a.nrd;
   depend_wait();
   a.src = after_wait(a.src);
-  load_line_twiddles(tw, after_wait(ax.tw), ax.m);
+  t.tab = after_wait(ax.tw);
+  load_line_twiddles(tw, t.tab, ax.m);
   for (int l = threadIdx.x; l < a.nr; l += blockDim.x) tile_pair(a, l, row + l, cnt + l);
   __syncthreads();
   const float* __restrict__ src = a.src;
@@ -93,7 +94,8 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_inv_kerne
   depend_wait();
   a.half_in = after_wait(a.half_in);
   a.dst = after_wait(a.dst);
-  load_line_twiddles(tw, after_wait(ax.tw), ax.m);
+  t.tab = after_wait(ax.tw);
+  load_line_twiddles(tw, t.tab, ax.m);
   for (int l = threadIdx.x; l < a.nr; l += blockDim.x) tile_pair(a, l, row + l, cnt + l);
   __syncthreads();
   const float2* __restrict__ half = a.half_in;
@@ -200,6 +202,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
   load_line_twiddles(tw, ax.tw, ax.m);
   depend_wait();
   epi_after_wait(a);
+  tl.tab = after_wait(ax.tw);
   const int s0 = a.shift[3 * w], s1 = a.shift[3 * w + 1], s2 = a.shift[3 * w + 2];
   const int sx = t.nd == 3 ? s2 : s1;
   const float dt = step_dt(t, a, w, sol);

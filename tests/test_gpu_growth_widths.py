@@ -59,7 +59,7 @@ def test_extreme_widths(cuda, world, n, C, per, width):
 
 
 @pytest.mark.parametrize('world,n,C,per', WORLDS)
-@pytest.mark.parametrize('width', [0.015, 0.03, 0.05, 0.07, 0.11, 0.13, -0.05])
+@pytest.mark.parametrize('width', [0.015, 0.05, 0.07, 0.09, 0.13, -0.05, -0.09])
 def test_potentials_with_infinite_squares(cuda, world, n, C, per, width):
     K, mp, upd, Ko, mpo = _model(cuda, world, C, per, width)
     rng = np.random.Generator(np.random.PCG64(6))
