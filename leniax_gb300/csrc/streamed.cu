@@ -699,24 +699,28 @@ __global__ void __launch_bounds__(RowInvCfg<N>::T, RowInvCfg<N>::MINB) row_inv_k
 // items one after another in N/2/GPB blocks, which leaves the chip idle and
 // the step as long as that chain.  Here a block owns the 32 / G packed rows of
 // one warp's transforms and one output channel, its warps take the channel's
-// kernels in turn (rows straight from L2 into the transform), the weighted
-// growths meet in shared memory, and the warps share the cells of the
-// epilogue; warp 0 then runs the fused forward transform of the new rows while
-// another sums the moments.  Bound by instruction issue of a lone block an SM
-// (48 blocks for one 128^2 world of three channels); 15 kernels of one 128^2
-// world: 43 us a step walking, 8.9 us split.
+// kernels in turn (rows straight from L2 into the transform), the growths meet
+// in shared memory, and the warps share the cells of the epilogue; warp 0 then
+// runs the fused forward transform of the new rows while another sums the
+// moments.  The growths of a cell are added in kernel order, as row_inv_kernel
+// adds them, so fields, potentials and states are the same bits whatever the
+// batch (the moments' sums are not: other blocks, other order).  Bound by
+// instruction issue of a lone block an SM (48 blocks for one 128^2 world of
+// three channels); 15 kernels of one 128^2 world: 43 us a step walking,
+// 9.3 us split.
 template <int N>
 struct SplitCfg {
   static constexpr int G = SCfg<N>::G;
   static constexpr int RPB = 32 / G;          // packed rows per block
   static constexpr int BPC = (N / 2) / RPB;   // blocks per world and channel
   static constexpr int XCH = RPB * (N + G);   // float2 of exchange scratch per warp
+  static constexpr int ACC = (N / G) * 32;    // float2: a row pair of growths per lane
 };
 constexpr int kSplitMinWarps = 4, kSplitMaxWarps = 8;
 
 template <int N>
 size_t row_inv_split_smem(int warps) {
-  return ((size_t)3 * N + (size_t)warps * SplitCfg<N>::XCH) * sizeof(float2) +
+  return ((size_t)3 * N + (size_t)warps * SplitCfg<N>::XCH + SplitCfg<N>::ACC) * sizeof(float2) +
          (size_t)warps * (RAW_CM + kMaxChannels) * sizeof(float);
 }
 
@@ -732,12 +736,14 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
   using GE = Geo<N, G>;
   constexpr int P = GE::P, Q = GE::Q;
   constexpr int RAWS_MAX = RAW_CM + kMaxChannels;
-  static_assert(SC::XCH >= P * 32, "a warp's scratch holds its weighted growths");
+  static_assert(SC::XCH >= P * 32 && SC::ACC == P * 32, "a warp's scratch holds its growths");
+  __shared__ float wk_s[kSplitMaxWarps];
   extern __shared__ __align__(16) float2 sm[];
   const int warps = blockDim.x >> 5, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float2* tw = sm;                      // 3N twiddles
   float2* xch = tw + 3 * N;             // [warps][XCH]
-  float* red = reinterpret_cast<float*>(xch + warps * SC::XCH);  // [warps][RAWS_MAX]
+  float2* sum = xch + warps * SC::XCH;  // [P][32] weighted growths of the rounds before the last
+  float* red = reinterpret_cast<float*>(sum + SC::ACC);  // [warps][RAWS_MAX]
   const int C = tab.C, K = tab.K;
   const int n = blockIdx.x / (BPC * C);
   if (n >= n_worlds) return;
@@ -753,7 +759,6 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
   // bit k: kernel k feeds this channel / an earlier one / any channel
   static_assert(kMaxKernels <= 64, "one bit per kernel");
   unsigned long long fed = 0ull, before = 0ull, any = 0ull;
-  float wsum = 0.f;
   for (int h = 0; h < K; h += 32) {
     const int k = h + lane;
     for (int c = 0; c < C; ++c) {
@@ -761,13 +766,12 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
       const unsigned long long b = (unsigned long long)__ballot_sync(0xffffffffu, w != 0.f) << h;
       any |= b;
       if (c < co) before |= b;
-      if (c == co) {
-        fed = fed | b;
-        wsum += w;
-      }
+      if (c == co) fed |= b;
     }
   }
-  wsum = warp_sum(wsum);
+  float wsum = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < K; ++k) wsum += __ldg(wt + co * K + k);
   // channel 0 also takes the kernels that feed no channel (their potentials count)
   const unsigned long long all = K == 64 ? ~0ull : (1ull << K) - 1ull;
   const unsigned long long mine = fed | (co == 0 ? all & ~any : 0ull);
@@ -785,59 +789,76 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
   const size_t base = ((size_t)n * C + co) * N * N + (size_t)(2 * r) * N;
   float cpot = 0.f;
   float2* scr = xch + wid * SC::XCH;
-  float2 acc[P];
-#pragma unroll
-  for (int k1 = 0; k1 < P; ++k1) acc[k1] = make_float2(0.f, 0.f);
+  // A round: every warp takes one kernel and leaves its growths in its scratch,
+  // then the warps add them up, cell by cell in kernel order (warp w the cells
+  // k1 = w, w + warps, ...); the last round's sum is taken by the epilogue.
+  auto add_round = [&](float2 f, int k1, int items) {
+    for (int q = 0; q < items; ++q) {
+      const float2 e = xch[q * SC::XCH + k1 * 32 + lane];
+      const float wk = wk_s[q];
+      f.x = fmaf(wk, e.x, f.x);
+      f.y = fmaf(wk, e.y, f.y);
+    }
+    return f;
+  };
+  unsigned long long todo = mine;  // kernels of this and later rounds
+  int left = __popcll(mine);
+  const bool rounds = left > warps;  // more than one
+  if (rounds)
+    for (int k1 = wid; k1 < P; k1 += warps) sum[k1 * 32 + lane] = make_float2(0.f, 0.f);
   __syncthreads();
-  int rank = 0;
-  for (unsigned long long todo = mine; todo; todo &= todo - 1) {
-    if (rank++ % warps != wid) continue;
-    const int k = __ffsll((long long)todo) - 1;
-    const float2* row = prod + (((size_t)n * K + k) * (N / 2) + r) * N;
-    float2 v[Q][G];
-    if constexpr (Q == 1) unpack_row_pair_q1<GE>(row, v, t);
-    else unpack_row_pair_pa<GE>(row, v, t);
-    float2 w[P];
-    __syncwarp();  // the previous item's exchange has been read
-    fft_mirrored<GE, true, true>(v, w, scr + grp * GE::SCR, tw + 2 * N, t, gmask);
-    if (!((before >> k) & 1ull)) {
+  for (;;) {
+    unsigned long long m = todo;
+    for (int q = 0; q < wid; ++q) m &= m - 1;
+    const int k = m ? __ffsll((long long)m) - 1 : 0;
+    if (m) {
+      const float2* row = prod + (((size_t)n * K + k) * (N / 2) + r) * N;
+      float2 v[Q][G];
+      if constexpr (Q == 1) unpack_row_pair_q1<GE>(row, v, t);
+      else unpack_row_pair_pa<GE>(row, v, t);
+      float2 w[P];
+      fft_mirrored<GE, true, true>(v, w, scr + grp * GE::SCR, tw + 2 * N, t, gmask);
+      if (!((before >> k) & 1ull)) {
 #pragma unroll
-      for (int k1 = 0; k1 < P; ++k1) cpot += (w[k1].x > kEps ? 1.f : 0.f) + (w[k1].y > kEps ? 1.f : 0.f);
-      if (pot_out) {
-        float* po = pot_out + ((size_t)n * K + k) * N * N + (size_t)(2 * r) * N;
+        for (int k1 = 0; k1 < P; ++k1) cpot += (w[k1].x > kEps ? 1.f : 0.f) + (w[k1].y > kEps ? 1.f : 0.f);
+        if (pot_out) {
+          float* po = pot_out + ((size_t)n * K + k) * N * N + (size_t)(2 * r) * N;
 #pragma unroll
-        for (int k1 = 0; k1 < P; ++k1) {
-          po[t + G * k1] = w[k1].x;
-          po[N + t + G * k1] = w[k1].y;
+          for (int k1 = 0; k1 < P; ++k1) {
+            po[t + G * k1] = w[k1].x;
+            po[N + t + G * k1] = w[k1].y;
+          }
         }
       }
-    }
-    if ((fed >> k) & 1ull) {
-      const float wk = __ldg(wt + co * K + k);
+      // a kernel that feeds no channel adds 0
+      const bool feeds = (fed >> k) & 1ull;
+      const float wk = feeds ? __ldg(wt + co * K + k) : 0.f;
+      if (lane == 0) wk_s[wid] = GF == GF_GENERIC ? wk : 2.f * wk;
       GrowthP g;
       g.m = __ldg(gf + 2 * k);
       g.s = __ldg(gf + 2 * k + 1);
       g.a = GF == GF_FAST_GAUSSIAN ? 0.84932180028801904272f / g.s : (GF == GF_FAST_POLY4 ? 1.f / (9.f * (g.s * g.s)) : 0.f);
       g.id = tab.gf[k];
+      __syncwarp();  // every group of the warp has read its exchange
 #pragma unroll
       for (int k1 = 0; k1 < P; ++k1) {
-        if constexpr (GF == GF_GENERIC) {
-          acc[k1].x = fmaf(wk, growth_cell<GF>(g, w[k1].x), acc[k1].x);
-          acc[k1].y = fmaf(wk, growth_cell<GF>(g, w[k1].y), acc[k1].y);
-        } else {  // w (2 e - 1) summed as 2 w e here, minus the channel's weight sum below
-          acc[k1] = __ffma2_rn(make_float2(2.f * wk, 2.f * wk), growth_core2<GF>(g, w[k1]), acc[k1]);
+        float2 e = make_float2(0.f, 0.f);
+        if (feeds) {
+          if constexpr (GF == GF_GENERIC) e = make_float2(growth_cell<GF>(g, w[k1].x), growth_cell<GF>(g, w[k1].y));
+          else e = growth_core2<GF>(g, w[k1]);  // w (2 e - 1): 2 w e here, minus the channel's weight sum below
         }
+        scr[k1 * 32 + lane] = e;
       }
     }
+    __syncthreads();
+    if (left <= warps) break;
+    for (int k1 = wid; k1 < P; k1 += warps) sum[k1 * 32 + lane] = add_round(sum[k1 * 32 + lane], k1, warps);
+    for (int q = 0; q < warps; ++q) todo &= todo - 1;
+    left -= warps;
+    __syncthreads();
   }
-  __syncwarp();
-#pragma unroll
-  for (int k1 = 0; k1 < P; ++k1) scr[k1 * 32 + lane] = acc[k1];
-  __syncthreads();
 
-  // field (weighted_sum / weighted_mean, core.py:202-242), state update,
-  // moments: warp w takes the cells k1 = w, w + warps, ...
-  const int nacc = rank < warps ? rank : warps;
+  // field (weighted_sum / weighted_mean, core.py:202-242), state update, moments
   const float cya = (float)(((2 * r - sy) & (N - 1)) - N / 2);
   const float cyb = (float)(((2 * r + 1 - sy) & (N - 1)) - N / 2);
   float Sa = 0.f, Sb = 0.f, Ga = 0.f, Gb = 0.f, cmass = 0.f, cgrow = 0.f, mxx = 0.f, gxx = 0.f, m2x = 0.f;
@@ -846,12 +867,8 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
   for (int k1 = wid; k1 < P; k1 += warps) {
     const int x = t + G * k1;
     const float sa = __ldg(state + base + x), sb = __ldg(state + base + N + x);
-    float fa = 0.f, fb = 0.f;
-    for (int q = 0; q < nacc; ++q) {
-      const float2 a = xch[q * SC::XCH + k1 * 32 + lane];
-      fa += a.x;
-      fb += a.y;
-    }
+    const float2 f = add_round(rounds ? sum[k1 * 32 + lane] : make_float2(0.f, 0.f), k1, left);
+    float fa = f.x, fb = f.y;
     if constexpr (GF != GF_GENERIC) {
       fa -= wsum;
       fb -= wsum;
