@@ -19,8 +19,6 @@ LIB = os.path.join(HERE, '_lgx.so')
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 NVCC_FLAGS = ['-O3', '-lineinfo', '-std=c++17', '--expt-relaxed-constexpr', '-Xcompiler', '-fPIC',
               '-Xcompiler', '-fvisibility=hidden', '-Xptxas', '-warn-spills']
-# the N-D engine's kernels hold one body per radix: their functions are compiled side by side
-SPLIT_FLAGS = ['--split-compile=4']
 
 
 def nvcc_path():
@@ -53,8 +51,7 @@ def build(verbose=False, force=False, extra_flags=()):
         obj = os.path.join(OBJ, os.path.basename(src)[:-3] + '.o')
         objs.append(obj)
         if force or _stale(obj, [src] + headers):
-            split = SPLIT_FLAGS if os.path.basename(src).startswith('nd_') else []
-            cmd = [nvcc] + ARCH + NVCC_FLAGS + split + list(extra_flags) + ['-c', src, '-o', obj]
+            cmd = [nvcc] + ARCH + NVCC_FLAGS + list(extra_flags) + ['-c', src, '-o', obj]
             jobs.append(cmd)
 
     def run(cmd):
