@@ -355,6 +355,11 @@ inline int epi_lanes(int W) {
   return best;
 }
 
+// Threads of an epilogue block: a world of many small tiles has its last block
+// walk as many partials (epi_finish), for which it needs warps.  A step of one
+// world, us, one warp -> four: 1024 x 8 x 8 85 -> 40, 4096 x 4 x 4 274 -> 113.
+inline int epi_threads(int threads, int bpw) { return bpw > 256 ? std::max(threads, 128) : threads; }
+
 // Block b of world w: reduce the threads' moments into the block's partial;
 // the world's last block to finish (a ticket on the world's counter; no block
 // waits) reduces all of the world's block partials in a fixed order into the
@@ -393,9 +398,23 @@ __device__ __forceinline__ void epi_finish(const NdTab& t, const EpiArgs& a, Epi
   __syncthreads();
   if (!sh.last) return;
   __threadfence();
+  // A world of small tiles has many partials and this block few warps: loads in
+  // flight, not one round trip to L2 a partial.  A step of one world, us, one
+  // load at a time -> sixteen (and epi_threads): 100^2 31.5 -> 26.0, 144^2
+  // 39.8 -> 26.2, 500^2 72 -> 52, 1031 x 64 94 -> 40, 1024 x 8 x 8 255 -> 40.
+  constexpr int kLoads = 16;
   for (int s = lane; s < RAWS; s += 32) {
     float acc = 0.f;
-    for (int bb = wid; bb < bpw; bb += NWARP) acc += __ldcg(pw + (long)bb * RAWS + s);
+    for (int b0 = wid; b0 < bpw; b0 += kLoads * NWARP) {
+      float v[kLoads];
+#pragma unroll
+      for (int j = 0; j < kLoads; ++j) {
+        const int bb = b0 + j * NWARP;
+        v[j] = bb < bpw ? __ldcg(pw + (long)bb * RAWS + s) : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < kLoads; ++j) acc += v[j];
+    }
     sh.red[wid][s] = acc;
   }
   __syncthreads();

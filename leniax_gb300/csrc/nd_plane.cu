@@ -356,7 +356,8 @@ cudaError_t nd_plane_epilogue(const NdTab& t, const NdAxes& ax, const EpiArgs& a
   auto f = t.C == 1 && t.K == 1 ? nd_plane_epi_kernel<true> : nd_plane_epi_kernel<false>;
   const cudaError_t e = nd_allow_smem((const void*)f);
   if (e != cudaSuccess) return e;
-  return launch_dependent(f, dim3((unsigned)blocks, a.split ? t.C : 1), p.threads, smem, st, t, a, p.g, ax.x, ax.y);
+  return launch_dependent(f, dim3((unsigned)blocks, a.split ? t.C : 1), epi_threads(p.threads, a.bpw), smem, st, t, a,
+                          p.g, ax.x, ax.y);
 }
 
 }  // namespace lgx

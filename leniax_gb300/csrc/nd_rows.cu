@@ -425,7 +425,7 @@ cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& a
   });
   const cudaError_t err = nd_allow_smem((const void*)f);
   if (err != cudaSuccess) return err;
-  return launch_dependent(f, dim3((unsigned)blocks, e.split ? t.C : 1), e.rt.threads, e.smem, st, t, a, g, x);
+  return launch_dependent(f, dim3((unsigned)blocks, e.split ? t.C : 1), epi_threads(e.rt.threads, a.bpw), e.smem, st, t, a, g, x);
 }
 
 }  // namespace lgx
