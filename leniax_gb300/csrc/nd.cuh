@@ -257,12 +257,11 @@ __device__ __forceinline__ void epi_channel_mass(EpiShared& sh, int c, float cm)
 
 // The epilogue of the packed pairs of potentials in Z [nl][zp] (C = K = 1):
 // growth, state update, stores and moments, the new cells left in Z.  `lanes`
-// neighbouring threads take a row pair (the power of two that W wastes least
-// of), so the row coordinates multiply row sums and the cells of a pair go
-// through the packed FP32x2 pipe.  A rolled loop of its own rather than the
-// middle of the row transform's butterflies: inlined there it was unrolled
-// over every radix, and blocks that run the code once stalled on instruction
-// fetch.
+// neighbouring threads take a row pair (epi_lanes), so the row coordinates
+// multiply row sums and the cells of a pair go through the packed FP32x2 pipe.
+// A rolled loop of its own rather than the middle of the row transform's
+// butterflies: inlined there it was unrolled over every radix, and blocks that
+// run the code once stalled on instruction fetch.
 template <bool GAUSS, bool V1>
 __device__ __forceinline__ void epi_pairs(const NdTab& t, const EpiArgs& a, const RowPair* rp, float2* Z, int nl,
                                           int zp, int lanes, int w, int sx, float dt, const NdGrowth& grow, float wf,
@@ -347,11 +346,16 @@ __device__ __forceinline__ void epi_single(const NdTab& t, const EpiArgs& a, con
   else
     epi_pairs<false, false>(t, a, rp, Z, nl, zp, lanes, w, sx, dt, grow, wf, mo);
 }
-// threads per row pair: the power of two in 8..32 that leaves the fewest idle
-inline int epi_lanes(int W) {
+// Threads per row pair: the power of two in 8..32 that leaves the fewest idle
+// along a row; more where a tile has fewer pairs than its threads have warps
+// (rows of thousands of cells).  A step, us, 32 -> 256 threads for a pair of
+// 4096: one world of 4 x 4096 70 -> 35, of 16 x 4096 66 -> 34, 32 of 4 x 4096
+// 69 -> 36.
+inline int epi_lanes(int W, int nl, int threads) {
   int best = 32;
   for (int p : {16, 8})
     if ((W + p - 1) / p * p < (W + best - 1) / best * best) best = p;
+  while (best >= 32 && threads % (2 * best) == 0 && 2 * best * nl <= threads && best < W) best *= 2;
   return best;
 }
 

@@ -286,7 +286,7 @@ PlanePlan plane_plan(const NdTab& t, const NdAxes& ax) {
   g.ppd = make_fastdiv((unsigned)g.pp);
   g.whd = make_fastdiv((unsigned)t.Wh);
   g.field_smem = 0;
-  g.lanes = epi_lanes(t.W);
+  g.lanes = 0;  // the epilogue's, by its threads
   p.threads = nd_threads(std::max(line_items(ax.x, g.pp), line_items(ax.y, t.Wh)));
   p.smem = (size_t)(t.W + t.H + 2 * g.buf + g.keep) * sizeof(float2);
   return p;
@@ -350,14 +350,15 @@ cudaError_t nd_plane_epilogue(const NdTab& t, const NdAxes& ax, const EpiArgs& a
   a.bpw = nd_plane_epi_blocks(t, ax, a.n_worlds, &field_global);
   a.split = a.bpw > a.tiles ? 1 : 0;
   p.g.field_smem = field_global ? 0 : 1;
+  const int threads = epi_threads(p.threads, a.bpw);
+  p.g.lanes = epi_lanes(t.W, p.g.pp, threads);
   const size_t smem = p.smem + (p.g.field_smem ? plane_field_bytes(t, p, a.split) : 0);
   const long blocks = (long)a.n_worlds * t.D;
   if (blocks >= (1L << 31)) return cudaErrorInvalidConfiguration;
   auto f = t.C == 1 && t.K == 1 ? nd_plane_epi_kernel<true> : nd_plane_epi_kernel<false>;
   const cudaError_t e = nd_allow_smem((const void*)f);
   if (e != cudaSuccess) return e;
-  return launch_dependent(f, dim3((unsigned)blocks, a.split ? t.C : 1), epi_threads(p.threads, a.bpw), smem, st, t, a,
-                          p.g, ax.x, ax.y);
+  return launch_dependent(f, dim3((unsigned)blocks, a.split ? t.C : 1), threads, smem, st, t, a, p.g, ax.x, ax.y);
 }
 
 }  // namespace lgx

@@ -411,7 +411,8 @@ cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& a
   g.nr = e.rt.nr;
   g.pitch = e.rt.pitch;
   g.zp = e.rt.zp;
-  g.lanes = epi_lanes(t.W);
+  const int threads = epi_threads(e.rt.threads, a.bpw);
+  g.lanes = epi_lanes(t.W, e.rt.nr, threads);
   g.buf = e.rt.buf;
   g.nrd = make_fastdiv((unsigned)g.nr);
   g.hd = make_fastdiv((unsigned)t.H);
@@ -425,7 +426,7 @@ cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& a
   });
   const cudaError_t err = nd_allow_smem((const void*)f);
   if (err != cudaSuccess) return err;
-  return launch_dependent(f, dim3((unsigned)blocks, e.split ? t.C : 1), epi_threads(e.rt.threads, a.bpw), e.smem, st, t, a, g, x);
+  return launch_dependent(f, dim3((unsigned)blocks, e.split ? t.C : 1), threads, e.smem, st, t, a, g, x);
 }
 
 }  // namespace lgx
