@@ -568,6 +568,29 @@ __device__ __forceinline__ void line_fft(const LineAxis& ax, const float2* tw, T
   }
 }
 
+// The same with rules that take a butterfly's points at once, as the stages do
+// (Bluestein lines: one point).
+template <bool INV, bool LINES, int KIND, class In, class Out>
+__device__ __forceinline__ void line_fft_rules(const LineAxis& ax, const float2* tw, Tile& t, const In& in,
+                                               const Out& out) {
+  if constexpr (KIND == LINE_BLUESTEIN) {
+    line_bluestein<INV, LINES>(
+        ax, tw, t,
+        [&](int l, int i) {
+          float2 v[1];
+          in(l, i, 0, v);
+          return v[0];
+        },
+        [&](int l, int i, float2 x) {
+          const float2 v[1] = {x};
+          out(l, i, 0, v);
+        });
+  } else {
+    line_head<INV, LINES, KIND == LINE_WIDE>(ax, tw, t, in);
+    line_tail<INV, LINES, KIND == LINE_WIDE>(ax, tw, t, out);
+  }
+}
+
 // An axis' twiddles into shared memory (m entries), without a barrier.  The
 // table is a parameter of its own: a kernel that writes to its LineAxis, whose
 // radices are indexed, keeps all of it in local memory.

@@ -138,12 +138,13 @@ struct NdGrowth {
     return __ffma2_rn(make_float2(2.f * w, 2.f * w), gauss(u), make_float2(-w, -w));
   }
   __device__ __forceinline__ static bool foldable(float w) { return fabsf(w) <= 0x1p126f; }
+  __device__ __forceinline__ float any(float u) const { return growth_any(id, u, m, s); }
   __device__ __forceinline__ float operator()(float u) const {
     if (inl) {
       const float d = u - m, d2 = d * d;
       return fmaf(2.f, fast_exp2(fmaf(d2, -c, d2 * -dc)), -1.f);
     }
-    return growth_any(id, u, m, s);
+    return any(u);
   }
 };
 
@@ -177,26 +178,28 @@ struct Moments {
   float m00 = 0.f, g00 = 0.f, cpot = 0.f, cmass = 0.f, cgrow = 0.f;
   float mz = 0.f, my = 0.f, mx = 0.f, gz = 0.f, gy = 0.f, gx = 0.f, qz = 0.f, qy = 0.f, qx = 0.f;
   bool border = false;
-  // one cell of both rows of a pair: entering states, fields, centred x
-  __device__ __forceinline__ void add(const RowPair& r, float2 s, float2 f, float cx, bool xedge) {
-    const float2 g = make_float2(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
-    const float ss = s.x + s.y, gg = g.x + g.y;
-    m00 += ss;
-    g00 += gg;
+  // one cell of both rows of a pair: entering states, positive fields, centred x
+  __device__ __forceinline__ void add_cell(float2 s, float2 g, float cx) {
+    const float ss = s.x + s.y;
     mx = fmaf(ss, cx, mx);
     qx = fmaf(ss * cx, cx, qx);
-    gx = fmaf(gg, cx, gx);
-    const float y0 = s.x * r.cy0, y1 = s.y * r.cy1, z0 = s.x * r.cz0, z1 = s.y * r.cz1;
+    gx = fmaf(g.x + g.y, cx, gx);
+    cmass += (s.x > kEps ? 1.f : 0.f) + (s.y > kEps ? 1.f : 0.f);
+    cgrow += (g.x > kEps ? 1.f : 0.f) + (g.y > kEps ? 1.f : 0.f);
+  }
+  // cells of one pair: their states' and positive fields' sums, the largest
+  // state of each row, whether a cell on the x border is alive
+  __device__ __forceinline__ void add_row(const RowPair& r, float2 S2, float2 G2, float2 most, bool lx) {
+    border |= lx || (most.x > kEps && (r.edge & 1)) || (most.y > kEps && (r.edge & 2));
+    m00 += S2.x + S2.y;
+    g00 += G2.x + G2.y;
+    const float y0 = S2.x * r.cy0, y1 = S2.y * r.cy1, z0 = S2.x * r.cz0, z1 = S2.y * r.cz1;
     my += y0 + y1;
     mz += z0 + z1;
     qy = fmaf(y0, r.cy0, fmaf(y1, r.cy1, qy));
     qz = fmaf(z0, r.cz0, fmaf(z1, r.cz1, qz));
-    gy = fmaf(g.x, r.cy0, fmaf(g.y, r.cy1, gy));
-    gz = fmaf(g.x, r.cz0, fmaf(g.y, r.cz1, gz));
-    const bool l0 = s.x > kEps, l1 = s.y > kEps;
-    cmass += (l0 ? 1.f : 0.f) + (l1 ? 1.f : 0.f);
-    cgrow += (g.x > kEps ? 1.f : 0.f) + (g.y > kEps ? 1.f : 0.f);
-    border |= (l0 && (xedge || (r.edge & 1))) || (l1 && (xedge || (r.edge & 2)));
+    gy = fmaf(G2.x, r.cy0, fmaf(G2.y, r.cy1, gy));
+    gz = fmaf(G2.x, r.cz0, fmaf(G2.y, r.cz1, gz));
   }
   __device__ __forceinline__ void count_pot(float2 u, int rows) {
     cpot += (u.x > kEps ? 1.f : 0.f) + (rows > 1 && u.y > kEps ? 1.f : 0.f);
@@ -309,29 +312,15 @@ __device__ __forceinline__ void epi_pairs(const NdTab& t, const EpiArgs& a, cons
       }
       mo.count_pot(u, r.rows);
       const float2 g = make_float2(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
-      const float ss = s.x + s.y;
       S2 = cadd(S2, s);
       G2 = cadd(G2, g);
-      mo.mx = fmaf(ss, cx, mo.mx);
-      mo.qx = fmaf(ss * cx, cx, mo.qx);
-      mo.gx = fmaf(g.x + g.y, cx, mo.gx);
-      mo.cmass += (s.x > kEps ? 1.f : 0.f) + (s.y > kEps ? 1.f : 0.f);
-      mo.cgrow += (g.x > kEps ? 1.f : 0.f) + (g.y > kEps ? 1.f : 0.f);
+      mo.add_cell(s, g, cx);
       most = make_float2(fmaxf(most.x, s.x), fmaxf(most.y, s.y));
       if (x == 0 || x == W - 1) lx |= fmaxf(s.x, s.y) > kEps;
       cx += (float)lanes;
       while (cx >= top) cx -= wrap;  // past the centred frame's end
     }
-    mo.border |= lx || (most.x > kEps && (r.edge & 1)) || (most.y > kEps && (r.edge & 2));
-    mo.m00 += S2.x + S2.y;
-    mo.g00 += G2.x + G2.y;
-    const float y0 = S2.x * r.cy0, y1 = S2.y * r.cy1, z0 = S2.x * r.cz0, z1 = S2.y * r.cz1;
-    mo.my += y0 + y1;
-    mo.mz += z0 + z1;
-    mo.qy = fmaf(y0, r.cy0, fmaf(y1, r.cy1, mo.qy));
-    mo.qz = fmaf(z0, r.cz0, fmaf(z1, r.cz1, mo.qz));
-    mo.gy = fmaf(G2.x, r.cy0, fmaf(G2.y, r.cy1, mo.gy));
-    mo.gz = fmaf(G2.x, r.cz0, fmaf(G2.y, r.cz1, mo.gz));
+    mo.add_row(r, S2, G2, most, lx);
   }
 }
 __device__ __forceinline__ void epi_single(const NdTab& t, const EpiArgs& a, const RowPair* rp, float2* Z, int nl,
@@ -346,6 +335,144 @@ __device__ __forceinline__ void epi_single(const NdTab& t, const EpiArgs& a, con
   else
     epi_pairs<false, false>(t, a, rp, Z, nl, zp, lanes, w, sx, dt, grow, wf, mo);
 }
+// Several kernels: the rules at the ends of a tile's row transforms.  They take
+// a butterfly's points at once: the pair's row, its addresses and the weights
+// are fetched once for the R points that are inlined behind every radix (code
+// that a block runs once waits for its instructions).  A step, us, cell by cell
+// -> so: one world of 3 x 15 kernels on 100^2 79 -> 60, of one channel with two
+// 47 -> 36; 4 worlds of 3 x 9 on 720^2 407 -> 347, on 48^3 56 -> 48.
+//
+// Kernel k's potentials (times scale) are stored and counted (`count`), their
+// weighted growths added to the fields F [channel lo..hi-1][nl][W].
+struct AddGrowth {
+  const NdTab& t;
+  const EpiArgs& a;
+  const RowPair* rp;
+  float2* F;
+  const float* wt;
+  NdGrowth grow;
+  float* pot;  // the kernel's potential plane, or null
+  int nl, k, lo, hi;
+  bool count;
+  Moments& mo;
+  template <int R>
+  __device__ __forceinline__ void operator()(int l, int at, int step, const float2 (&v)[R]) const {
+    const int rows = rp[l].rows;
+    if (rows == 0) return;
+    float2 g[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) g[q] = __fmul2_rn(v[q], make_float2(a.scale, a.scale));
+    if (count) {
+      if (pot) {
+        float* p = pot + rp[l].cell + at;
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+          p[q * step] = g[q].x;
+          if (rows > 1) p[q * step + t.W] = g[q].y;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < R; ++q) mo.count_pot(g[q], rows);
+    }
+    if (grow.inl) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) g[q] = __ffma2_rn(make_float2(2.f, 2.f), grow.gauss(g[q]), make_float2(-1.f, -1.f));
+    } else {
+#pragma unroll
+      for (int q = 0; q < R; ++q) g[q] = make_float2(grow.any(g[q].x), grow.any(g[q].y));
+    }
+    for (int c = lo; c < hi; ++c) {
+      const float wk = __ldg(wt + c * t.K + k);
+      if (wk == 0.f) continue;
+      float2* f = F + ((long)(c - lo) * nl + l) * t.W + at;
+#pragma unroll
+      for (int q = 0; q < R; ++q) f[q * step] = __ffma2_rn(g[q], make_float2(wk, wk), f[q * step]);
+    }
+  }
+};
+// A channel's new cells from its fields F [nl][W]: update, stores, moments.
+struct UpdateCells {
+  const NdTab& t;
+  const EpiArgs& a;
+  const RowPair* rp;
+  const float2* F;
+  long plane;  // the channel's first cell
+  int sx;
+  float dt, wsum;
+  Moments& mo;
+  template <int R>
+  __device__ __forceinline__ void operator()(int l, int j, int nb, float2 (&v)[R]) const {
+    const RowPair r = rp[l];
+    const int W = t.W;
+    if (r.rows == 0) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = make_float2(0.f, 0.f);
+      return;
+    }
+    const bool two = r.rows > 1;
+    const float2* f = F + (long)l * W + j;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      v[q] = f[q * nb];
+      if (t.mean) v[q] = make_float2(v[q].x / wsum, v[q].y / wsum);
+      if (!two) v[q].y = 0.f;
+    }
+    const long off = plane + r.cell + j;
+    if (a.field_out) {
+      float* p = a.field_out + off;
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        p[q * nb] = v[q].x;
+        if (two) p[q * nb + W] = v[q].y;
+      }
+    }
+    float2 S2 = make_float2(0.f, 0.f), G2 = S2, most = S2;
+    bool lx = false;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int x = j + q * nb;
+      const float* p = a.state + off + q * nb;
+      const float2 s = make_float2(__ldg(p), two ? __ldg(p + W) : 0.f);
+      if (a.state_copy) {
+        a.state_copy[off + q * nb] = s.x;
+        if (two) a.state_copy[off + q * nb + W] = s.y;
+      }
+      const float2 g = make_float2(fmaxf(v[q].x, 0.f), fmaxf(v[q].y, 0.f));
+      v[q] = make_float2(state_fn(t.state_fn, s.x, v[q].x, dt), two ? state_fn(t.state_fn, s.y, v[q].y, dt) : 0.f);
+      a.state_out[off + q * nb] = v[q].x;
+      if (two) a.state_out[off + q * nb + W] = v[q].y;
+      S2 = cadd(S2, s);
+      G2 = cadd(G2, g);
+      mo.add_cell(s, g, centred_in(x, sx, W));
+      most = make_float2(fmaxf(most.x, s.x), fmaxf(most.y, s.y));
+      if (x == 0 || x == W - 1) lx |= fmaxf(s.x, s.y) > kEps;
+    }
+    mo.add_row(r, S2, G2, most, lx);
+  }
+};
+// Channel c's update as the rule of its tile's forward transform (spectra()),
+// or of nothing where no next step follows; its mass is kept for epi_finish.
+template <class Spectra>
+__device__ __forceinline__ void epi_channel(const NdTab& t, const EpiArgs& a, const RowPair* rp, const float2* F,
+                                            int nl, int w, int c, int sx, float dt, const float* wt, Moments& mo,
+                                            EpiShared& sh, const Spectra& spectra) {
+  float wsum = 0.f;
+  for (int k = 0; k < t.K; ++k) wsum += __ldg(wt + c * t.K + k);
+  const float before = mo.m00;
+  mo.m00 = 0.f;  // this channel's mass
+  const UpdateCells update{t, a, rp, F, ((long)w * t.C + c) * t.cells, sx, dt, wsum, mo};
+  if (a.S) {
+    spectra(update);
+  } else {
+    for (int i = threadIdx.x; i < nl * t.W; i += blockDim.x) {
+      float2 v[1];
+      update(i / t.W, i % t.W, 0, v);
+    }
+  }
+  epi_channel_mass(sh, c, mo.m00);
+  mo.m00 += before;
+}
+
 // Threads per row pair: the power of two in 8..32 that leaves the fewest idle
 // along a row; more where a tile has fewer pairs than its threads have warps
 // (rows of thousands of cells).  A step, us, 32 -> 256 threads for a pair of

@@ -165,38 +165,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_epi_kerne
   }
   __syncthreads();
   Moments mo;
-  const long plane0 = (long)w * C * t.cells;
-  const float* __restrict__ state = a.state + plane0;
   float2* Z = p.keep;
-  auto update = [&](const RowPair& r, int c, int x, float2 s, float2 f) {
-    const long off = plane0 + (long)c * t.cells + r.cell + x;
-    float2 n = make_float2(state_fn(t.state_fn, s.x, f.x, dt), 0.f);
-    a.state_out[off] = n.x;
-    if (a.field_out) a.field_out[off] = f.x;
-    if (a.state_copy) a.state_copy[off] = s.x;
-    if (r.rows > 1) {
-      n.y = state_fn(t.state_fn, s.y, f.y, dt);
-      a.state_out[off + W] = n.y;
-      if (a.field_out) a.field_out[off + W] = f.y;
-      if (a.state_copy) a.state_copy[off + W] = s.y;
-    } else {
-      f.y = 0.f;
-    }
-    mo.add(r, s, f, centred_in(x, s2, W), x == 0 || x == W - 1);
-    return n;
-  };
-  auto load_state = [&](const RowPair& r, int c, int x) {
-    const float* q = state + (long)c * t.cells + r.cell + x;
-    return make_float2(__ldg(q), r.rows > 1 ? __ldg(q + W) : 0.f);
-  };
-  auto store_pot = [&](const RowPair& r, int k, int x, float2 u) {
-    if (a.pot_out) {
-      float* q = a.pot_out + ((long)w * K + k) * t.cells + r.cell + x;
-      q[0] = u.x;
-      if (r.rows > 1) q[W] = u.y;
-    }
-    mo.count_pot(u, r.rows);
-  };
   auto store_z = [=](int l, int k, float2 v) { Z[l * zp + k] = v; };
   const long hplane = (long)H * Wh;
   const KeptRows kept{p.keep, g.hp, H, W, Wh};
@@ -221,47 +190,23 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_epi_kerne
     __syncthreads();
     for (int k = 0; k < K; ++k) {
       if (!((ch.todo >> k) & 1ull)) continue;
-      const bool count = (ch.count >> k) & 1ull;
-      const NdGrowth grow(t.gf[k], __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1));
       columns_inverse(p, g, ay, Wh, a.P + ((long)w * K + k) * t.hcells + z * hplane);
       as_rows(p.t, g);
-      line_fft<true, false, false>(ax, p.twx, p.t, kept, [&](int l, int x, float2 v) {
-        const RowPair& r = rp[l];
-        const float2 u = make_float2(v.x * a.scale, v.y * a.scale);
-        if (count) store_pot(r, k, x, u);
-        const float2 gr = make_float2(grow(u.x), grow(u.y));
-        for (int c = ch.lo; c < ch.hi; ++c) {
-          const float wk = __ldg(wt + c * K + k);
-          if (wk == 0.f) continue;
-          float2* f = F + ((long)(c - ch.lo) * g.pp + l) * W + x;
-          *f = __ffma2_rn(gr, make_float2(wk, wk), *f);
-        }
-      });
+      const AddGrowth add{t, a, rp, F, wt, NdGrowth(t.gf[k], __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1)),
+                          a.pot_out ? a.pot_out + ((long)w * K + k) * t.cells : nullptr,
+                          g.pp, k, ch.lo, ch.hi, (bool)((ch.count >> k) & 1ull), mo};
+      line_fft_rules<true, false, LINE_PLAIN>(ax, p.twx, p.t, each_in(kept), add);
       __syncthreads();  // the half plane is rewritten by the next kernel
     }
-    for (int c = ch.lo; c < ch.hi; ++c) {
-      float wsum = 0.f;
-      for (int k = 0; k < K; ++k) wsum += __ldg(wt + c * K + k);
-      const float before = mo.m00;
-      mo.m00 = 0.f;  // this channel's mass
-      auto new_cells = [&](int l, int x) {
-        const RowPair& r = rp[l];
-        float2 f = F[((long)(c - ch.lo) * g.pp + l) * W + x];
-        if (t.mean) f = make_float2(f.x / wsum, f.y / wsum);
-        return update(r, c, x, load_state(r, c, x), f);
-      };
-      if (a.S) {
-        as_rows(p.t, g);
-        line_fft<false, false, false>(ax, p.twx, p.t, new_cells, store_z);
-        __syncthreads();
-        columns_from_rows(p, g, ay, W, Wh, a.S + ((long)w * C + c) * t.hcells + z * hplane);
-        __syncthreads();  // Z is rewritten by the next channel
-      } else {
-        for (int i = threadIdx.x; i < g.pp * W; i += blockDim.x) new_cells(i / W, i % W);
-      }
-      epi_channel_mass(sh, c, mo.m00);
-      mo.m00 += before;
-    }
+    for (int c = ch.lo; c < ch.hi; ++c)
+      epi_channel(t, a, rp, F + (long)(c - ch.lo) * g.pp * W, g.pp, w, c, s2, dt, wt, mo, sh,
+                  [&](const UpdateCells& update) {
+                    as_rows(p.t, g);
+                    line_fft_rules<false, false, LINE_PLAIN>(ax, p.twx, p.t, update, each_out(store_z));
+                    __syncthreads();
+                    columns_from_rows(p, g, ay, W, Wh, a.S + ((long)w * C + c) * t.hcells + z * hplane);
+                    __syncthreads();  // Z is rewritten by the next channel
+                  });
     for (int c = 0; c < C; ++c)
       if (c < ch.lo || c >= ch.hi) epi_channel_mass(sh, c, 0.f);
   }

@@ -181,8 +181,8 @@ struct RowsEpi {
 
 // SINGLE (C = K = 1): the epilogue works on the potentials in Z and leaves the
 // new cells there.  Otherwise the weighted fields of the tile accumulate over
-// the kernels in F, and the update is the load rule of each channel's forward
-// transform.
+// the kernels in F (AddGrowth, the store rule of their inverse transforms), and
+// the update (UpdateCells) is the load rule of each channel's forward one.
 template <bool SINGLE, int KIND>
 __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kernel(NdTab t, EpiArgs a, RowsEpi g, LineAxis ax) {
   extern __shared__ __align__(16) float2 sm[];
@@ -216,8 +216,6 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
   }
   __syncthreads();
   Moments mo;
-  const long plane0 = (long)w * C * t.cells;  // the world's first cell
-  const float* __restrict__ state = a.state + plane0;
   // the product rows of kernel k, packed
   auto load_rows = [&](int k) {
     const float2* __restrict__ src = a.P + ((long)w * K + k) * t.hcells + (long)2 * b * g.nr * Wh;
@@ -228,28 +226,6 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
       const float2 z = make_float2(0.f, 0.f);
       return pack_rows(n > 0 ? __ldg(p) : z, n > 1 ? __ldg(p + Wh) : z, i, W);
     };
-  };
-  // both cells of a pair: state update, stores, moments; returns the new cells
-  auto update = [&](const RowPair& r, int c, int x, float2 s, float2 f) {
-    const long off = plane0 + (long)c * t.cells + r.cell + x;
-    float2 n = make_float2(state_fn(t.state_fn, s.x, f.x, dt), 0.f);
-    a.state_out[off] = n.x;
-    if (a.field_out) a.field_out[off] = f.x;
-    if (a.state_copy) a.state_copy[off] = s.x;
-    if (r.rows > 1) {
-      n.y = state_fn(t.state_fn, s.y, f.y, dt);
-      a.state_out[off + W] = n.y;
-      if (a.field_out) a.field_out[off + W] = f.y;
-      if (a.state_copy) a.state_copy[off + W] = s.y;
-    } else {
-      f.y = 0.f;
-    }
-    mo.add(r, s, f, centred_in(x, sx, W), x == 0 || x == W - 1);
-    return n;
-  };
-  auto load_state = [&](const RowPair& r, int c, int x) {
-    const float* p = state + (long)c * t.cells + r.cell + x;
-    return make_float2(__ldg(p), r.rows > 1 ? __ldg(p + W) : 0.f);
   };
   // half spectra of the tile's new rows (in Z) into S
   auto store_spectra = [&](int c) {
@@ -288,51 +264,21 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
     __syncthreads();
     for (int k = 0; k < K; ++k) {
       if (!((ch.todo >> k) & 1ull)) continue;
-      const bool count = (ch.count >> k) & 1ull;
-      const NdGrowth grow(t.gf[k], __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1));
-      line_fft<true, false, KIND>(ax, tw, tl, load_rows(k), [&](int l, int x, float2 v) {
-        const int rows = rp[l].rows;
-        if (rows == 0) return;
-        const float2 u = make_float2(v.x * a.scale, v.y * a.scale);
-        if (count && a.pot_out) {
-          float* p = a.pot_out + ((long)w * K + k) * t.cells + rp[l].cell + x;
-          p[0] = u.x;
-          if (rows > 1) p[W] = u.y;
-        }
-        if (count) mo.count_pot(u, rows);
-        const float2 gr = make_float2(grow(u.x), grow(u.y));
-        for (int c = ch.lo; c < ch.hi; ++c) {
-          const float wk = __ldg(wt + c * K + k);
-          if (wk == 0.f) continue;
-          float2* f = F + ((long)(c - ch.lo) * g.nr + l) * W + x;
-          *f = __ffma2_rn(gr, make_float2(wk, wk), *f);
-        }
-      });
+      const auto rows = load_rows(k);
+      const AddGrowth add{t, a, rp, F, wt, NdGrowth(t.gf[k], __ldg(gf + 2 * k), __ldg(gf + 2 * k + 1)),
+                          a.pot_out ? a.pot_out + ((long)w * K + k) * t.cells : nullptr,
+                          g.nr, k, ch.lo, ch.hi, (bool)((ch.count >> k) & 1ull), mo};
+      line_fft_rules<true, false, KIND>(ax, tw, tl, each_in(rows), add);
     }
     __syncthreads();
-    for (int c = ch.lo; c < ch.hi; ++c) {
-      float wsum = 0.f;
-      for (int k = 0; k < K; ++k) wsum += __ldg(wt + c * K + k);
-      const float before = mo.m00;
-      mo.m00 = 0.f;  // this channel's mass
-      auto new_cells = [&](int l, int x) {
-        const RowPair& r = rp[l];
-        if (r.rows == 0) return make_float2(0.f, 0.f);
-        float2 f = F[((long)(c - ch.lo) * g.nr + l) * W + x];
-        if (t.mean) f = make_float2(f.x / wsum, f.y / wsum);
-        return update(r, c, x, load_state(r, c, x), f);
-      };
-      if (a.S) {
-        line_fft<false, false, KIND>(ax, tw, tl, new_cells, store_z);
-        __syncthreads();
-        store_spectra(c);
-        __syncthreads();  // Z is rewritten by the next channel
-      } else {
-        for (int i = threadIdx.x; i < g.nr * W; i += blockDim.x) new_cells(i / W, i % W);
-      }
-      epi_channel_mass(sh, c, mo.m00);
-      mo.m00 += before;
-    }
+    for (int c = ch.lo; c < ch.hi; ++c)
+      epi_channel(t, a, rp, F + (long)(c - ch.lo) * g.nr * W, g.nr, w, c, sx, dt, wt, mo, sh,
+                  [&](const UpdateCells& update) {
+                    line_fft_rules<false, false, KIND>(ax, tw, tl, update, each_out(store_z));
+                    __syncthreads();
+                    store_spectra(c);
+                    __syncthreads();  // Z is rewritten by the next channel
+                  });
     for (int c = 0; c < C; ++c)
       if (c < ch.lo || c >= ch.hi) epi_channel_mass(sh, c, 0.f);
   }
