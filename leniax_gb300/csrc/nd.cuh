@@ -104,25 +104,20 @@ struct NdGrowth {
   float m, s;
   // the exponent's coefficient log2(e) / (2 s^2) as an unevaluated sum c + dc:
   // rounded to one float its error is the same in every cell of a world, and a
-  // world's growth shows it where cells' roundings average out.  c is rounded
-  // down and dc > 0, so that both parts of the exponent of an infinite square
-  // are -inf (growth -1), not inf - inf.
+  // world's growth shows it where cells' roundings average out.  c lies below
+  // the coefficient (four units in the last place cover the roundings of 1/q,
+  // the product, s^2 and the constant), so dc > 0 and both parts of the
+  // exponent of an infinite square are -inf (growth -1), not inf - inf.
   float c, dc;
   // Widths whose square, coefficient and remainder are all normal floats; for
-  // the others (0, tiny, huge, infinite, NaN) growth_fn's quotient is exact
-  // where the sum c + dc is infinite or NaN.
+  // the others (0, tiny, huge, infinite, NaN) c + dc is infinite or NaN and
+  // growth_fn's quotient stands.
   __device__ __forceinline__ static bool regular(float s) { return fabsf(s) >= 0x1p-50f && fabsf(s) <= 0x1p50f; }
   __device__ __forceinline__ NdGrowth(int id, float m, float s)
-      : id(id), inl(id == LGX_GF_GAUSSIAN && regular(s)), m(m), s(s), c(0.f), dc(0.f) {
-    if (!inl) return;
-    const float q = s * s, dq = fmaf(s, s, -q);  // s^2 = q + dq
-    const auto rest = [=](float c) { return (fmaf(-c, q, kC) + (kDc - c * dq)) / q; };
-    c = kC / q;
-    dc = rest(c);
-    if (!(dc > 0.f)) {
-      c = __int_as_float(__float_as_int(c) - 1);
-      dc = rest(c);
-    }
+      : id(id), inl(id == LGX_GF_GAUSSIAN && regular(s)), m(m), s(s) {
+    const float q = s * s, dq = fmaf(s, s, -q), inv = 1.f / q;  // s^2 = q + dq
+    c = __int_as_float(__float_as_int(kC * inv) - 4);
+    dc = (fmaf(-c, q, kC) + (kDc - c * dq)) * inv;
   }
   static constexpr double kLog2E2 = 0.72134752044448170368;  // log2(e) / 2
   static constexpr float kC = (float)kLog2E2, kDc = (float)(kLog2E2 - (double)kC);
