@@ -128,6 +128,11 @@ struct RowTile {
   int nr, pitch, zp, threads;
   long buf;
 };
+// Dynamic shared memory of an epilogue block that three of fit an SM: a third
+// of its 228 KB, less the system's kilobyte a block and the kernel's own static
+// arrays.
+constexpr long kThreeBlocksSmem =
+    (228 * 1024 / 3 - 1024 - (long)(sizeof(EpiShared) + kMaxTileLines * sizeof(RowPair))) / 256 * 256;
 RowTile row_tile(const LineAxis& x, long pairs, long group_pairs, bool three = false) {
   RowTile r;
   // `three`: no more lines than leave room for three blocks an SM, as many as
@@ -135,8 +140,11 @@ RowTile row_tile(const LineAxis& x, long pairs, long group_pairs, bool three = f
   // kernels and of wide lines measured slower when cut: 8 worlds of 360 x 480,
   // 3 x 15 kernels 4169 -> 5438 us).  12-step rollouts, us, larger tiles ->
   // these: 32 worlds of 128 x 512 771 -> 580, 512 of 80^2 782 -> 708, 128 of
-  // 144^2 819 -> 792; 100^2 and 250^2 as before.
-  const long pts = 74 * 1024L / (long)sizeof(float2) - x.m;
+  // 144^2 819 -> 792; where only the last 2.5 KB decide (two blocks at 74 KB):
+  // 32 of 250^2 700 -> 568, 128 1879 -> 1695, 32 of 576^2 3067 -> 2693, 24 of
+  // 480^2 1555 -> 1411, of 720^2 4968 -> 4462, 200 of 224^2 2367 -> 2142 (a
+  // batch whose waves fall badly loses: 64 of 224^2 758 -> 802).
+  const long pts = kThreeBlocksSmem / (long)sizeof(float2) - x.m;
   const long by_smem = three ? std::max(1L, pts / (2 * line_pitch(false, x, 1) + (x.n | 1))) : kMaxTileLines;
   const long fill = (pairs + kFillBlocks - 1) / kFillBlocks;
   // one butterfly per thread at most twice over
