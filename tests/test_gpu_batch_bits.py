@@ -51,7 +51,7 @@ def test_streamed_worlds(cuda, side, C, per, slugs, limit, mean):
                                               ((66, 40), 2, 2, 100), ((1024, 1024), 1, 1, 3), ((24, 24, 24), 1, 1, 40),
                                               ((48, 48, 48), 2, 2, 9), ((40, 80, 72), 1, 1, 5), ((128, 512), 1, 1, 32),
                                               ((224, 224), 1, 1, 64), ((480, 480), 1, 1, 13),
-                                              ((576, 576), 1, 1, 9), ((4, 4096), 1, 1, 30)])
+                                              ((576, 576), 1, 1, 9), ((16, 4096), 1, 1, 30)])
 @pytest.mark.parametrize('mean', [True, False])
 def test_nd_worlds(cuda, world, C, per, most, mean):
     rng = np.random.Generator(np.random.PCG64(sum(world)))
