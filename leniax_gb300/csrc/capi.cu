@@ -105,9 +105,9 @@ int select_engine(const Model& m, int requested) {
   if (requested == LGX_ENGINE_ND) return nd_supported(m) ? LGX_ENGINE_ND : -1;
   if (requested != LGX_ENGINE_AUTO) return -1;
   if (resident_supported(m)) return LGX_ENGINE_RESIDENT;
-  // even sides that are not powers of two: N-D steps, several times the
-  // mixed-radix streamed step from a few planes on (see update_engine), which
-  // stays available on request
+  // even sides that are not powers of two: N-D steps, faster than the
+  // mixed-radix streamed step (see update_engine), which stays available on
+  // request
   if (streamed_supported(m) && !(generic_size(m.H) && nd_supported(m))) return LGX_ENGINE_STREAMED;
   if (cta_supported(m)) return LGX_ENGINE_CTA;
   if (nd_supported(m)) return LGX_ENGINE_ND;
@@ -231,14 +231,14 @@ size_t run_workspace(const Model& m, int n_sols, int n_init, int steps, int e) {
 // The engine of one lgx_update step: a streamed step for 2D powers of two
 // (resident sizes included), one world per CTA for 3D batches that fill the
 // chip, else an N-D step.  `general`: the engine taken where the workspace has
-// no room for the N-D step's.  Other even squares run the mixed-radix streamed
-// step only for one or two planes; a step, us, streamed / N-D: 100^2, 1 plane
-// 40 / 44, 64 86 / 39, 8 worlds of 3 channels x 9 kernels 98 / 73, 64 of them
-// 342 / 139; 360^2, 1 plane 61 / 73, 8 96 / 61, one world of 3 x 9 156 / 100;
-// 48^2, 1 plane 41 / 37, one world of 3 x 9 89 / 67.
+// no room for the N-D step's.  For the other even squares that is the
+// mixed-radix streamed step; a step, us, that / N-D: one plane of 48^2
+// 36 / 31, of 100^2 40 / 37, of 360^2 59 / 56, of 480^2 65 / 44, of 500^2 62 / 65
+// (the one side of eighteen where it is ahead); two channels with eight
+// kernels on 100^2 80 / 52, on 360^2 148 / 66; 64 planes of 100^2 86 / 39.
 int update_engine(const Model& m, long n, bool general = false) {
   if (streamed_supported(m))
-    return !general && generic_size(m.H) && n * m.C > 2 && nd_supported(m) ? LGX_ENGINE_ND : LGX_ENGINE_STREAMED;
+    return !general && generic_size(m.H) && nd_supported(m) ? LGX_ENGINE_ND : LGX_ENGINE_STREAMED;
   if (cta_supported(m)) return !general && few_3d_worlds(m, n) ? LGX_ENGINE_ND : LGX_ENGINE_CTA;
   return nd_supported(m) ? LGX_ENGINE_ND : -1;
 }

@@ -60,3 +60,16 @@ def test_nd_worlds(cuda, world, C, per, most, mean):
     for n in (1, 2, most // 2):
         few = _run(cuda, world, C, per, ('gaussian', ), mean, cells[:n], 'nd')
         assert all(torch.equal(a, b[:, :n]) for a, b in zip(few, whole))
+
+
+@pytest.mark.parametrize('side,C,per', [(24, 1, 1), (100, 1, 1), (126, 2, 2), (360, 1, 3), (500, 1, 1)])
+def test_update_steps_on_even_squares(cuda, side, C, per):
+    kp = random_multichannel_params(C, per, seed=7, R_range=(3.0, 5.0), world_R=5.0)
+    K, mp = kernels.get_kernels_and_mapping(kp, [side, side], C, 5.0, True, cuda)
+    upd = helpers.build_update_fn(K.shape, mp)
+    rng = np.random.Generator(np.random.PCG64(side))
+    cells = torch.from_numpy(rng.random((9, C, side, side), dtype=np.float32)).to(cuda)
+    args = (K, mp.get_gf_params(cuda), mp.get_kernels_weight_per_channel(cuda), 0.1)
+    whole = upd(None, cells, *args)
+    for n in (1, 2, 3):
+        assert all(torch.equal(a, b[:n]) for a, b in zip(upd(None, cells[:n], *args), whole))
