@@ -151,8 +151,7 @@ struct RowPair {
   int edge;          // bit 0 / 1: the row lies on the outer layer of the un-centred world
 };
 
-__device__ __forceinline__ RowPair row_pair(const NdTab& t, int z0, int y0, int z1, int y1, int rows, int s0, int s1,
-                                            int s2) {
+__device__ __forceinline__ RowPair row_pair(const NdTab& t, int z0, int y0, int z1, int y1, int rows, int s0, int s1) {
   RowPair r;
   r.cell = ((long)z0 * t.H + y0) * t.W;
   r.rows = rows;
@@ -164,7 +163,6 @@ __device__ __forceinline__ RowPair row_pair(const NdTab& t, int z0, int y0, int 
   const bool e0 = y0 == 0 || y0 == t.H - 1 || (t.nd == 3 && (z0 == 0 || z0 == t.D - 1));
   const bool e1 = y1 == 0 || y1 == t.H - 1 || (t.nd == 3 && (z1 == 0 || z1 == t.D - 1));
   r.edge = (e0 ? 1 : 0) | (e1 ? 2 : 0);
-  (void)s2;
   return r;
 }
 

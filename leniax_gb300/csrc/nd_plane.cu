@@ -54,7 +54,7 @@ __device__ __forceinline__ void columns_from_rows(PlaneTile& p, const PlaneGeo& 
   const float2* Z = p.keep;
   const int zp = g.zp;
   as_columns(p.t, g, Wh);
-  line_fft<false, true, false>(
+  line_fft<false, true, LINE_PLAIN>(
       ay, p.twy, p.t,
       [=](int l, int i) {
         const float2* z = Z + (i >> 1) * zp;
@@ -70,7 +70,7 @@ __device__ __forceinline__ void columns_inverse(PlaneTile& p, const PlaneGeo& g,
   float2* h = p.keep;
   const int hp = g.hp;
   as_columns(p.t, g, Wh);
-  line_fft<true, true, false>(
+  line_fft<true, true, LINE_PLAIN>(
       ay, p.twy, p.t, [=](int l, int i) { return __ldg(src + i * Wh + l); },
       [=](int l, int i, float2 v) { h[i * hp + l] = v; });
   __syncthreads();
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_fwd_kerne
   const float* __restrict__ src = a.src + (long)blockIdx.x * H * W;
   float2* Z = p.keep;
   as_rows(p.t, g);
-  line_fft<false, false, false>(
+  line_fft<false, false, LINE_PLAIN>(
       ax, p.twx, p.t,
       [=](int l, int i) {
         const float* q = src + 2 * l * W + i;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_inv_kerne
   const float scale = a.scale;
   const bool add = a.accumulate != 0;
   as_rows(p.t, g);
-  line_fft<true, false, false>(ax, p.twx, p.t, KeptRows{p.keep, g.hp, H, W, Wh}, [=](int l, int x, float2 v) {
+  line_fft<true, false, LINE_PLAIN>(ax, p.twx, p.t, KeptRows{p.keep, g.hp, H, W, Wh}, [=](int l, int x, float2 v) {
     float* q = dst + 2 * l * W + x;
     q[0] = add ? fmaf(v.x, scale, q[0]) : v.x * scale;
     if (2 * l + 1 < H) q[W] = add ? fmaf(v.y, scale, q[W]) : v.y * scale;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_epi_kerne
   const float* wt = a.w + sol * a.w_sol_stride;
   for (int l = threadIdx.x; l < g.pp; l += blockDim.x) {
     const int y1 = min(2 * l + 1, H - 1);
-    rp[l] = row_pair(t, z, 2 * l, z, y1, 2 * l + 1 < H ? 2 : 1, s0, s1, s2);
+    rp[l] = row_pair(t, z, 2 * l, z, y1, 2 * l + 1 < H ? 2 : 1, s0, s1);
   }
   __syncthreads();
   Moments mo;
@@ -172,12 +172,12 @@ __global__ void __launch_bounds__(kNdThreads, kNdBlocksPerSm) nd_plane_epi_kerne
   if constexpr (SINGLE) {
     columns_inverse(p, g, ay, Wh, a.P + (long)w * t.hcells + z * hplane);
     as_rows(p.t, g);
-    line_fft<true, false, false>(ax, p.twx, p.t, kept, store_z);
+    line_fft<true, false, LINE_PLAIN>(ax, p.twx, p.t, kept, store_z);
     __syncthreads();
     epi_single(t, a, rp, Z, g.pp, zp, g.lanes, w, s2, dt, mo);
     if (a.S) {
       __syncthreads();
-      line_fft<false, false, false>(ax, p.twx, p.t, [=](int l, int i) { return Z[l * zp + i]; }, store_z);
+      line_fft<false, false, LINE_PLAIN>(ax, p.twx, p.t, [=](int l, int i) { return Z[l * zp + i]; }, store_z);
       __syncthreads();
       columns_from_rows(p, g, ay, W, Wh, a.S + (long)w * t.hcells + z * hplane);
     }

@@ -180,7 +180,7 @@ cudaError_t rows_args(const LineAxis& x, long planes, int rows, RowsArgs* a, Row
 
 // ------------------------------------------------------------------ epilogue
 struct RowsEpi {
-  int pp, nr, pitch, zp;  // pairs per world, pairs per tile, pitches
+  int nr, pitch, zp;      // pairs per tile, pitches
   int lanes;              // threads per row pair of the epilogue
   long buf;
   FastDivU nrd, hd, whd;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kNdThreads, nd_blocks(KIND)) nd_rows_epi_kerne
     const int r0 = 2 * (b * g.nr + l), rows = max(0, min(2, t.D * t.H - r0));
     const int q0 = rows > 0 ? r0 : 0, q1 = rows > 1 ? r0 + 1 : q0;
     const int z0 = g.hd.div(q0), z1 = g.hd.div(q1);
-    rp[l] = row_pair(t, z0, q0 - z0 * t.H, z1, q1 - z1 * t.H, rows, s0, s1, s2);
+    rp[l] = row_pair(t, z0, q0 - z0 * t.H, z1, q1 - z1 * t.H, rows, s0, s1);
   }
   __syncthreads();
   Moments mo;
@@ -361,7 +361,6 @@ cudaError_t nd_rows_epilogue(const NdTab& t, const LineAxis& x, const EpiArgs& a
   a.split = e.split ? 1 : 0;
   a.bpw = e.tiles * (e.split ? t.C : 1);
   RowsEpi g;
-  g.pp = (t.D * t.H + 1) / 2;
   g.nr = e.rt.nr;
   g.pitch = e.rt.pitch;
   g.zp = e.rt.zp;
