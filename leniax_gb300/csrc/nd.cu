@@ -616,8 +616,10 @@ AdjLayout adj_layout(const Model& m, int n_sols, int n_init) {
 
 size_t nd_adjoint_workspace_bytes(const Model& m, int n_sols, int n_init) { return adj_layout(m, n_sols, n_init).end; }
 
+// A whole complex plane a (world, kernel), the size the interface has answered
+// from the start; the half spectra that the adjoint accumulates fill the front.
 size_t nd_kernel_grad_acc_bytes(const Model& m, int n_sols, int n_init) {
-  return (size_t)n_sols * n_init * m.K * m.D * m.H * (m.W / 2 + 1) * sizeof(float2);
+  return (size_t)n_sols * n_init * m.K * m.cells * sizeof(float2);
 }
 
 cudaError_t launch_nd_adjoint(const Model& m, const NdAdjoint& j, void* ws, cudaStream_t st) {
