@@ -775,16 +775,32 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
   // channel 0 also takes the kernels that feed no channel (their potentials count)
   const unsigned long long all = K == 64 ? ~0ull : (1ull << K) - 1ull;
   const unsigned long long mine = fed | (co == 0 ? all & ~any : 0ull);
+  float dt;
+  if (tab.dt_mode == 0) dt = __ldg(dtp);
+  else if (tab.dt_mode == 1) dt = __ldg(dtp + n);
+  else dt = 1.f / __ldg(dtp + sol);
+  // this warp's kernel among those of a round (-1: none) and its parameters,
+  // fetched ahead of the rows; a kernel that feeds no channel has weight 0
+  int k = -1;
+  float wk = 0.f;
+  GrowthP g;
+  auto next_item = [&](unsigned long long todo) {
+    for (int q = 0; q < wid; ++q) todo &= todo - 1;
+    k = __ffsll((long long)todo) - 1;
+    if (k < 0) return;
+    wk = (fed >> k) & 1ull ? __ldg(wt + co * K + k) : 0.f;
+    g.m = __ldg(gf + 2 * k);
+    g.s = __ldg(gf + 2 * k + 1);
+    g.a = GF == GF_FAST_GAUSSIAN ? 0.84932180028801904272f / g.s : (GF == GF_FAST_POLY4 ? 1.f / (9.f * (g.s * g.s)) : 0.f);
+    g.id = tab.gf[k];
+  };
+  next_item(mine);
 
   depend_wait();
   depend_trigger();
   prod = after_wait(prod);
   state = after_wait(state);
   shift = after_wait(shift);
-  float dt;
-  if (tab.dt_mode == 0) dt = __ldg(dtp);
-  else if (tab.dt_mode == 1) dt = __ldg(dtp + n);
-  else dt = 1.f / __ldg(dtp + sol);
   const int sy = shift[3 * n], sx = shift[3 * n + 1];
   const size_t base = ((size_t)n * C + co) * N * N + (size_t)(2 * r) * N;
   float cpot = 0.f;
@@ -793,6 +809,7 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
   // then the warps add them up, cell by cell in kernel order (warp w the cells
   // k1 = w, w + warps, ...); the last round's sum is taken by the epilogue.
   auto add_round = [&](float2 f, int k1, int items) {
+#pragma unroll 4
     for (int q = 0; q < items; ++q) {
       const float2 e = xch[q * SC::XCH + k1 * 32 + lane];
       const float wk = wk_s[q];
@@ -808,10 +825,7 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
     for (int k1 = wid; k1 < P; k1 += warps) sum[k1 * 32 + lane] = make_float2(0.f, 0.f);
   __syncthreads();
   for (;;) {
-    unsigned long long m = todo;
-    for (int q = 0; q < wid; ++q) m &= m - 1;
-    const int k = m ? __ffsll((long long)m) - 1 : 0;
-    if (m) {
+    if (k >= 0) {
       const float2* row = prod + (((size_t)n * K + k) * (N / 2) + r) * N;
       float2 v[Q][G];
       if constexpr (Q == 1) unpack_row_pair_q1<GE>(row, v, t);
@@ -830,15 +844,8 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
           }
         }
       }
-      // a kernel that feeds no channel adds 0
       const bool feeds = (fed >> k) & 1ull;
-      const float wk = feeds ? __ldg(wt + co * K + k) : 0.f;
       if (lane == 0) wk_s[wid] = GF == GF_GENERIC ? wk : 2.f * wk;
-      GrowthP g;
-      g.m = __ldg(gf + 2 * k);
-      g.s = __ldg(gf + 2 * k + 1);
-      g.a = GF == GF_FAST_GAUSSIAN ? 0.84932180028801904272f / g.s : (GF == GF_FAST_POLY4 ? 1.f / (9.f * (g.s * g.s)) : 0.f);
-      g.id = tab.gf[k];
       __syncwarp();  // every group of the warp has read its exchange
 #pragma unroll
       for (int k1 = 0; k1 < P; ++k1) {
@@ -855,6 +862,7 @@ __global__ void __launch_bounds__(32 * kSplitMaxWarps) row_inv_split_kernel(
     for (int k1 = wid; k1 < P; k1 += warps) sum[k1 * 32 + lane] = add_round(sum[k1 * 32 + lane], k1, warps);
     for (int q = 0; q < warps; ++q) todo &= todo - 1;
     left -= warps;
+    next_item(todo);
     __syncthreads();
   }
 
