@@ -537,7 +537,10 @@ __device__ __forceinline__ void epi_finish(const NdTab& t, const EpiArgs& a, Epi
         v[j] = bb < bpw ? __ldcg(pw + (long)bb * RAWS + s) : 0.f;
       }
 #pragma unroll
-      for (int j = 0; j < kLoads; ++j) acc += v[j];
+      for (int d = kLoads / 2; d > 0; d /= 2)  // by pairs: a chain of hundreds of partials rounds as often
+#pragma unroll
+        for (int j = 0; j < d; ++j) v[j] += v[j + d];
+      acc += v[0];
     }
     sh.red[wid][s] = acc;
   }

@@ -44,3 +44,19 @@ def test_statistics_match_the_oracle(cuda, world, n, C, per):
     cell = R**2 / cells[0].size
     mean = np.stack(growths) * cell
     assert (np.abs(sd['growth'].cpu().numpy() * cell - mean) <= 41e-6 * np.maximum(mean, 1) + 1e-5 * mean).all()
+
+
+@pytest.mark.parametrize('world', [(4096, 4, 4), (1024, 8, 8), (2048, 6, 4), (1000, 1000)])
+@pytest.mark.parametrize('value', [0.1, 0.37, 0.7, 0.9])
+def test_masses_of_constant_worlds(cuda, world, value):
+    # equal terms round the same way in a chain; by pairs a sum of n blocks is log2(n) roundings deep.  At most
+    # 64 roundings from a cell to its world's mass: a thread's cells, a warp, a block's warps, the partials
+    R = 2.0
+    kp = random_multichannel_params(1, 1, seed=3, R_range=(0.7 * R, R), world_R=R)
+    K, mp = kernels.get_kernels_and_mapping(kp, list(world), 1, R, True, cuda)
+    upd = helpers.build_update_fn(K.shape, mp, 'v1', True)
+    cells = torch.full((1, 1) + world, value, device=cuda)
+    *_, sd = runner.run_scan(None, cells, K, mp.get_gf_params(cuda), mp.get_kernels_weight_per_channel(cuda),
+                             torch.tensor(10.0), 1, R, upd, statistics.ComputeStatsFn(list(world), R, 10.0), engine='nd')
+    mass = float(np.float32(value)) * np.prod(world) / R**2
+    assert abs(float(sd['mass'][0, 0]) / mass - 1) <= 64 * 2.0**-24
