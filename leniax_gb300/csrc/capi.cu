@@ -204,9 +204,9 @@ NdLayout nd_layout(const Model& m, int n_sols, int n_init, int steps) {
 // chip idle: their default engine (LGX_ENGINE_CTA) runs them by N-D steps,
 // each step spread over all SMs.  A CTA round is as long for one world as for
 // one a SM; an N-D step grows with the worlds.  8-step rollouts on 152 SMs,
-// us, one CTA a world / N-D steps: 64^3, 64 worlds 2680 / 2140, 128 2696 /
-// 3853, 256 (two rounds) 5179 / 7233, and 343 for one world, 730 for 16; 32^3,
-// 64 worlds 474 / 571, 256 822 / 1628, and 300 for one world, 325 for 16.
+// us, one CTA a world / N-D steps: 64^3, 64 worlds 2667 / 1997, 92 2678 / 2689,
+// 152 2693 / 4161, 180 (two rounds) 5106 / 4859, and 343 for one world; 32^3,
+// 40 worlds 476 / 436, 64 478 / 501, 256 822 / 1628, and 300 for one world.
 bool few_3d_worlds(const Model& m, long nw) {
   if (!cta_supported(m) || !nd_supported(m)) return false;
   const long sms = sm_count_now(), rounds = (nw + sms - 1) / sms;
