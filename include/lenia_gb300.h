@@ -75,7 +75,9 @@ extern "C" {
 #define LGX_ENGINE_CTA 4      /* one world per CTA, persistent over a work queue: 3D
                                  worlds of side 32 / 64 (C = K = 1).  As the default
                                  engine of such worlds it runs a batch too small to fill
-                                 the chip by the N-D engine's steps                     */
+                                 the chip by the N-D engine's steps, which round
+                                 otherwise: name an engine where bits must not depend
+                                 on the batch                                           */
 #define LGX_ENGINE_PLAIN_STREAMED 5 /* one world and one step per launch through the streamed
                                  engine's kernel sequence (row, column, row-inverse and
                                  reduce kernels), for any model the streamed engine runs */
